@@ -56,6 +56,29 @@ void rf_twiddles_t(int n, std::vector<C>* tw, F w) {
 inline void rf_twiddles(int n, std::vector<float2>* tw) { rf_twiddles_t(n, tw, twiddle_f); }
 inline void rf_twiddles64(int n, std::vector<double2>* tw) { rf_twiddles_t(n, tw, twiddle_d); }
 
+// Stage twiddles of BlockFft<., n, e> (wig_fft.cuh): per stage of sub-length ns > 1 and radix r1,
+// k < ns: w^{4 k a} and w^{k b} (a, b = 1..3) of radix 16, else w^{k r} (r = 1..r1 - 1),
+// w = exp(-2 pi i / (ns r1)).
+inline std::vector<double2> block_twiddles(int n, int e) {
+  std::vector<double2> tw;
+  int shrt = n;
+  while (shrt > e) shrt /= e;
+  for (int ns = 1; ns < n;) {
+    const int r1 = ns == (n <= e * e ? 1 : e) ? shrt : e;
+    const auto row = [&](int m) {
+      for (int k = 0; k < ns; ++k) tw.push_back(twiddle_d(ns * r1, (long long)k * m));
+    };
+    if (ns > 1 && r1 == 16) {
+      for (int a = 1; a < 4; ++a) row(4 * a);
+      for (int b = 1; b < 4; ++b) row(b);
+    } else if (ns > 1) {
+      for (int r = 1; r < r1; ++r) row(r);
+    }
+    ns *= r1;
+  }
+  return tw;
+}
+
 // One batched instance: constants of BInst (b.off, b.tw_*, work-list fields
 // are set by the caller) and its factor tables, appended to ft (FP32) and fd
 // (FP64; offsets kept even so the double2 sub-table is 16-byte aligned).

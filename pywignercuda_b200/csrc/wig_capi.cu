@@ -57,6 +57,7 @@ struct Driver {
   PFN_cuModuleLoadData load = nullptr;
   PFN_cuModuleGetFunction getf = nullptr;
   PFN_cuLaunchKernel launch = nullptr;
+  PFN_cuLaunchKernelEx launchex = nullptr;
   PFN_cuFuncSetAttribute setattr = nullptr;
   PFN_cuGetErrorString errstr = nullptr;
   PFN_cuTensorMapEncodeTiled encode = nullptr;   // optional: TMA tile loads need it
@@ -81,7 +82,7 @@ int driver(Driver** out) {
   std::lock_guard<std::mutex> lk(g_mu);
   if (!g_drv.ok) {
     if (!(entry("cuModuleLoadData", g_drv.load) && entry("cuModuleGetFunction", g_drv.getf) &&
-          entry("cuLaunchKernel", g_drv.launch) && entry("cuFuncSetAttribute", g_drv.setattr) &&
+          entry("cuLaunchKernel", g_drv.launch) && entry("cuLaunchKernelEx", g_drv.launchex) && entry("cuFuncSetAttribute", g_drv.setattr) &&
           entry("cuGetErrorString", g_drv.errstr)))
       return fail(WIG_ERR_CUDA, "CUDA driver entry points unavailable (no GPU driver?)");
     if (!entry("cuTensorMapEncodeTiled", g_drv.encode)) g_drv.encode = nullptr;
@@ -214,6 +215,26 @@ int launch(CUfunction f, unsigned grid, unsigned block, unsigned smem, cudaStrea
   return WIG_OK;
 }
 
+int launch_after(CUfunction f, unsigned grid, unsigned block, unsigned smem, cudaStream_t st, void** args) {
+  CUlaunchAttribute at;
+  memset(&at, 0, sizeof(at));
+  at.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  at.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchConfig c;
+  memset(&c, 0, sizeof(c));
+  c.gridDimX = grid;
+  c.gridDimY = c.gridDimZ = 1;
+  c.blockDimX = block;
+  c.blockDimY = c.blockDimZ = 1;
+  c.sharedMemBytes = smem;
+  c.hStream = (CUstream)st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  CUresult r = g_drv.launchex(&c, f, args, nullptr);
+  if (r != CUDA_SUCCESS) return fail(WIG_ERR_CUDA, "cuLaunchKernelEx: %s", cu_err(r));
+  return WIG_OK;
+}
+
 int launch2d(CUfunction f, unsigned gx, unsigned gy, unsigned block, unsigned smem, cudaStream_t st, void** args) {
   CUresult r = g_drv.launch(f, gx, gy, 1, block, 1, 1, smem, (CUstream)st, args, nullptr);
   if (r != CUDA_SUCCESS) return fail(WIG_ERR_CUDA, "cuLaunchKernel: %s", cu_err(r));
@@ -340,6 +361,13 @@ struct wig_handle {
   int odm = 0, smem_odm_x = 0, smem_odm_p = 0;
   double2* odm_T = nullptr;                    // 5 planes of ODM intermediates
   double odm_coef[2] = {0., 0.}, odm_sign[2] = {1., -1.};
+  // launch shapes of the x- and p-pass; blocked ones (BlockFft) start with programmatic serialisation, and
+  // their x-pass and first-half p-pass have one CTA more (the sample)
+  int bx = 0, bp = 0, gx = 1, gx_nt = 256, gx_smem = 0, gp_n = 1, gp_nt = 256, gp_smem = 0, gph_smem = 0;
+  int odm2 = 0, gox = 1, gox_nt = 256, gop = 1, gop_nt = 256;   // ODM on BlockFft
+  const double2 *btw_ox = nullptr, *btw_op = nullptr;
+  CUfunction f_gcb = nullptr, f_gpb = nullptr;   // Gross-Pitaevskii terms on BlockFft
+  int gpb_n = 1, gpb_smem = 0, gpb_chunks = 1;
   int rf = 0;                                   // register-FFT x- and p-pass (wig_wigner_rf.cuh)
   int tma = 0, rf_c = 1;                        // the p-pass tile (rf_c columns) arrives by 2-D tensor copies
   wig::TensorMap tmap{};                        // tensor map of the W it was last encoded for
@@ -359,6 +387,10 @@ struct wig_handle {
 
 // Validation, tiling and the JIT source of one Wigner instance (no CUDA calls).
 struct WigPlan {
+  // register-blocked passes: elements a thread, rows / columns a CTA, CTAs per SM
+  int bx = 0, bxe = 8, bxr = 1, bxmb = 1, bp = 0, bpe = 8, bpc = 1, bpmb = 1, bpa = 1;
+  int gx = 1, gx_nt = 256, gx_smem = 0, gp_n = 1, gp_nt = 256, gp_smem = 0, gph_smem = 0;
+  int odm2 = 0, oe = 8, oxr = 1, oxmb = 1, opc = 1, opmb = 1;
   int rf = 0, rfxw = 4, rfpw = 2;   // register-FFT passes (wig_wigner_rf.cuh) and their warps per CTA
   int tma = 0;                      // their p-pass tile by 2-D tensor copies (WIG_TMA)
   int xrows, xnt, pc, pnt, rnt, n_cta_x, n_cta_p, n_cta_r, smem_x, smem_p, damp;
@@ -495,6 +527,73 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
     P->smem_p = (P->damp ? 2 : 1) * P->rfpw * spp * NP * (int)sizeof(double2) + 1024;   // + alignment slack
   }
 
+  // ---- register-blocked passes (BlockFft)
+  {
+    const bool stockham = P->rf || getenv("WIG_TILING") || getenv("WIG_RADIX");   // tile overrides of the other forms
+    P->bx = !stockham && NX >= 64 ? 1 : 0;
+    P->bp = !stockham && NP >= 64 ? 1 : 0;
+    // Elements a thread: as many as the grid leaves threads for.  16 (two stage boundaries in
+    // shared memory up to 4096 points, 128 registers, 16 warps per SM) from 2^19 points, 8 from
+    // 2^17, below that 4, where the step is a chain of latencies and more warps shorten it.
+    // Damped Lie step, us: 1024^2 65 / 83 with 16 / 8; 512^2 32 / 26 / 32 with 16 / 8 / 4;
+    // 512 x 256 - / 21 / 21; 256^2 24 / 18 / 15; 128^2 24 / 17 / 13; 1024 x 64 - / 20 / 16.
+    const long pts = (long)NX * NP;
+    const auto elems = [&](int n) { return std::max(pts >= (1L << 19) ? 16 : (pts >= (1L << 17) ? 8 : 4), n / 512); };
+    P->bxe = elems(NX);
+    P->bpe = elems(NP);
+    // x: one row per CTA (at least a warp).  p: two columns (32-byte segments of a grid row) where that
+    // leaves a CTA for every SM, else one: 256^2 undamped step 9.1 / 10.2 us with one / two, 128 x 1024
+    // damped 22 / 28, 512 x 256 21 / 21, 1024^2 98 / 76.
+    P->bxr = std::max(1, 32 * P->bxe / NX);
+    P->bpc = std::max(P->bpe >= 8 && NX / 2 >= 148 ? 2 : 1, 32 * P->bpe / NP);
+    while (P->bpc > 1 && P->bpc * (NP / P->bpe) > 512) P->bpc /= 2;
+    P->bxmb = P->bpmb = 0;
+    // the Caldeira-Leggett base: with 16 elements a thread in tensor memory (1024^2 damped step 65 us;
+    // in shared memory, two CTAs per SM instead of four, 70), else in registers
+    P->bpa = P->damp && P->bpe == 16 ? 1 : 0;
+    // WIG_BTILING="xe,xr,xmb,pe,pc,pmb,pa" overrides the tiles for tuning runs (0: default; pa: -1 default)
+    if (const char* tv = getenv("WIG_BTILING")) {
+      int v[7];
+      if (sscanf(tv, "%d,%d,%d,%d,%d,%d,%d", &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6]) == 7) {
+        if (v[0] == 4 || v[0] == 8 || v[0] == 16) P->bxe = v[0];
+        P->bxr = std::max(1, 32 * P->bxe / NX);
+        if (v[1] > 0) P->bxr = clampi(v[1], P->bxr, NP);
+        if (v[2] > 0) P->bxmb = v[2];
+        if (v[3] == 4 || v[3] == 8 || v[3] == 16) P->bpe = v[3];
+        P->bpc = std::max(1, 32 * P->bpe / NP);
+        if (v[4] > 0) P->bpc = clampi(v[4], std::max(1, 32 * P->bpe / NP), std::min(NX, 32));
+        if (v[5] > 0) P->bpmb = v[5];
+        if (v[6] >= 0) P->bpa = v[6] ? 1 : 0;
+      }
+    }
+    const int nt = P->bxr * (NX / P->bxe), ntp = P->bpc * (NP / P->bpe);
+    const auto pad = [](int n, int e) { return n + n / std::min(e, 8); };
+    // 512 threads per SM: 128 registers each (the x-pass of 16 elements a thread: 448, 144, no spill)
+    if (!P->bxmb) P->bxmb = std::max(1, std::min(32, (P->bxe == 16 ? 448 : 512) / nt));
+    if (!P->bpmb) P->bpmb = std::max(1, std::min(32, 512 / ntp));
+    if (nt > 1024 || ntp > 1024 || (P->bpc & (P->bpc - 1)) || NP % P->bxr)
+      return fail(WIG_ERR_ARG, "WIG_BTILING: tiles of %d / %d threads", nt, ntp);
+    P->gx = NP / P->bxr + 1;
+    P->gx_nt = nt;
+    P->gx_smem = P->bxr * pad(NX, P->bxe) * (int)sizeof(double2);
+    P->gp_n = NX / P->bpc;
+    P->gp_nt = ntp;
+    P->gph_smem = P->bpc * wig::blk_stride(pad(NP, P->bpe), P->bpc) * (int)sizeof(double2);
+    P->gp_smem = P->gph_smem;
+    if (!P->bx) { P->gx = P->n_cta_x; P->gx_nt = P->xnt; P->gx_smem = P->smem_x; }
+    if (!P->bp) { P->gp_n = P->n_cta_p; P->gp_nt = P->pnt; P->gp_smem = P->smem_p; P->gph_smem = P->smem_ph; }
+    P->odm2 = P->odm && P->bx && P->bp ? 1 : 0;
+    P->oe = 8;
+    P->oxr = std::max(1, 32 * P->oe / NX);
+    P->opc = std::max(2, 32 * P->oe / NP);
+    P->oxmb = std::max(1, std::min(32, 512 / (P->oxr * (NX / P->oe))));
+    P->opmb = std::max(1, std::min(32, 512 / (P->opc * (NP / P->oe))));
+    if (P->odm2) {
+      P->smem_odm_x = P->oxr * (pad(NX, P->oe) * (int)sizeof(double2) + (NX + 1) * (int)sizeof(double));
+      P->smem_odm_p = P->opc * wig::blk_stride(pad(NP, P->oe), P->opc) * (int)sizeof(double2);
+    }
+  }
+
   // ---- JIT source
   P->dX = 2. * d->x_amplitude / (double)NX;
   P->dP = 2. * d->p_amplitude / (double)NP;
@@ -519,6 +618,26 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
            NX, NP, P->xrows, P->xnt, d->kinetic_from_string ? 1 : 0, P->pc, P->pnt, P->damp, P->rnt,
            P->xminb, P->pminb, d->potential_phase == WIG_PHASE_KVN ? 1 : 0, P->strang, P->xr, P->pr);
   src += macros;
+  snprintf(macros, sizeof(macros), "#define WIG_ODM %d\n", P->odm ? 1 + P->odm2 : 0);
+  src += macros;
+  if (P->bx) {
+    snprintf(macros, sizeof(macros), "#define WIG_BX 1\n#define WIG_BXR %d\n#define WIG_BXE %d\n#define WIG_BXMB %d\n",
+             P->bxr, P->bxe, P->bxmb);
+    src += macros;
+  }
+  if (P->bp) {
+    snprintf(macros, sizeof(macros),
+             "#define WIG_BP 1\n#define WIG_BPC %d\n#define WIG_BPE %d\n#define WIG_BPMB %d\n#define WIG_BPA %d\n",
+             P->bpc, P->bpe, P->bpmb, P->bpa);
+    src += macros;
+    if (P->bpa) src += "#define WIG_TMEM 1\n";
+  }
+  if (P->odm2) {
+    snprintf(macros, sizeof(macros),
+             "#define WIG_OE %d\n#define WIG_OXR %d\n#define WIG_OXMB %d\n#define WIG_OPC %d\n#define WIG_OPMB %d\n",
+             P->oe, P->oxr, P->oxmb, P->opc, P->opmb);
+    src += macros;
+  }
   if (P->rf) {
     // 255 registers a thread (a 32-element FP64 sequence per lane is 128 of them)
     snprintf(macros, sizeof(macros),
@@ -558,6 +677,14 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
   h->xrows = P.xrows; h->xnt = P.xnt; h->pc = P.pc; h->pnt = P.pnt; h->rnt = P.rnt;
   h->n_cta_x = P.n_cta_x; h->n_cta_p = P.n_cta_p; h->n_cta_r = P.n_cta_r;
   h->smem_x = P.smem_x; h->smem_p = P.smem_p;
+  h->bx = P.bx; h->bp = P.bp;
+  h->gx = P.gx; h->gx_nt = P.gx_nt; h->gx_smem = P.gx_smem;
+  h->gp_n = P.gp_n; h->gp_nt = P.gp_nt; h->gp_smem = P.gp_smem; h->gph_smem = P.gph_smem;
+  h->odm2 = P.odm2;
+  if (P.odm2) {
+    h->gox = d->n_p / P.oxr; h->gox_nt = P.oxr * (d->n_x / P.oe);
+    h->gop = d->n_x / P.opc; h->gop_nt = P.opc * (d->n_p / P.oe);
+  }
   h->odm = P.odm; h->smem_odm_x = P.smem_odm_x; h->smem_odm_p = P.smem_odm_p;
   const double dX = P.dX, dP = P.dP, dTheta = P.dTheta, dLambda = P.dLambda;
   const std::string& src = P.src;
@@ -567,8 +694,8 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
   h->tma = P.tma;
   if (P.rf) h->rf_c = P.rfpw * wig::rf_spw(NP);
   if (h->tma && !g_drv.encode) { delete h; return fail(WIG_ERR_CUDA, "cuTensorMapEncodeTiled unavailable (set WIG_TMA=0)"); }
-  if (!rc) rc = get_fn(mod, P.rf ? "wig_xpass_rf" : "wig_xpass", &h->f_x, h->smem_x);
-  if (!rc) rc = get_fn(mod, P.rf ? "wig_ppass_rf" : "wig_ppass", &h->f_p, h->smem_p);
+  if (!rc) rc = get_fn(mod, P.rf ? "wig_xpass_rf" : "wig_xpass", &h->f_x, P.gx_smem);
+  if (!rc) rc = get_fn(mod, P.rf ? "wig_ppass_rf" : "wig_ppass", &h->f_p, P.gp_smem);
   if (!rc) rc = get_fn(mod, "wig_reduce", &h->f_r, 0);
   if (!rc) rc = get_fn(mod, "wig_finalize", &h->f_fin, 0);
   if (!rc) rc = get_fn(mod, "wig_scale", &h->f_scale, 0);
@@ -578,11 +705,18 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
   if (!rc && h->odm) rc = get_fn(mod, "wig_odm_ppass", &h->f_op, h->smem_odm_p);
   h->strang = P.strang; h->gp = P.gp; h->smem_ph = P.smem_ph; h->smem_gph = P.smem_gph;
   h->n_chunks = NP / 16;
-  if (!rc && h->strang) rc = get_fn(mod, "wig_ppass_half", &h->f_ph, h->smem_ph);
-  if (!rc && h->strang) rc = get_fn(mod, "wig_ppass_half_final", &h->f_phf, h->smem_p);
+  if (!rc && h->strang) rc = get_fn(mod, "wig_ppass_half", &h->f_ph, h->gph_smem);
+  if (!rc && h->strang) rc = get_fn(mod, "wig_ppass_half_final", &h->f_phf, h->gp_smem);
   if (!rc && h->gp) rc = get_fn(mod, "wig_gp_colsum", &h->f_gcs, 0);
   if (!rc && h->gp) rc = get_fn(mod, "wig_gp_marginal", &h->f_gm, 0);
   if (!rc && h->gp) rc = get_fn(mod, "wig_gp_phase", &h->f_gph, h->smem_gph);
+  if (!rc && h->gp && h->bx && h->bp) {
+    h->gpb_n = (NP / 2 + P.bxr) / P.bxr;                 // rows 0 .. n_p / 2
+    h->gpb_smem = P.gx_smem + NX * (int)sizeof(double);
+    h->gpb_chunks = NP / std::min(NP, 64);
+    rc = get_fn(mod, "wig_gp_colsum_b", &h->f_gcb, 0);
+    if (!rc) rc = get_fn(mod, "wig_gp_phase_b", &h->f_gpb, h->gpb_smem);
+  }
   if (!rc && h->strang) rc = get_fn(mod, "wig_bloch_ppass", &h->f_bph, h->smem_ph);
   if (!rc && h->strang) rc = get_fn(mod, "wig_bloch_xpass", &h->f_bx, h->smem_x);
   if (!rc && h->strang) rc = get_fn(mod, "wig_bloch_reduce", &h->f_br, 0);
@@ -620,7 +754,7 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
   std::vector<double2> twx = twiddles(NX), twp = twiddles(NP);
   double *x_d, *p_d, *dv_d, *v0_d, *ths_d, *rl_d, *rt_d, *m1_d, *m2_d, *sfp_d, *part_d;
   double2 *twx_d, *twp_d;
-  const int nparts = std::max(std::max(h->n_cta_x, h->n_cta_p), h->n_cta_r);
+  const int nparts = std::max(std::max(h->n_cta_x, std::max(h->gp_n, h->gop)), h->n_cta_r);
   DevBuf& B = h->bufs;
   rc = B.alloc(&x_d, NX, xt.data());
   if (!rc) rc = B.alloc(&p_d, NP, pt.data());
@@ -640,7 +774,28 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
                                            : shifted_range(dLambda * NX / 2., NX);
   double* lam_d = nullptr;
   if (!rc) rc = B.alloc(&lam_d, NX, lt.data());
-  if (!rc && h->odm) rc = B.alloc(&h->odm_T, 5 * (size_t)NX * NP);
+  if (!rc && h->odm) rc = B.alloc(&h->odm_T, (h->odm2 ? 3 : 5) * (size_t)NX * NP);
+  double2 *bx_d = nullptr, *bp_d = nullptr, *box_d = nullptr, *bop_d = nullptr, *c2_d = nullptr, *ct_d = nullptr;
+  const auto upload_tw = [&](double2** dst, int n, int e) {
+    const std::vector<double2> tw = block_twiddles(n, e);
+    rc = B.alloc(dst, std::max<size_t>(tw.size(), 1), tw.empty() ? nullptr : tw.data());
+  };
+  if (!rc && h->bx) upload_tw(&bx_d, NX, P.bxe);
+  if (!rc && h->bp) upload_tw(&bp_d, NP, P.bpe);
+  if (!rc && h->odm2) {
+    upload_tw(&box_d, NX, P.oe);
+    if (!rc) upload_tw(&bop_d, NP, P.oe);
+    std::vector<double2> c2(NX), ct(NP);
+    for (int k = 0; k < NX; ++k) c2[k] = make_double2(cos(2. * xt[k]), sin(2. * xt[k]));
+    for (int k = 0; k < NP; ++k) {
+      const double th = ths[k] * (double)NP;   // the exact Theta (N_p a power of two)
+      ct[k] = make_double2(cos(d->hbar * th), sin(d->hbar * th));
+    }
+    if (!rc) rc = B.alloc(&c2_d, (size_t)NX, c2.data());
+    if (!rc) rc = B.alloc(&ct_d, (size_t)NP, ct.data());
+    h->btw_ox = box_d;
+    h->btw_op = bop_d;
+  }
   // ODM steps do not keep sum W real: the samples need the imaginary moment sums too
   double* part_im_d = nullptr;
   if (!rc && h->odm) rc = B.alloc(&part_im_d, (size_t)nparts * wig::NIM);
@@ -649,6 +804,8 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
   if (!rc && h->gp) rc = B.alloc(&h->gp_chunks, (size_t)h->n_chunks * NX);
   if (!rc && h->gp) rc = B.alloc(&h->gp_P, NX);
   if (!rc && h->gp) rc = B.alloc(&h->gp_phase, (size_t)NX * NP);
+  double2* colsum_d = nullptr;
+  if (!rc && h->f_gpb && !h->odm) rc = B.alloc(&colsum_d, (size_t)NX);
   if (!rc && h->strang) rc = B.alloc(&h->bloch_part, (size_t)h->n_cta_r * wig::NBL);
   if (!rc && h->strang) rc = B.alloc(&h->rowsums, (size_t)NP);
   if (!rc && h->gp) rc = B.alloc(&h->bloch_psq, (size_t)1);
@@ -663,6 +820,11 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
   if (rc) { B.free_all(); delete h; return rc; }
   a.rtw_x = rtwx_d;
   a.rtw_p = rtwp_d;
+  a.btw_x = bx_d;
+  a.btw_p = bp_d;
+  a.colsum = colsum_d;
+  a.cs2x = c2_d;
+  a.csth = ct_d;
   {
     int zero = 0;
     if (int rc2 = B.alloc(&h->status, (size_t)1, &zero)) { B.free_all(); delete h; return rc2; }
@@ -745,10 +907,20 @@ static int wig_run_begin(wig_handle* h, WigRunState* S, void* W_dev, int64_t t_i
   return WIG_OK;
 }
 
-// Gross-Pitaevskii phase of the current W into h->gp_phase: column sums, the
-// marginal (with the pending normalisation of scale_mode; psq_out may be null)
-// and the per-row phase.
-static int wig_gp_terms(wig_handle* h, WigRunState* S, int scale_mode, double* psq_out, cudaStream_t st) {
+// Gross-Pitaevskii phase of the current W into h->gp_phase: column sums (have_colsum: the
+// preceding final half p-pass left them in S->a.colsum), the marginal (with the pending
+// normalisation of scale_mode; psq_out may be null) and the per-row phase.
+static int wig_gp_terms(wig_handle* h, WigRunState* S, int scale_mode, double* psq_out, cudaStream_t st,
+                        bool have_colsum = false) {
+  if (h->f_gpb) {
+    const double2* ch = have_colsum ? S->a.colsum : h->gp_chunks;
+    int nch = have_colsum ? 1 : h->gpb_chunks;
+    void* cargs[] = {&S->W, &h->gp_chunks};
+    if (!have_colsum)
+      if (int rc = launch_after(h->f_gcb, (unsigned)(h->d.n_x / 32 * nch), 256, 0, st, cargs)) return rc;
+    void* pargs[] = {&S->a, &ch, &nch, &scale_mode, &h->gp_phase, &psq_out};
+    return launch_after(h->f_gpb, h->gpb_n, h->gx_nt, h->gpb_smem, st, pargs);
+  }
   const int NX = h->d.n_x, NP = h->d.n_p, cnt = NX < 256 ? NX : 256;
   void* cargs[] = {&S->W, &h->gp_chunks};   // grid: columns x row chunks of 16
   if (int rc = launch2d(h->f_gcs, (unsigned)(NX / cnt), (unsigned)(NP / 16), (unsigned)cnt, 0, st, cargs)) return rc;
@@ -757,6 +929,27 @@ static int wig_gp_terms(wig_handle* h, WigRunState* S, int scale_mode, double* p
   if (int rc = launch(h->f_gm, 1, 256, 0, st, margs)) return rc;
   void* pargs[] = {&S->a, &h->gp_P, &h->gp_phase};
   return launch(h->f_gph, h->n_cta_x, h->xnt, h->smem_gph, st, pargs);
+}
+
+// One first-order Lindblad (ODM) term on W: its x- and p-pass.
+static int wig_odm_term(wig_handle* h, WigRunState* S, double coef, double sign, cudaStream_t st) {
+  if (h->odm2) {
+    wig::WigArgs a = S->a;
+    a.btw_x = h->btw_ox;
+    a.btw_p = h->btw_op;
+    void* xargs[] = {&a, &S->W, &h->odm_T, &sign};
+    if (int rc = launch_after(h->f_ox, h->gox, h->gox_nt, h->smem_odm_x, st, xargs)) return rc;
+    void* pargs[] = {&a, &S->W, &h->odm_T, &coef};
+    if (int rc = launch_after(h->f_op, h->gop, h->gop_nt, h->smem_odm_p, st, pargs)) return rc;
+    S->a.n_partials = h->gop;
+    return WIG_OK;
+  }
+  void* xargs[] = {&S->a, &S->W, &h->odm_T};
+  if (int rc = launch(h->f_ox, h->n_cta_x, h->xnt, h->smem_odm_x, st, xargs)) return rc;
+  void* pargs[] = {&S->a, &S->W, &h->odm_T, &coef, &sign};
+  if (int rc = launch(h->f_op, h->n_cta_p, h->pnt, h->smem_odm_p, st, pargs)) return rc;
+  S->a.n_partials = h->n_cta_p;
+  return WIG_OK;
 }
 
 // One step of GPU_Wigner2D_GPitaevskii.Run (:1897-1975): [GP terms] half
@@ -771,28 +964,23 @@ static int wig_run_step_strang(wig_handle* h, WigRunState* S, int64_t n, cudaStr
   double* gph = h->gp ? h->gp_phase : nullptr;
   if (prof) WIG_CUDA(cudaEventRecord(h->ev[3 * n], st));
   if (h->gp)
-    if (int rc = wig_gp_terms(h, S, mode, nullptr, st)) return rc;
+    if (int rc = wig_gp_terms(h, S, mode, nullptr, st, n > 0 && S->a.colsum)) return rc;
   void* hargs[] = {&S->a, &S->W, &t, &mode, &obs_row, &gph};
-  if (int rc = launch(h->f_ph, h->n_cta_p, h->pnt, h->smem_ph, st, hargs)) return rc;
+  if (int rc = (h->bp ? launch_after : launch)(h->f_ph, h->gp_n + h->bp, h->gp_nt, h->gph_smem, st, hargs)) return rc;
   int zero = 0;
   double* none = nullptr;
   void* xargs[] = {&S->a, &S->W, &zero, &none};
-  if (int rc = launch(h->f_x, h->n_cta_x, h->xnt, h->smem_x, st, xargs)) return rc;
+  if (int rc = (h->bx ? launch_after : launch)(h->f_x, h->gx, h->gx_nt, h->gx_smem, st, xargs)) return rc;
   if (prof) WIG_CUDA(cudaEventRecord(h->ev[3 * n + 1], st));
   if (h->gp)
     if (int rc = wig_gp_terms(h, S, 0, h->psq + n, st)) return rc;
   void* fargs[] = {&S->a, &S->W, &t, &gph};
-  if (int rc = launch(h->f_phf, h->n_cta_p, h->pnt, h->smem_p, st, fargs)) return rc;
-  if (h->odm) {
-    // Lindbladian_ODM_Order1 with weight 1, sign 1 (GPU_Wigner2D_GPitaevskii.Run :1966-1969)
-    void* oxargs[] = {&S->a, &S->W, &h->odm_T};
-    if (int rc = launch(h->f_ox, h->n_cta_x, h->xnt, h->smem_odm_x, st, oxargs)) return rc;
-    double coef = h->odm_coef[0], sign = 1.;
-    void* opargs[] = {&S->a, &S->W, &h->odm_T, &coef, &sign};
-    if (int rc = launch(h->f_op, h->n_cta_p, h->pnt, h->smem_odm_p, st, opargs)) return rc;
-  }
+  if (int rc = (h->bp ? launch_after : launch)(h->f_phf, h->gp_n, h->gp_nt, h->gp_smem, st, fargs)) return rc;
+  S->a.n_partials = h->gp_n;
+  // Lindbladian_ODM_Order1 with weight 1, sign 1 (GPU_Wigner2D_GPitaevskii.Run :1966-1969)
+  if (h->odm)
+    if (int rc = wig_odm_term(h, S, h->odm_coef[0], 1., st)) return rc;
   if (prof) WIG_CUDA(cudaEventRecord(h->ev[3 * n + 2], st));
-  S->a.n_partials = h->n_cta_p;
   return WIG_OK;
 }
 
@@ -840,31 +1028,25 @@ static int wig_run_step(wig_handle* h, WigRunState* S, int64_t n, cudaStream_t s
   const bool prof = h->ev_used != 0;
   if (prof) WIG_CUDA(cudaEventRecord(h->ev[3 * n], st));
   void* xargs[] = {&S->a, &S->W, &mode, &obs_row};
-  if (int rc = launch(h->f_x, h->n_cta_x, h->xnt, h->smem_x, st, xargs)) return rc;
+  if (int rc = (h->bx ? launch_after : launch)(h->f_x, h->gx, h->gx_nt, h->gx_smem, st, xargs)) return rc;
   if (prof) WIG_CUDA(cudaEventRecord(h->ev[3 * n + 1], st));
   double t = (double)(S->t_index0 + n) * h->d.dt;
   if (h->rf) {
     if (h->tma && h->tmap_W != (const void*)S->W)
       if (int rc = encode_tile_map(h, S->W)) return rc;
     void* rargs[] = {&S->a, &S->W, &t, &h->tmap};
-    if (int rc = launch(h->f_p, h->n_cta_p, h->pnt, h->smem_p, st, rargs)) return rc;
+    if (int rc = launch(h->f_p, h->gp_n, h->gp_nt, h->gp_smem, st, rargs)) return rc;
   } else {
     void* pargs[] = {&S->a, &S->W, &t};
-    if (int rc = launch(h->f_p, h->n_cta_p, h->pnt, h->smem_p, st, pargs)) return rc;
+    if (int rc = (h->bp ? launch_after : launch)(h->f_p, h->gp_n, h->gp_nt, h->gp_smem, st, pargs)) return rc;
   }
-  if (h->odm) {
-    // Lindbladian_ODM_Order1 (:1637-1643); GPU_Wigner2D_ODM2 applies a damping
-    // (sign +1, weight1) then a pumping (sign -1, weight2) term (:2169-2176)
-    for (int j = 0; j < h->d.n_lindblad; ++j) {
-      void* oxargs[] = {&S->a, &S->W, &h->odm_T};
-      if (int rc = launch(h->f_ox, h->n_cta_x, h->xnt, h->smem_odm_x, st, oxargs)) return rc;
-      double coef = h->odm_coef[j], sign = h->odm_sign[j];
-      void* opargs[] = {&S->a, &S->W, &h->odm_T, &coef, &sign};
-      if (int rc = launch(h->f_op, h->n_cta_p, h->pnt, h->smem_odm_p, st, opargs)) return rc;
-    }
-  }
+  S->a.n_partials = h->gp_n;
+  // Lindbladian_ODM_Order1 (:1637-1643); GPU_Wigner2D_ODM2 applies a damping
+  // (sign +1, weight1) then a pumping (sign -1, weight2) term (:2169-2176)
+  if (h->odm)
+    for (int j = 0; j < h->d.n_lindblad; ++j)
+      if (int rc = wig_odm_term(h, S, h->odm_coef[j], h->odm_sign[j], st)) return rc;
   if (prof) WIG_CUDA(cudaEventRecord(h->ev[3 * n + 2], st));
-  S->a.n_partials = h->n_cta_p;
   return WIG_OK;
 }
 

@@ -190,6 +190,28 @@ template <bool INV, class C> __device__ __forceinline__ void dft16(C* v) {
   }
 }
 
+// 16-point DFT of the inputs v[4 a + b] w4^a w1^b (w4[a - 1], w1[b - 1] given): w4^a before the
+// radix-4 over a, w1^b after it.
+template <bool INV, class C> __device__ __forceinline__ void dft16_tw(C* v, const C* w4, const C* w1) {
+  C t[16];
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    C a0 = v[b], a1 = cmul(v[b + 4], w4[0]), a2 = cmul(v[b + 8], w4[1]), a3 = cmul(v[b + 12], w4[2]);
+    dft4<INV>(a0, a1, a2, a3);
+    t[b] = a0; t[b + 4] = a1; t[b + 8] = a2; t[b + 12] = a3;   // t[4 k1 + b]
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < 4; ++k1)
+#pragma unroll
+    for (int b = 1; b < 4; ++b) t[4 * k1 + b] = twc32<INV>(cmul(t[4 * k1 + b], w1[b - 1]), 2 * b * k1);
+#pragma unroll
+  for (int k1 = 0; k1 < 4; ++k1) {
+    C a0 = t[4 * k1], a1 = t[4 * k1 + 1], a2 = t[4 * k1 + 2], a3 = t[4 * k1 + 3];
+    dft4<INV>(a0, a1, a2, a3);
+    v[k1] = a0; v[k1 + 4] = a1; v[k1 + 8] = a2; v[k1 + 12] = a3;   // X[k1 + 4 k2]
+  }
+}
+
 // 32-point DFT: radix-2 decimation in time over two 16-point DFTs.
 template <bool INV, class C> __device__ __forceinline__ void dft32(C* v) {
   C e[16], o[16];
@@ -313,6 +335,228 @@ template <class C, int N, int NB, int NT, bool INV, class Map, int MAXR> struct 
 template <class C, int N, int NB, int NT, bool INV, class Map, int MAXR = 8>
 __device__ __forceinline__ void cta_fft(C* s, const C* __restrict__ tw) {
   FftRun<C, N, 1, NB, NT, INV, Map, MAXR>::run(s, tw);
+}
+
+// ---------------------------------------------------------------- register-blocked FFT
+// Stockham transform of one sequence of N elements held in the registers of
+// T = N / E threads: thread t holds v[m] = x[t + T m], on input and on output
+// (natural order both ways), so pointwise factors apply between transforms
+// without touching shared memory.  Only the stage boundaries go through shared
+// memory: one store and one load per element and boundary, against a store and a
+// load per stage and per pointwise factor of cta_fft.
+//
+// Every stage has radix E but one, which takes what is left: the second of three or
+// more (1024 = 16 4 16, 512 = 16 2 16 or 8 8 8, 256 = 8 4 8 or 4 4 4 4), where its
+// E / R butterflies share their twiddles, or the first of two (128 = 8 16).
+//
+// Twiddles.  The input r of a radix-16 butterfly carries w^{k r}, w = exp(-2 pi i /
+// (16 NS)); with r = 4 a + b the factor w^{4 k a} is applied before the butterfly's
+// first four 4-point DFTs (over a) and w^{k b} after them, so 6 table entries serve
+// a butterfly instead of 15: the loads, not the FP64 pipe, bound these passes
+// (shared + L1 wavefronts 75 % of peak, FP64 34 %, 1024^2 damped p-pass).
+// Table (host: wighost::block_twiddles), stage after stage (NS > 1), NS entries
+// each: radix 16: w^{4 k a}, a = 1..3, then w^{k b}, b = 1..3; radix R < 16: w^{k r},
+// r = 1..R - 1, w = exp(-2 pi i / (R NS)).  Entry k of one factor is next to k + 1:
+// the lanes of a warp read consecutive entries.  The inverse conjugates.
+//
+// Boundary after a stage (sub-length NS, radix R): consecutive threads store runs of
+// NS elements, NS R apart.  Element i lies at i + NS (i / (NS R)), which puts the runs
+// on distinct 16-byte bank groups (runs of 8 or more need no padding; below 8
+// elements a group, one pad per 8 does it; 4 elements' radix-2 stage is left
+// unpadded, its pads would be half the region); the loads stay consecutive.  The
+// indices of a boundary differ in disjoint bits, so slot(i + j) = slot(i) + slot(j):
+// one address and constant offsets.
+template <class C, int N, int E> struct BlockFft {
+  static constexpr int T = N / E;
+  static constexpr int REGION = N + N / (E < 8 ? E : 8);
+  static_assert(E >= 4 && E <= 16 && T >= 1 && (N & (N - 1)) == 0 && (E & (E - 1)) == 0, "BlockFft: powers of two");
+  // radix of the stage of sub-length ns
+  __host__ __device__ static constexpr int radix(int ns) {
+    int shrt = N;
+    while (shrt > E) shrt /= E;
+    const int at = N <= E * E ? 1 : E;   // the short stage's sub-length
+    return ns == at ? shrt : E;
+  }
+  template <int NS, int R> __device__ __forceinline__ static int slot(int i) {
+    if (NS >= 8 || (NS > 1 && R < 4)) return i;
+    return NS * R < 8 ? i + (i >> 3) : i + NS * (i / (NS * R));   // at most N / min(R, 8) pads
+  }
+
+  // s: the sequence's exchange region; sync() orders the T threads' accesses to it.
+  template <bool INV, class Sync>
+  __device__ __forceinline__ static void run(C (&v)[E], C* s, const C* __restrict__ tw, int t, const Sync& sync) {
+    stage<1, INV>(v, s, tw, t, sync);
+  }
+
+  // the stage of sub-length NS: butterflies t + T q, q < E / R
+  template <int NS, bool INV, class Sync>
+  __device__ __forceinline__ static void stage(C (&v)[E], C* s, const C* __restrict__ tw, int t, const Sync& sync) {
+    constexpr int R = radix(NS), Q = E / R;
+    static_assert(T % NS == 0, "a stage's butterflies share their twiddles");
+    const int k = t & (NS - 1);
+    if constexpr (NS > 1 && R == 16) {
+      C w4[3], w1[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        w4[a] = __ldg(tw + a * NS + k);
+        w1[a] = __ldg(tw + (3 + a) * NS + k);
+        if (INV) { w4[a] = cconj(w4[a]); w1[a] = cconj(w1[a]); }
+      }
+      dft16_tw<INV>(v, w4, w1);
+    } else {
+      C w[R];
+      if constexpr (NS > 1) {
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+          w[r] = __ldg(tw + (r - 1) * NS + k);
+          if (INV) w[r] = cconj(w[r]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        C u[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) u[r] = NS > 1 && r > 0 ? cmul(v[q + r * Q], w[r]) : v[q + r * Q];
+        dft_r<R, INV>(u);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[q + r * Q] = u[r];
+      }
+    }
+    if constexpr (NS * R < N) {
+      sync();   // the region's previous contents have been read
+      C* d = s + slot<NS, R>((t - k) * R + k);
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r) d[slot<NS, R>(T * q * R) + slot<NS, R>(r * NS)] = v[q + r * Q];
+      sync();
+      const C* g = s + slot<NS, R>(t);
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[m] = g[slot<NS, R>(T * m)];
+      stage<NS * R, INV>(v, s, tw + (NS > 1 ? (R == 16 ? 6 : R - 1) * NS : 0), t, sync);
+    }
+  }
+};
+
+// Barriers over the threads that share an exchange region.
+struct SyncWarp {
+  __device__ __forceinline__ void operator()() const { __syncwarp(); }
+};
+struct SyncCta {
+  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+// NTH threads (a multiple of 32) of the CTA, on a hardware barrier of their own
+template <int NTH> struct SyncGroup {
+  int id;
+  __device__ __forceinline__ void operator()() const {
+#ifdef __CUDA_ARCH__
+    asm volatile("bar.sync %0, %1;" ::"r"(id + 1), "n"(NTH) : "memory");
+#else
+    __syncthreads();   // host execution: one barrier for the block
+#endif
+  }
+};
+// The barrier of a sequence of T threads, `per_cta` sequences in the CTA (consecutive threads)
+template <int T, int PER_CTA> struct SeqSync {
+  __device__ __forceinline__ static auto make(int seq) {
+    if constexpr (T <= 32) return SyncWarp{};
+    else if constexpr (PER_CTA == 1) return SyncCta{};
+    else return SyncGroup<T>{seq};
+  }
+};
+
+// The pointer, opaque to the optimiser: loads through it are not moved out of the
+// loop that takes it (a rolled loop of transforms would otherwise keep every
+// twiddle and factor of an iteration in registers, and spill them).
+template <class P> __device__ __forceinline__ P* fresh(P* p) {
+#ifdef __CUDA_ARCH__
+  asm volatile("" : "+l"(p));
+#endif
+  return p;
+}
+
+// Tensor memory as a per-thread register file: NR 32-bit registers a thread, thread
+// l of warp w in lane 32 (w % 4) + l, columns from (w / 4) NR.  Used to keep the
+// Caldeira-Leggett base of a column out of registers and of the shared-memory
+// pipe, which bounds the pass.  alloc / release by every thread of the CTA (warp 0
+// acts); NR WARPS / 4 columns, a power of two in [32, 512]; the holders of an
+// allocation never wait for another CTA, so an alloc that finds the columns taken
+// waits for CTAs that run on.
+#if defined(WIG_TMEM) && defined(__CUDA_ARCH__)
+template <int NR, int WARPS> struct Tmem {
+  static constexpr int COLS = NR * ((WARPS + 3) / 4);
+  static_assert(NR % 16 == 0 && COLS >= 32 && COLS <= 512 && (COLS & (COLS - 1)) == 0, "tensor-memory columns");
+  unsigned base, mine;
+  __device__ __forceinline__ void alloc(unsigned* slot) {
+    if (threadIdx.x < 32) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(slot)),
+                   "n"(COLS)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    base = *slot;
+    const unsigned w = threadIdx.x >> 5;
+    mine = base + ((w & 3u) << 21) + (w >> 2) * NR;
+  }
+  __device__ __forceinline__ void release() {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (threadIdx.x < 32)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(COLS) : "memory");
+  }
+  // four double2 (16 registers) from column 16 q of the thread's slice
+  __device__ __forceinline__ void put(int q, const double2* v) const {
+    unsigned r[16];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      r[4 * i] = (unsigned)__double2loint(v[i].x);
+      r[4 * i + 1] = (unsigned)__double2hiint(v[i].x);
+      r[4 * i + 2] = (unsigned)__double2loint(v[i].y);
+      r[4 * i + 3] = (unsigned)__double2hiint(v[i].y);
+    }
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15, %16};" ::"r"(mine + 16 * q),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+  }
+  __device__ __forceinline__ static void put_done() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+  __device__ __forceinline__ void get(int q, double2* v) const {
+    unsigned r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+        "[%16];\n\ttcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(mine + 16 * q)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      v[i] = make_double2(__hiloint2double((int)r[4 * i + 1], (int)r[4 * i]),
+                          __hiloint2double((int)r[4 * i + 3], (int)r[4 * i + 2]));
+  }
+};
+#endif
+
+// Programmatic dependent launch: a kernel launched with the attribute may start
+// while its predecessor drains.  grid_wait() returns once the predecessor's
+// memory is visible (at once without the attribute); every thread calls it
+// before its first access to anything an earlier kernel writes.
+__device__ __forceinline__ void grid_wait() {
+#ifdef __CUDA_ARCH__
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void grid_launch_next() {
+#ifdef __CUDA_ARCH__
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
 }
 
 }  // namespace wig

@@ -34,6 +34,9 @@ int nvrtc_compile_locked(const std::string& src, std::vector<char>* cubin, std::
 int get_module(const std::string& src, int device, CUmodule* mod);
 int get_fn(CUmodule mod, const char* name, CUfunction* f, int dyn_smem);
 int launch(CUfunction f, unsigned grid, unsigned block, unsigned smem, cudaStream_t st, void** args);
+// The same with programmatic stream serialisation: the kernel may start while its predecessor in the
+// stream drains, and must call wig::grid_wait() before it reads or writes what an earlier kernel touches.
+int launch_after(CUfunction f, unsigned grid, unsigned block, unsigned smem, cudaStream_t st, void** args);
 int copy_log(const std::string& log, char* out, int64_t cap);
 // Blocks that can be resident per SM for a launch shape (1 when the query is unavailable).
 int occupancy(CUfunction f, int threads, int dyn_smem);

@@ -24,6 +24,33 @@
 #ifndef WIG_RF
 #define WIG_RF 0
 #endif
+// WIG_BX / WIG_BP 1: the x- / p-pass on the register-blocked transform: WIG_BXR rows / WIG_BPC columns
+// a CTA, WIG_BXE / WIG_BPE elements a thread, WIG_BXMB / WIG_BPMB CTAs per SM; WIG_BPA 1: the
+// p-pass's Caldeira-Leggett base in tensor memory (needs WIG_TMEM)
+#ifndef WIG_BX
+#define WIG_BX 0
+#endif
+#ifndef WIG_BP
+#define WIG_BP 0
+#endif
+#ifndef WIG_BPA
+#define WIG_BPA 0
+#endif
+// WIG_ODM 0: a plan without ODM damping (its kernels are not compiled); 2: ODM on the register-blocked
+// transforms, tiles WIG_OXR rows, WIG_OPC columns, WIG_OE elements a thread
+#ifndef WIG_ODM
+#define WIG_ODM 1
+#endif
+#if WIG_BX
+#define WIG_X_BOUNDS __launch_bounds__(WIG_BXR * (WIG_NX / WIG_BXE), WIG_BXMB)
+#else
+#define WIG_X_BOUNDS __launch_bounds__(WIG_XNT, WIG_XMINB)
+#endif
+#if WIG_BP
+#define WIG_P_BOUNDS __launch_bounds__(WIG_BPC * (WIG_NP / WIG_BPE), WIG_BPMB)
+#else
+#define WIG_P_BOUNDS __launch_bounds__(WIG_PNT, WIG_PMINB)
+#endif
 #include "wig_wigner.cuh"
 #include "wig_wigner_rf.cuh"
 
@@ -34,15 +61,25 @@ __device__ __forceinline__ UserPhys user_phys(const wig::WigArgs& a) {
   return ph;
 }
 
-extern "C" __global__ void __launch_bounds__(WIG_XNT, WIG_XMINB)
+extern "C" __global__ void WIG_X_BOUNDS
 wig_xpass(wig::WigArgs a, double2* W, int scale_mode, double* obs_row) {
+#if WIG_BX
+  wig::xpass_blk_body<UserPhys, WIG_NX, WIG_NP, WIG_BXR, WIG_BXE, WIG_KIN_STRING != 0>(a, user_phys(a), W,
+                                                                                        scale_mode, obs_row);
+#else
   wig::xpass_body<UserPhys, WIG_NX, WIG_NP, WIG_XROWS, WIG_XNT, WIG_KIN_STRING != 0>(
       a, user_phys(a), W, scale_mode, obs_row);
+#endif
 }
 
-extern "C" __global__ void __launch_bounds__(WIG_PNT, WIG_PMINB)
+extern "C" __global__ void WIG_P_BOUNDS
 wig_ppass(wig::WigArgs a, double2* W, double t) {
+#if WIG_BP
+  wig::ppass_blk_body<UserPhys, WIG_NX, WIG_NP, WIG_BPC, WIG_BPE, WIG_DAMP, WIG_KVN, 0, 1, WIG_BPA, WIG_ODM != 2>(
+      a, user_phys(a), W, t, a.partials);
+#else
   wig::ppass_body<UserPhys, WIG_NX, WIG_NP, WIG_PC, WIG_PNT, WIG_DAMP, WIG_KVN>(a, user_phys(a), W, t, a.partials);
+#endif
 }
 
 #if WIG_RF
@@ -68,19 +105,30 @@ wig_ppass_rf(wig::WigArgs a, double2* W, double t, const __grid_constant__ wig::
 // (consumes the previous partials, normalises on load, records the sample),
 // then -- after the kinetic x-pass -- the final half p-pass with the damping
 // and the partial sums.  gp_phase: the Gross-Pitaevskii phase array or null.
-extern "C" __global__ void __launch_bounds__(WIG_PNT, WIG_PMINB)
+extern "C" __global__ void WIG_P_BOUNDS
 wig_ppass_half(wig::WigArgs a, double2* W, double t, int scale_mode, double* obs_row, const double* gp_phase) {
+#if WIG_BP
+  wig::ppass_blk_body<UserPhys, WIG_NX, WIG_NP, WIG_BPC, WIG_BPE, 0, 0, 1, 0, WIG_BPA>(
+      a, user_phys(a), W, t, a.partials, scale_mode, obs_row, gp_phase);
+#else
   wig::ppass_body<UserPhys, WIG_NX, WIG_NP, WIG_PC, WIG_PNT, 0, 0, 1, 0>(a, user_phys(a), W, t, a.partials,
                                                                         scale_mode, obs_row, gp_phase);
+#endif
 }
 
-extern "C" __global__ void __launch_bounds__(WIG_PNT, WIG_PMINB)
+extern "C" __global__ void WIG_P_BOUNDS
 wig_ppass_half_final(wig::WigArgs a, double2* W, double t, const double* gp_phase) {
+#if WIG_BP
+  wig::ppass_blk_body<UserPhys, WIG_NX, WIG_NP, WIG_BPC, WIG_BPE, WIG_DAMP, 0, 1, 1, WIG_BPA, WIG_ODM != 2>(
+      a, user_phys(a), W, t, a.partials, 0, nullptr, gp_phase);
+#else
   wig::ppass_body<UserPhys, WIG_NX, WIG_NP, WIG_PC, WIG_PNT, WIG_DAMP, 0, 1, 1>(a, user_phys(a), W, t, a.partials,
                                                                                 0, nullptr, gp_phase);
+#endif
 }
 
 #define WIG_GP_RCH 16
+#define WIG_GP_RCHB (WIG_NP < 64 ? WIG_NP : 64)   // rows a chunk of wig_gp_colsum_b
 #define WIG_GP_CNT (WIG_NX < 256 ? WIG_NX : 256)
 extern "C" __global__ void __launch_bounds__(WIG_GP_CNT)
 wig_gp_colsum(const double2* W, double2* chunks) {
@@ -96,6 +144,19 @@ extern "C" __global__ void __launch_bounds__(WIG_XNT)
 wig_gp_phase(wig::WigArgs a, const double* P, double* phase_out) {
   wig::gp_phase_body<WIG_NX, WIG_NP, WIG_XROWS, WIG_XNT>(a, P, phase_out);
 }
+
+#if WIG_BX
+// the Strang step's Gross-Pitaevskii terms on the register-blocked transform
+extern "C" __global__ void __launch_bounds__(256)
+wig_gp_colsum_b(const double2* W, double2* chunks) {
+  wig::colsum_blk_body<WIG_NX, WIG_NP, WIG_GP_RCHB>(W, chunks);
+}
+
+extern "C" __global__ void WIG_X_BOUNDS
+wig_gp_phase_b(wig::WigArgs a, const double2* chunks, int n_chunks, int scale_mode, double* phase_out, double* psq) {
+  wig::gp_phase_blk_body<WIG_NX, WIG_NP, WIG_BXR, WIG_BXE>(a, chunks, n_chunks, scale_mode, phase_out, psq);
+}
+#endif
 
 // Bloch (imaginary-time) step pieces, GPU_Wigner2D_GPitaevskii_Bloch (:2064-2545)
 extern "C" __global__ void __launch_bounds__(WIG_PNT, WIG_PMINB)
@@ -144,6 +205,17 @@ wig_scale(double2* W, long n, const double2* s) {
   wig::scale_body<WIG_RNT>(W, n, s);
 }
 
+#if WIG_ODM == 2
+extern "C" __global__ void __launch_bounds__(WIG_OXR * (WIG_NX / WIG_OE), WIG_OXMB)
+wig_odm_xpass(wig::WigArgs a, const double2* W, double2* R, double sign) {
+  wig::odm_xpass_blk_body<UserPhys, WIG_NX, WIG_NP, WIG_OXR, WIG_OE>(a, user_phys(a), W, R, sign);
+}
+
+extern "C" __global__ void __launch_bounds__(WIG_OPC * (WIG_NP / WIG_OE), WIG_OPMB)
+wig_odm_ppass(wig::WigArgs a, double2* W, const double2* R, double coef) {
+  wig::odm_ppass_blk_body<WIG_NX, WIG_NP, WIG_OPC, WIG_OE>(a, W, R, coef);
+}
+#elif WIG_ODM == 1
 extern "C" __global__ void __launch_bounds__(WIG_XNT)
 wig_odm_xpass(wig::WigArgs a, const double2* W, double2* T) {
   wig::odm_xpass_body<UserPhys, WIG_NX, WIG_NP, WIG_XROWS, WIG_XNT>(a, user_phys(a), W, T);
@@ -153,6 +225,7 @@ extern "C" __global__ void __launch_bounds__(WIG_PNT)
 wig_odm_ppass(wig::WigArgs a, double2* W, const double2* T, double coef, double sign) {
   wig::odm_ppass_body<WIG_NX, WIG_NP, WIG_PC, WIG_PNT>(a, W, T, coef, sign);
 }
+#endif
 
 // Per-instance 1-D factor tables, computed on the device with the same
 // expressions (and CUDA math) as the reference's kernels:

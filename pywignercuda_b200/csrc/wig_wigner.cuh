@@ -76,6 +76,13 @@ struct WigArgs {
   const double2* rtw_x;
   const double2* rtw_p;
   int* status;              // [1] set to 1 by a bounded wait that gave up (read and cleared by the host)
+  // stage twiddles of the register-blocked passes (BlockFft); null when the plan uses the Stockham ones
+  const double2* btw_x;
+  const double2* btw_p;
+  // ODM on the register-blocked passes: (cos, sin) of 2 X [n_x] and of hbar Theta [n_p]
+  const double2* cs2x;
+  const double2* csth;
+  double2* colsum;          // [n_x] column sums of W left by the final half p-pass (Gross-Pitaevskii); may be null
 };
 
 // ------------------------------------------------------------------ reductions
@@ -746,5 +753,503 @@ __device__ __forceinline__ void odm_ppass_body(const WigArgs& a, double2* __rest
   if (with_im) store_partials_im<NT>(a, im, red);
 }
 
-}  // namespace wig
+// ------------------------------------------------------------------ register-blocked passes
+// The passes of axes of at least 64 points on BlockFft (wig_fft.cuh): a thread
+// holds E elements of its row or column from the global load to the global
+// store; shared memory carries only the transforms' stage boundaries.
+//
+// Pointwise factors exp(-i phase) are odd in the phase's frequency (lambda or
+// theta: exact, the two coordinates differ in sign only), so a sequence's
+// threads evaluate them for k <= N/2, hand them round through the exchange
+// region and take the conjugate at N - k: half the sincos and half the
+// evaluations of the user's expressions.  k = N/2 is evaluated like the others.
 
+// factor(k) for this thread's elements t + T m, applied to v; s: the exchange region
+template <int N, int E, class Sync, class Factor>
+__device__ __forceinline__ void apply_odd_factor(double2 (&v)[E], double2* s, int t, const Sync& sync,
+                                                 const Factor& factor) {
+  constexpr int T = N / E;
+  sync();   // the region's previous contents have been read
+#pragma unroll 2
+  for (int k = t; k <= N / 2; k += T) s[k] = factor(k);
+  sync();
+#pragma unroll
+  for (int m = 0; m < E; ++m) {
+    const int k = t + T * m;
+    const double2 f = k <= N / 2 ? s[k] : cconj(s[N - k]);
+    v[m] = cmul(v[m], f);
+  }
+}
+
+// x-pass: ROWS rows per CTA, NX / E threads per row; the last CTA of the grid
+// (block NP / ROWS) only records the previous pass's sample, so that no row's
+// CTA waits for that reduction.  Shared memory: ROWS exchange regions.
+template <class Phys, int NX, int NP, int ROWS, int E, bool KIN_STRING>
+__device__ __forceinline__ void xpass_blk_body(const WigArgs& a, const Phys& ph, double2* __restrict__ W,
+                                               int scale_mode, double* obs_row) {
+  typedef BlockFft<double2, NX, E> F;
+  constexpr int T = F::T, NT = ROWS * T;
+  static_assert(NT % 32 == 0 && (T % 32 == 0 || 32 % T == 0), "x-pass rows per CTA");
+  extern __shared__ double2 sm[];
+  __shared__ double red[NT / 32][NACC];
+  grid_wait();
+  grid_launch_next();
+  if (blockIdx.x == NP / ROWS) {
+    if (obs_row != nullptr) consume_partials<NT>(a, scale_mode, obs_row, red);
+    return;
+  }
+  const int seq = threadIdx.x / T, t = threadIdx.x % T, row = blockIdx.x * ROWS + seq;
+  WIG_BOUNDS_CHECK("x-pass row", row, NP);
+  double2* Wr = W + (size_t)row * NX;
+  double2 v[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) v[m] = Wr[t + T * m];
+  if (scale_mode != 0) {
+    const double2 s = consume_partials<NT>(a, scale_mode, nullptr, red);
+#pragma unroll
+    for (int m = 0; m < E; ++m) v[m] = cmul(v[m], s);
+  }
+  double2* X = sm + seq * F::REGION;
+  const auto sync = SeqSync<T, ROWS>::make(seq);
+  F::template run<false>(v, X, a.btw_x, t, sync);
+  const int ii = (row + NP / 2) % NP;
+  const double p = a.dp * (ii - 0.5 * NP);
+  const double inv_n = 1.0 / (double)NX;
+  apply_odd_factor<NX, E>(v, X, t, sync, [&](int k) {
+    const int jj = (k + NX / 2) % NX;
+    const double lambda = a.dlambda * (jj - 0.5 * NX);
+    double phase;
+    if (KIN_STRING)
+      phase = a.dt * ((ph.KineticEnergy(p + a.hbar * lambda / 2.) -
+                       ph.KineticEnergy(p - a.hbar * lambda / 2.)) / a.hbar);
+    else
+      phase = a.dt * lambda * p / a.mass;
+    const double rr = __ldg(a.r_lambda + k) * inv_n;
+    double sn, cs;
+    sincos(phase, &sn, &cs);
+    return make_double2(rr * cs, -rr * sn);
+  });
+  F::template run<true>(v, X, a.btw_x, t, sync);
+#pragma unroll
+  for (int m = 0; m < E; ++m) Wr[t + T * m] = v[m];
+}
+
+// Exchange-region stride of a tile of C columns: lanes walk the columns first, so
+// the regions are offset by 8 / C sixteen-byte bank groups.
+__host__ __device__ constexpr int blk_stride(int region, int c) {
+  return c >= 8 ? region | 1 : region + ((8 / c - region % 8) % 8 + 8) % 8;
+}
+
+// Per-CTA observable partials from per-column moments: a thread's elements lie
+// in one column (c = threadIdx.x % C), so it sums w, Im w, w p, w p^2 and the
+// negative part, the threads of a column are combined, and the functions of x
+// enter once per column.
+template <int C, int NT, int NM>
+__device__ __forceinline__ void column_moments(double (&mom)[NM], double (*red)[C][NM]) {
+  static_assert(C <= 32, "columns within a warp");
+#pragma unroll
+  for (int q = 0; q < NM; ++q) {
+#pragma unroll
+    for (int o = 16; o >= C; o >>= 1) mom[q] += __shfl_xor_sync(0xffffffffu, mom[q], o);
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane < C) {
+#pragma unroll
+    for (int q = 0; q < NM; ++q) red[warp][lane][q] = mom[q];
+  }
+  __syncthreads();
+}
+
+// Sum over the CTA's columns of observable slot v of `partials` (accumulate_obs),
+// from the moments m0 (sum of w), m1 (w p), m2 (w p^2) of `base`; im: slots of
+// accumulate_obs_im instead (base: the moments of Im w, then of the negative part).
+template <int C, int NW, int NM>
+__device__ __forceinline__ double column_observable(const WigArgs& a, double (*red)[C][NM], int v, int col0, int im) {
+  double total = 0.;
+  for (int c = 0; c < C; ++c) {
+    double m[NM];
+#pragma unroll
+    for (int q = 0; q < NM; ++q) {
+      double s = 0.;
+      for (int w = 0; w < NW; ++w) s += red[w][c][q];
+      m[q] = s;
+    }
+    const double x = a.x_tab[col0 + c], dv = a.dV_tab[col0 + c], v0 = a.V0_tab[col0 + c];
+    // m: Re w [0], w p [2], w p^2 [3], negative [4]; Im w [1], then (ODM) Im w p [5], Im w p^2 [6], Im of the negative [7]
+    const double s0 = im ? m[1] : m[0], s1 = im ? m[NM > 5 ? 5 : 2] : m[2], s2 = im ? m[NM > 6 ? 6 : 3] : m[3];
+    const int slot = im ? v + 2 : v;
+    double f;
+    switch (slot) {
+      case 0: f = m[0]; break;
+      case 1: f = m[1]; break;
+      case 2: f = s0 * x; break;
+      case 3: f = s0 * (x * x); break;
+      case 4: f = s1; break;
+      case 5: f = s2; break;
+      case 6: f = s1 * x; break;
+      case 7: f = s0 * dv; break;
+      case 8: f = s1 * dv; break;
+      case 9: f = s0 * (dv * x); break;
+      case 10: f = s2 / (2. * a.mass_exact) + s0 * v0; break;
+      default: f = im ? m[NM > 7 ? 7 : 4] : m[4]; break;
+    }
+    total += f;
+  }
+  return total;
+}
+
+// p-pass: a tile of C columns per CTA, NP / E threads per column (column =
+// threadIdx.x % C: the C * 16 bytes of a grid row are one segment).  Flags as
+// ppass_body; OBS 0 leaves the partial sums out (plans whose damping passes
+// write them).  The Caldeira-Leggett base A is kept in registers (TM 0) or, where a
+// thread's E elements leave no room for a second set, in tensor memory (TM 1).
+// Shared memory: C exchange regions.  gp_phase rows theta <= N_p / 2 are read (odd in theta).
+// With scale_mode or obs_row (Strang) the last CTA (block NX / C) only records
+// the sample, as in the x-pass.
+template <class Phys, int NX, int NP, int C, int E, int DAMP, int KVN = 0, int HALF = 0, int FINAL = 1, int TM = 0,
+          int OBS = 1>
+__device__ __forceinline__ void ppass_blk_body(const WigArgs& a, const Phys& ph, double2* __restrict__ W, double t,
+                                               double* __restrict__ partials, int scale_mode = 0,
+                                               double* obs_row = nullptr,
+                                               const double* __restrict__ gp_phase = nullptr) {
+  typedef BlockFft<double2, NP, E> F;
+  constexpr int T = F::T, NT = C * T, RS = blk_stride(F::REGION, C);
+  static_assert(NT % 32 == 0 && C <= 32, "p-pass columns per CTA");
+  extern __shared__ double2 sm[];
+  grid_wait();
+  grid_launch_next();
+  if (FINAL == 0) {
+    __shared__ double red[NT / 32][NACC];
+    if (blockIdx.x == NX / C) {
+      if (obs_row != nullptr) consume_partials<NT>(a, scale_mode, obs_row, red);
+      return;
+    }
+  }
+  const int c = threadIdx.x % C, th = threadIdx.x / C, col = blockIdx.x * C + c;
+  WIG_BOUNDS_CHECK("p-pass tile column", col, NX);
+  double2* Wc = W + (size_t)th * NX + col;
+  double2 v[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) v[m] = Wc[(size_t)(T * m) * NX];
+  if (FINAL == 0 && scale_mode != 0) {
+    __shared__ double red2[NT / 32][NACC];
+    const double2 s = consume_partials<NT>(a, scale_mode, nullptr, red2);
+#pragma unroll
+    for (int m = 0; m < E; ++m) v[m] = cmul(v[m], s);
+  }
+  double2* X = sm + c * RS;
+  const auto sync = SeqSync<NT, 1>::make(0);
+  const int jj = (col + NX / 2) % NX;
+  const double x = a.dx * (jj - 0.5 * NX);
+  const double mask = a.mask1[col] * a.mask2s[col];
+  double2 A[E];   // unused with TM
+  // it 0: the potential factor; 1..3 (Caldeira-Leggett): A + c3 D(A + c12 D(A + c1 D A)),
+  // D = IFFT_p[theta FFT_p(sign(p) f(p) .)] / n_p, the c's imaginary.  One rolled loop, so the
+  // kernel holds one copy of each transform.
+  constexpr int N_IT = DAMP == 1 && FINAL ? 4 : 1;
+#ifdef WIG_TMEM
+  __shared__ unsigned tm_slot;
+  Tmem<TM ? 4 * E : 64, NT / 32> tm;
+  if constexpr (TM && N_IT > 1) tm.alloc(&tm_slot);
+#endif
+#pragma unroll 1
+  for (int it = 0; it < N_IT; ++it) {
+    if (it > 0) {
+      const double* sfp = fresh(a.sfp + th);
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[m] = cscale(v[m], __ldg(sfp + T * m));
+    }
+    F::template run<false>(v, X, fresh(a.btw_p), th, sync);
+    if (it == 0) {
+      apply_odd_factor<NP, E>(v, X, th, sync, [&](int k) {
+        const int ii = (k + NP / 2) % NP;
+        const double theta = a.dtheta * (ii - 0.5 * NP);
+        double phase = KVN ? a.dt * (-ph.DPotential(t, x) * theta)
+                           : (HALF ? 0.5 * a.dt : a.dt) * ((ph.Potential(t, x - a.hbar * theta / 2.) -
+                                                            ph.Potential(t, x + a.hbar * theta / 2.)) / a.hbar);
+        if (HALF && gp_phase != nullptr) phase -= gp_phase[(size_t)k * NX + col];
+        const double r = __ldg((HALF ? a.r_theta_half : a.r_theta) + k) * mask;
+        double sn, cs;
+        sincos(phase, &sn, &cs);
+        return make_double2(r * cs, -r * sn);
+      });
+    } else {
+      const double* ths = fresh(a.theta_s + th);
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[m] = cscale(v[m], __ldg(ths + T * m));
+    }
+    F::template run<true>(v, X, fresh(a.btw_p), th, sync);
+    if (it > 0) {
+      const double cf = it == 1 ? a.cl_k1.y : (it == 2 ? a.cl_k12.y : a.cl_c3.y);
+#ifdef WIG_TMEM
+      if constexpr (TM) {
+#pragma unroll
+        for (int m = 0; m < E; m += 4) {
+          double2 At[4];
+          tm.get(m / 4, At);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            v[m + i] = make_double2(At[i].x - cf * v[m + i].y, At[i].y + cf * v[m + i].x);
+        }
+        continue;
+      }
+#endif
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[m] = make_double2(A[m].x - cf * v[m].y, A[m].y + cf * v[m].x);
+    } else if (N_IT > 1) {
+#ifdef WIG_TMEM
+      if constexpr (TM) {
+#pragma unroll
+        for (int m = 0; m < E; m += 4) tm.put(m / 4, &v[m]);
+        tm.put_done();
+        continue;
+      }
+#endif
+#pragma unroll
+      for (int m = 0; m < E; ++m) A[m] = v[m];
+    }
+  }
+#ifdef WIG_TMEM
+  if constexpr (TM && N_IT > 1) tm.release();
+#endif
+  double2* Wo = fresh(Wc);
+#pragma unroll
+  for (int m = 0; m < E; ++m) Wo[(size_t)(T * m) * NX] = v[m];
+  if (FINAL && OBS) {
+    __shared__ double red5[NT / 32][C][5];
+    double mom[5] = {0., 0., 0., 0., 0.};
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      const double p = __ldg(a.p_tab + th + T * m), wp = v[m].x * p;
+      mom[0] += v[m].x;
+      mom[1] += v[m].y;
+      mom[2] += wp;
+      mom[3] = fma(wp, p, mom[3]);
+      mom[4] += v[m].x < 0. ? v[m].x : 0.;
+    }
+    column_moments<C, NT, 5>(mom, red5);
+    if (HALF && a.colsum != nullptr && threadIdx.x < C) {
+      double2 s = make_double2(0., 0.);
+      for (int w = 0; w < NT / 32; ++w) { s.x += red5[w][threadIdx.x][0]; s.y += red5[w][threadIdx.x][1]; }
+      a.colsum[blockIdx.x * C + threadIdx.x] = s;
+    }
+    if (threadIdx.x < NACC)
+      partials[(size_t)blockIdx.x * NACC + threadIdx.x] =
+          column_observable<C, NT / 32, 5>(a, red5, threadIdx.x, blockIdx.x * C, 0);
+  }
+}
+
+// ODM Lindblad passes (odm_xpass_body / odm_ppass_body) with the trigonometric
+// factors split by cos a cos b = (cos(a + b) + cos(a - b)) / 2 and its kin,
+// a + b = 2 X, a - b = hbar Theta: with T_k = IFFT_x[FFT_x(W) G_k] / n_x the sum is
+//   cos(2X)/2 (T0 - T3) + i s sin(2X)/2 (T1 - T2) + T4           a function of x: R0
+//   + cos(hbar Theta) (T0 + T3)/2 + sin(hbar Theta) i s (T1 + T2)/2     R1, R2
+// so the x-pass leaves three planes instead of five and the p-pass transforms
+// three columns instead of five.  g(p + hbar lambda / 2) is evaluated once per
+// point (g(p - hbar lambda / 2) is its value at -lambda) instead of twice per term.
+// Shared memory of the x-pass: ROWS regions, then ROWS (NX + 1) doubles (g).
+template <class Phys, int NX, int NP, int ROWS, int E>
+__device__ __forceinline__ void odm_xpass_blk_body(const WigArgs& a, const Phys& ph, const double2* __restrict__ W,
+                                                   double2* __restrict__ R, double sign) {
+  typedef BlockFft<double2, NX, E> F;
+  constexpr int T = F::T, NT = ROWS * T;
+  static_assert(NT % 32 == 0 && (T % 32 == 0 || 32 % T == 0), "ODM x-pass rows per CTA");
+  extern __shared__ double2 sm[];
+  const int seq = threadIdx.x / T, t = threadIdx.x % T, row = blockIdx.x * ROWS + seq;
+  WIG_BOUNDS_CHECK("ODM x-pass row", row, NP);
+  double2* X = sm + seq * F::REGION;
+  double* g = reinterpret_cast<double*>(sm + ROWS * F::REGION) + seq * (NX + 1);
+  const auto sync = SeqSync<T, ROWS>::make(seq);
+  const double p = a.p_tab[row];
+#pragma unroll 2
+  for (int k = t; k < NX; k += T) g[k] = odm_g(a, ph, p + 0.5 * a.hbar_exact * a.lambda_tab[k]);
+  if (t == 0) g[NX] = odm_g(a, ph, p - 0.5 * a.hbar_exact * a.lambda_tab[NX / 2]);
+  grid_wait();
+  grid_launch_next();
+  const size_t plane = (size_t)NX * NP, base = (size_t)row * NX;
+  double2 f[E], r0[E], v[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) f[m] = W[base + t + T * m];
+  F::template run<false>(f, X, a.btw_x, t, sync);
+  const double inv_n = 1.0 / (double)NX;
+  sync();   // g is complete
+  // term 0: G1 - G2, 1: G0 - G3, 2: G4, 3: G0 + G3, 4: G1 + G2
+#pragma unroll 1
+  for (int term = 0; term < 5; ++term) {
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      const int k = t + T * m;
+      const double lam = a.lambda_tab[k], gp = g[k], gm = g[k == 0 ? 0 : (k == NX / 2 ? NX : NX - k)];
+      const double sp = sgn(p + 0.5 * a.hbar_exact * lam), sn = sgn(p - 0.5 * a.hbar_exact * lam), gg = gp * gm;
+      double q;
+      if (term == 0) q = gg * (sn - sp);
+      else if (term == 1) q = gg * (1. - sp * sn);
+      else if (term == 2) q = -0.5 * gp * gp - 0.5 * gm * gm;
+      else if (term == 3) q = gg * (1. + sp * sn);
+      else q = gg * (sn + sp);
+      v[m] = cscale(f[m], q * inv_n);
+    }
+    F::template run<true>(v, X, fresh(a.btw_x), t, sync);
+    const double2* c2 = fresh(a.cs2x + t);
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      const double2 cs = __ldg(c2 + T * m);
+      if (term == 0) {
+        const double h = 0.5 * sign * cs.y;
+        r0[m] = make_double2(-h * v[m].y, h * v[m].x);
+      } else if (term == 1) {
+        r0[m] = make_double2(r0[m].x + 0.5 * cs.x * v[m].x, r0[m].y + 0.5 * cs.x * v[m].y);
+      } else if (term == 2) {
+        R[base + t + T * m] = cadd(r0[m], v[m]);
+      } else if (term == 3) {
+        R[plane + base + t + T * m] = cscale(v[m], 0.5);
+      } else {
+        const double h = 0.5 * sign;
+        R[2 * plane + base + t + T * m] = make_double2(-h * v[m].y, h * v[m].x);
+      }
+    }
+  }
+}
+
+// W <- W + coef IFFT_p[FFT_p(R0) + cos(hbar Theta) FFT_p(R1) + sin(hbar Theta) FFT_p(R2)], then the
+// observable sums with their imaginary parts.  Shared memory: C exchange regions.
+template <int NX, int NP, int C, int E>
+__device__ __forceinline__ void odm_ppass_blk_body(const WigArgs& a, double2* __restrict__ W,
+                                                   const double2* __restrict__ R, double coef) {
+  typedef BlockFft<double2, NP, E> F;
+  constexpr int T = F::T, NT = C * T, RS = blk_stride(F::REGION, C);
+  static_assert(NT % 32 == 0 && C <= 32, "ODM p-pass columns per CTA");
+  extern __shared__ double2 sm[];
+  __shared__ double red8[NT / 32][C][8];
+  grid_wait();
+  grid_launch_next();
+  const int c = threadIdx.x % C, th = threadIdx.x / C, col = blockIdx.x * C + c;
+  WIG_BOUNDS_CHECK("ODM p-pass tile column", col, NX);
+  double2* X = sm + c * RS;
+  const auto sync = SeqSync<NT, 1>::make(0);
+  const size_t plane = (size_t)NX * NP;
+  double2 acc[E], v[E];
+#pragma unroll 1
+  for (int q = 0; q < 3; ++q) {
+    const double2* Rc = R + q * plane + col;
+#pragma unroll
+    for (int m = 0; m < E; ++m) v[m] = Rc[(size_t)(th + T * m) * NX];
+    F::template run<false>(v, X, fresh(a.btw_p), th, sync);
+    const double2* ct = fresh(a.csth + th);
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      const double2 cs = __ldg(ct + T * m);
+      if (q == 0) acc[m] = v[m];
+      else {
+        const double f = q == 1 ? cs.x : cs.y;
+        acc[m] = make_double2(fma(f, v[m].x, acc[m].x), fma(f, v[m].y, acc[m].y));
+      }
+    }
+  }
+  F::template run<true>(acc, X, a.btw_p, th, sync);
+  double mom[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
+#pragma unroll
+  for (int m = 0; m < E; ++m) {
+    double2* Wp = W + (size_t)(th + T * m) * NX + col;
+    const double2 w = cadd(*Wp, cscale(acc[m], coef));
+    *Wp = w;
+    const double p = __ldg(a.p_tab + th + T * m);
+    mom[0] += w.x;
+    mom[1] += w.y;
+    mom[2] += w.x * p;
+    mom[3] += w.x * (p * p);
+    mom[5] += w.y * p;
+    mom[6] += w.y * (p * p);
+    if (w.x < 0.) { mom[4] += w.x; mom[7] += w.y; }
+  }
+  column_moments<C, NT, 8>(mom, red8);
+  if (threadIdx.x < NACC) {
+    const int v_ = threadIdx.x, col0 = blockIdx.x * C;
+    a.partials[(size_t)blockIdx.x * NACC + v_] = column_observable<C, NT / 32, 8>(a, red8, v_, col0, 0);
+    if (a.partials_im && v_ < NIM)
+      a.partials_im[(size_t)blockIdx.x * NIM + v_] = column_observable<C, NT / 32, 8>(a, red8, v_, col0, 1);
+  }
+}
+
+// Column sums of W over chunks of RCH rows: out[chunk][x], 32 columns x RCH / 8 rows a
+// thread group (grid NX / 32 x NP / RCH, 256 threads).
+template <int NX, int NP, int RCH>
+__device__ __forceinline__ void colsum_blk_body(const double2* __restrict__ W, double2* __restrict__ out) {
+  __shared__ double2 part[8][33];
+  grid_wait();
+  grid_launch_next();
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int nxb = NX / 32, bx = blockIdx.x % nxb, by = blockIdx.x / nxb;
+  const double2* w = W + (size_t)(by * RCH + g) * NX + bx * 32 + lane;
+  double2 s = make_double2(0., 0.);
+#pragma unroll
+  for (int r = 0; r < RCH / 8; ++r) s = cadd(s, w[(size_t)(8 * r) * NX]);
+  part[g][lane] = s;
+  __syncthreads();
+  if (g == 0) {
+#pragma unroll
+    for (int q = 1; q < 8; ++q) s = cadd(s, part[q][lane]);
+    out[(size_t)by * NX + bx * 32 + lane] = s;
+  }
+}
+
+// Gross-Pitaevskii phase rows theta <= N_p / 2 (gp_phase_body; the phase is odd in theta): the
+// marginal P(x) from the chunk sums with the pending normalisation of scale_mode, its spectrum
+// once per row group, and per row one inverse transform.  psq (may be null) as gp_marginal_body.
+// Shared memory: ROWS exchange regions, then N_x doubles.
+template <int NX, int NP, int ROWS, int E>
+__device__ __forceinline__ void gp_phase_blk_body(const WigArgs& a, const double2* __restrict__ chunks, int n_chunks,
+                                                  int scale_mode, double* __restrict__ phase_out,
+                                                  double* __restrict__ psq) {
+  typedef BlockFft<double2, NX, E> F;
+  constexpr int T = F::T, NT = ROWS * T;
+  static_assert(NT % 32 == 0 && (T % 32 == 0 || 32 % T == 0), "phase rows per CTA");
+  extern __shared__ double2 sm[];
+  __shared__ double red[NT / 32][NACC];
+  const int seq = threadIdx.x / T, t = threadIdx.x % T, row = blockIdx.x * ROWS + seq;
+  double2* X = sm + seq * F::REGION;
+  double* Ps = reinterpret_cast<double*>(sm + ROWS * F::REGION);
+  const auto sync = SeqSync<T, ROWS>::make(seq);
+  grid_wait();
+  grid_launch_next();
+  double2 s = make_double2(1., 0.);
+  if (scale_mode != 0) s = consume_partials<NT>(a, scale_mode, nullptr, red);
+  double acc[1] = {0.};
+  for (int x = threadIdx.x; x < NX; x += NT) {
+    double2 c = make_double2(0., 0.);
+    for (int q = 0; q < n_chunks; ++q) c = cadd(c, chunks[(size_t)q * NX + x]);
+    const double px = a.dP * (s.x * c.x - s.y * c.y);
+    Ps[x] = px;
+    acc[0] += px * px;
+  }
+  __syncthreads();
+  if (psq != nullptr && blockIdx.x == 0) {
+    __shared__ double red1[NT / 32][1];
+    block_sum<NT, 1>(acc, red1);
+    if (threadIdx.x == 0) *psq = red1[0][0] * a.dX;
+  }
+  double2 v[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) v[m] = make_double2(Ps[t + T * m], 0.);
+  F::template run<false>(v, X, a.btw_x, t, sync);
+  const double th = a.theta_s[row <= NP / 2 ? row : 0] * (double)NP;    // exact shifted Theta
+  // sin(lambda theta / 2) is odd in lambda: as apply_odd_factor, one value per pair
+  double* fs = reinterpret_cast<double*>(X);
+  sync();
+#pragma unroll 2
+  for (int k = t; k <= NX / 2; k += T) fs[k] = 2. * sin(0.5 * a.lambda_tab[k] * th);
+  sync();
+#pragma unroll
+  for (int m = 0; m < E; ++m) {
+    const int k = t + T * m;
+    const double sn = k <= NX / 2 ? fs[k] : -fs[NX - k];
+    v[m] = make_double2(sn * v[m].y, -sn * v[m].x);
+  }
+  F::template run<true>(v, X, a.btw_x, t, sync);
+  if (row > NP / 2) return;
+  const double c = -0.5 * a.dt * a.gp_coef / a.hbar * (1.0 / (double)NX);
+#pragma unroll
+  for (int m = 0; m < E; ++m) phase_out[(size_t)row * NX + t + T * m] = c * v[m].x;
+}
+
+}  // namespace wig

@@ -1,0 +1,48 @@
+"""The register-blocked complex128 Wigner2D passes on the GPU against the oracle,
+over the tiles that the planner picks: axes from 64 to 4096 points, 4, 8 and 16
+elements a thread (grids below 2^18, 2^19 points and above; the last with the
+Caldeira-Leggett base in tensor memory), one axis of 32 points left to the
+Stockham passes.  Bars: those of the other complex128 paths (relative L2 1e-10,
+observables 1e-10 of their scale)."""
+import numpy as np
+import pytest
+
+from oracle.common import rel_l2
+from oracle.gpitaevskii import GPitaevskiiOracle
+from oracle.wigner2d import WignerOracle, WignerParams, wigner_harmonic_oscillator
+from golden_cases import obs_close
+from instances import gp_instance, wigner_instance, wigner_obs
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-10
+POT, DPOT = '0.05*pow(x,4) - pow(x,2) + 0.1*x*sin(3.*t)', '0.2*pow(x,3) - 2.*x + 0.1*sin(3.*t)'
+
+CASES = [(64, 64, 'cl'), (128, 64, 'none'), (64, 256, 'odm2'), (512, 32, 'cl'), (32, 512, 'odm'), (2048, 64, 'kvn'),
+         (64, 2048, 'cl'), (4096, 64, 'cl'), (64, 4096, 'cl'), (512, 512, 'cl'), (1024, 256, 'odm'),
+         (512, 1024, 'cl'), (1024, 1024, 'kvn'), (256, 2048, 'none'), (2048, 512, 'odm2'), (256, 4096, 'cl'),
+         (64, 64, 'gp'), (256, 64, 'gp'), (512, 1024, 'gp'), (64, 128, 'gpodm')]
+
+
+@pytest.mark.parametrize('n_x,n_p,form', CASES)
+def test_blocked_passes_match_oracle(n_x, n_p, form):
+    odm = 'odm' in form
+    prm = WignerParams(n_x, n_p, 10., 8., 0.01, hbar=0.9, mass=1.3, d_theta=0.05, d_lambda=0.01,
+                       gamma=0. if form == 'none' else 0.05, potential=POT, dpotential=DPOT,
+                       damping='ODM' if odm else 'CaldeiraLeggett', fp_damping='p*p/sqrt(p*p + 0.5)', L_material=2.,
+                       kvn=form == 'kvn', odm2=form == 'odm2', weight1=1., weight2=0.5 if form == 'odm2' else 0.)
+    W0 = wigner_harmonic_oscillator(prm, 0, 1., 1.5, -0.5)
+    if form.startswith('gp'):
+        inst = gp_instance(prm, 0.5, W0, 2)
+        inst.Run()
+        obs, W, psq = GPitaevskiiOracle(prm, 0.5).run(W0, 3)
+        assert np.max(np.abs(inst.ProbabilitySquare_average - psq) / np.abs(psq)) < TOL
+    else:
+        inst = wigner_instance(prm, W0, 2)
+        inst.Run()
+        obs, W = WignerOracle(prm).run(W0, 3)
+        obs = obs[:3]
+    assert rel_l2(inst.W_end_complex, W) < TOL
+    got = wigner_obs(inst)
+    assert obs_close(got[:, :9], obs[:3, 1:10], TOL) < TOL
+    # the negative area sums the points below zero: those within rounding of zero enter one sum and not the other
+    assert np.max(np.abs(got[:, 9] - obs[:3, 10])) < 1e-10
