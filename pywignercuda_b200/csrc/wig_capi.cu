@@ -585,7 +585,7 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
     P->odm2 = P->odm && P->bx && P->bp ? 1 : 0;
     P->oe = 8;
     P->oxr = std::max(1, 32 * P->oe / NX);
-    P->opc = std::max(2, 32 * P->oe / NP);
+    P->opc = NP / P->oe >= 512 ? 1 : std::max(2, 32 * P->oe / NP);
     P->oxmb = std::max(1, std::min(32, 512 / (P->oxr * (NX / P->oe))));
     P->opmb = std::max(1, std::min(32, 512 / (P->opc * (NP / P->oe))));
     if (P->odm2) {
@@ -751,9 +751,13 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
   std::vector<double> dv(NX, 0.), v0(NX, 0.);
   if (d->dv_table) dv.assign(d->dv_table, d->dv_table + NX);
   if (d->v0_table) v0.assign(d->v0_table, d->v0_table + NX);
-  std::vector<double2> twx = twiddles(NX), twp = twiddles(NP);
+  // Stockham twiddles: where a pass (or the Strang / Bloch / five-plane ODM kernels) still takes them
+  const bool stx = !P.bx || P.strang || (P.odm && !P.odm2), stp = !P.bp || P.strang || (P.odm && !P.odm2);
+  std::vector<double2> twx, twp;
+  if (stx) twx = twiddles(NX);
+  if (stp) twp = twiddles(NP);
   double *x_d, *p_d, *dv_d, *v0_d, *ths_d, *rl_d, *rt_d, *m1_d, *m2_d, *sfp_d, *part_d;
-  double2 *twx_d, *twp_d;
+  double2 *twx_d = nullptr, *twp_d = nullptr;
   const int nparts = std::max(std::max(h->n_cta_x, std::max(h->gp_n, h->gop)), h->n_cta_r);
   DevBuf& B = h->bufs;
   rc = B.alloc(&x_d, NX, xt.data());
@@ -766,8 +770,8 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
   if (!rc) rc = B.alloc(&m1_d, NX);
   if (!rc) rc = B.alloc(&m2_d, NX);
   if (!rc) rc = B.alloc(&sfp_d, NP);
-  if (!rc) rc = B.alloc(&twx_d, NX, twx.data());
-  if (!rc) rc = B.alloc(&twp_d, NP, twp.data());
+  if (!rc && stx) rc = B.alloc(&twx_d, NX, twx.data());
+  if (!rc && stp) rc = B.alloc(&twp_d, NP, twp.data());
   if (!rc) rc = B.alloc(&part_d, (size_t)nparts * wig::NACC);
   if (!rc) rc = B.alloc(&h->scale, 1);
   std::vector<double> lt = d->lambda_table ? std::vector<double>(d->lambda_table, d->lambda_table + NX)
@@ -1346,8 +1350,9 @@ struct dirac_handle {
   dirac_desc d{};
   wig::DiracArgs a{};
   CUfunction f_row = nullptr, f_col = nullptr, f_fin = nullptr, f_scale = nullptr;
-  int rows = 1, rnt = 256, cc = 1, cnt = 256, snt = 256;
+  int rnt = 256, cnt = 256, snt = 256;
   int n_row = 1, n_col = 1, smem_row = 0, smem_col = 0;
+  int blk = 0;                                  // register-blocked passes (one row-pass CTA more: the sample)
   DevBuf bufs;
   double* obs = nullptr;
   size_t obs_cap = 0;
@@ -1356,6 +1361,7 @@ struct dirac_handle {
 };
 
 struct DiracPlan {
+  int blk = 0, brows = 1, bre = 4, brmb = 1, bc = 1, bce = 4, bcmb = 1;   // register-blocked passes
   int rows, rnt, rmb, cc, cnt, cmb, snt, n_row, n_col, smem_row, smem_col;
   double dX, dY, Pxa, Pya, dPx, dPy;
   std::string src;
@@ -1409,6 +1415,35 @@ static int dirac_plan(const dirac_desc* d, DiracPlan* P) {
   P->n_col = NX / P->cc;
   P->smem_row = wig::padded_size(4 * P->rows * NX) * (int)sizeof(double2);
   P->smem_col = wig::padded_size(4 * P->cc * NY) * (int)sizeof(double2);
+  // ---- register-blocked passes (axes of at least 64 points; a tile override keeps the Stockham ones):
+  // 8 elements of four components a thread (255 registers, 8 warps per SM), 4 on grids below 2^17
+  // points, where more warps shorten the chains (step, us: 512^2 38 / 47 with 8 / 4, 256^2 24 / 20,
+  // 128 x 64 19 / 14; the Stockham passes 68 at 512^2).  Column tiles of 4 where the grid is wide
+  // enough and the tile fits (512^2: 36.8 / 38.4 / 44.9 us with 4 / 2 / 1).
+  P->blk = NX >= 64 && NY >= 64 && !getenv("WIG_DIRAC_TILING") ? 1 : 0;
+  if (P->blk) {
+    const int e = (long)NX * NY >= (1L << 17) ? 8 : 4;
+    P->bre = P->bce = e;
+    int v[6] = {0, 0, 0, 0, 0, 0};
+    // WIG_DIRAC_BTILING="re,rows,rmb,ce,cols,cmb" overrides the tiles for tuning runs (0: default)
+    if (const char* tv = getenv("WIG_DIRAC_BTILING"))
+      sscanf(tv, "%d,%d,%d,%d,%d,%d", &v[0], &v[1], &v[2], &v[3], &v[4], &v[5]);
+    if (v[0] == 4 || v[0] == 8) P->bre = v[0];
+    if (v[3] == 4 || v[3] == 8) P->bce = v[3];
+    P->brows = std::max(v[1], std::max(1, 32 * P->bre / NX));
+    P->bc = std::max(v[4] > 0 ? v[4] : (e == 8 && NX >= 512 ? (NY <= 512 ? 4 : (NY <= 1024 ? 2 : 1)) : 1), std::max(1, 32 * P->bce / NY));
+    P->rnt = P->brows * (NX / P->bre);
+    P->cnt = P->bc * (NY / P->bce);
+    P->brmb = v[2] > 0 ? v[2] : std::max(1, std::min(32, (P->bre == 8 ? 256 : 512) / P->rnt));
+    P->bcmb = v[5] > 0 ? v[5] : std::max(1, std::min(32, (P->bce == 8 ? 256 : 512) / P->cnt));
+    const auto pad = [](int n, int e) { return n + n / std::min(e, 8); };
+    P->n_row = NY / P->brows;
+    P->n_col = NX / P->bc;
+    P->smem_row = P->brows * 4 * pad(NX, P->bre) * (int)sizeof(double2);
+    P->smem_col = P->bc * wig::blk_stride(4 * pad(NY, P->bce), P->bc) * (int)sizeof(double2);
+    if (P->rnt > 1024 || P->cnt > 1024 || NY % P->brows || NX % P->bc)
+      return fail(WIG_ERR_ARG, "WIG_DIRAC_BTILING: tiles of %d / %d threads", P->rnt, P->cnt);
+  }
   // GPU_Dirac2D.py:312-346
   P->dX = 2. * d->x_amplitude / (double)NX;
   P->dY = 2. * d->y_amplitude / (double)NY;
@@ -1433,6 +1468,13 @@ static int dirac_plan(const dirac_desc* d, DiracPlan* P) {
            "#define DIR_C %d\n#define DIR_CNT %d\n#define DIR_CMB %d\n#define DIR_SNT %d\n",
            NX, NY, P->rows, P->rnt, P->rmb, P->cc, P->cnt, P->cmb, P->snt);
   src += macros;
+  if (P->blk) {
+    snprintf(macros, sizeof(macros),
+             "#define DIR_B 1\n#define DIR_BROWS %d\n#define DIR_BRE %d\n#define DIR_BRMB %d\n#define DIR_BC %d\n"
+             "#define DIR_BCE %d\n#define DIR_BCMB %d\n",
+             P->brows, P->bre, P->brmb, P->bc, P->bce, P->bcmb);
+    src += macros;
+  }
   src += kJitDiracSource;
   P->src.swap(src);
   return WIG_OK;
@@ -1461,7 +1503,8 @@ extern "C" int dirac_create(const dirac_desc* d, dirac_handle** out) {
   h->d = *d;
   h->device = device;
   const int NX = d->n_x, NY = d->n_y, cm = d->constants;
-  h->rows = P.rows; h->rnt = P.rnt; h->cc = P.cc; h->cnt = P.cnt; h->snt = P.snt;
+  h->rnt = P.rnt; h->cnt = P.cnt; h->snt = P.snt;
+  h->blk = P.blk;
   h->n_row = P.n_row; h->n_col = P.n_col; h->smem_row = P.smem_row; h->smem_col = P.smem_col;
   const double dX = P.dX, dY = P.dY, Pxa = P.Pxa, Pya = P.Pya, dPx = P.dPx, dPy = P.dPy;
   const std::string& src = P.src;
@@ -1483,9 +1526,8 @@ extern "C" int dirac_create(const dirac_desc* d, dirac_handle** out) {
   std::vector<double> yt = d->y_table ? std::vector<double>(d->y_table, d->y_table + NY) : shifted_range(d->y_amplitude, NY);
   std::vector<double> pxt = d->px_table ? std::vector<double>(d->px_table, d->px_table + NX) : shifted_range(Pxa, NX);
   std::vector<double> pyt = d->py_table ? std::vector<double>(d->py_table, d->py_table + NY) : shifted_range(Pya, NY);
-  std::vector<double2> twx = twiddles(NX), twy = twiddles(NY);
   double *x_d, *y_d, *px_d, *py_d, *bx_d, *by_d, *pr0, *pr1, *pc;
-  double2 *twx_d, *twy_d;
+  double2 *twx_d = nullptr, *twy_d = nullptr, *btx_d = nullptr, *bty_d = nullptr;
   DevBuf& B = h->bufs;
   rc = B.alloc(&x_d, NX, xt.data());
   if (!rc) rc = B.alloc(&y_d, NY, yt.data());
@@ -1493,14 +1535,19 @@ extern "C" int dirac_create(const dirac_desc* d, dirac_handle** out) {
   if (!rc) rc = B.alloc(&py_d, NY, pyt.data());
   if (!rc) rc = B.alloc(&bx_d, 2 * (size_t)NX);
   if (!rc) rc = B.alloc(&by_d, 2 * (size_t)NY);
-  if (!rc) rc = B.alloc(&twx_d, NX, twx.data());
-  if (!rc) rc = B.alloc(&twy_d, NY, twy.data());
+  {
+    const std::vector<double2> tx = P.blk ? block_twiddles(NX, P.bre) : twiddles(NX);
+    const std::vector<double2> ty = P.blk ? block_twiddles(NY, P.bce) : twiddles(NY);
+    if (!rc) rc = B.alloc(P.blk ? &btx_d : &twx_d, tx.size(), tx.data());
+    if (!rc) rc = B.alloc(P.blk ? &bty_d : &twy_d, ty.size(), ty.data());
+  }
   if (!rc) rc = B.alloc(&pr0, (size_t)h->n_row * wig::DNR);
   if (!rc) rc = B.alloc(&pr1, (size_t)h->n_row * wig::DNR);
   if (!rc) rc = B.alloc(&pc, (size_t)h->n_col * wig::DNC);
   if (!rc) rc = B.alloc(&h->scale, 1);
   if (rc) { B.free_all(); delete h; return rc; }
   a.x_tab = x_d; a.y_tab = y_d; a.px_tab = px_d; a.py_tab = py_d; a.bx = bx_d; a.by = by_d;
+  a.btw_x = btx_d; a.btw_y = bty_d;
   a.tw_x = twx_d; a.tw_y = twy_d; a.part_row[0] = pr0; a.part_row[1] = pr1; a.part_col = pc;
   a.n_row_cta = h->n_row; a.n_col_cta = h->n_col;
   for (int i = 0; i < 8; ++i) a.coef[i] = d->coef[i];
@@ -1533,6 +1580,10 @@ static int dirac_run_check(dirac_handle* h, void* psi_dev, int64_t n_steps) {
   return ensure_obs(&h->obs, &h->obs_cap, (size_t)n_steps * DIRAC_NOBS);
 }
 
+static int dirac_launch_row(dirac_handle* h, cudaStream_t st, void** args) {
+  return (h->blk ? launch_after : launch)(h->f_row, h->n_row + h->blk, h->rnt, h->smem_row, st, args);
+}
+
 static int dirac_run_begin(dirac_handle* h, DiracRunState* S, void* psi_dev, int64_t t_index0, int64_t n_steps,
                            cudaStream_t st) {
   S->a = h->a;
@@ -1543,18 +1594,18 @@ static int dirac_run_begin(dirac_handle* h, DiracRunState* S, void* psi_dev, int
   double t_step = 0., t_obs = h->d.dt * (double)(t_index0 + 1);
   double* obs_row = nullptr;
   void* args[] = {&S->a, &S->psi, &mode, &parity, &t_step, &t_obs, &obs_row};
-  return launch(h->f_row, h->n_row, h->rnt, h->smem_row, st, args);
+  return dirac_launch_row(h, st, args);
 }
 
 static int dirac_run_step(dirac_handle* h, DiracRunState* S, int64_t n, cudaStream_t st) {
   void* cargs[] = {&S->a, &S->psi};
-  if (int rc = launch(h->f_col, h->n_col, h->cnt, h->smem_col, st, cargs)) return rc;
+  if (int rc = (h->blk ? launch_after : launch)(h->f_col, h->n_col, h->cnt, h->smem_col, st, cargs)) return rc;
   const double dt = h->d.dt;
   int mode = (n == S->n_steps - 1) ? 2 : 1, parity = (int)((n + 1) & 1);
   double t_step = dt * (double)(S->t_index0 + n + 1), t_obs = dt * (double)(S->t_index0 + n + 2);
   double* obs_row = h->obs + (size_t)n * DIRAC_NOBS;
   void* args[] = {&S->a, &S->psi, &mode, &parity, &t_step, &t_obs, &obs_row};
-  return launch(h->f_row, h->n_row, h->rnt, h->smem_row, st, args);
+  return dirac_launch_row(h, st, args);
 }
 
 static int dirac_run_end(dirac_handle* h, DiracRunState* S, cudaStream_t st) {

@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -15,6 +16,7 @@
 #include "../../include/wigner_b200.h"
 #include "wig_dirac3.cuh"
 #include "wig_host.h"
+#include "wig_batch_host.h"      // register-blocked transforms' twiddle tables
 #include "wig_dirac3_src.inc"   // kJitDirac3Source (generated by build.py)
 
 using namespace wighost;
@@ -24,6 +26,8 @@ namespace {
 constexpr int kMaxCta = 148 * 16;   // grid-stride passes: at most 16 CTAs per SM
 
 struct Dirac3Plan {
+  // register-blocked passes (x, y, z): lines a CTA, elements a thread, CTAs per SM
+  int blk = 0, bc[3] = {1, 1, 1}, be[3] = {8, 8, 8}, bmb[3] = {1, 1, 1};
   int rows, xnt, yc, ynt, zc, znt, snt;
   // largest Stockham radix / CTAs per SM of each pass: radix 16 only where it fits the register
   // budget without spilling (the z-pass: 126 registers, 3.00 vs 3.08 ms per 256^3 step)
@@ -94,6 +98,45 @@ int d3_plan(const dirac3_desc* d, Dirac3Plan* P) {
   P->smem_x = wig::padded_size(4 * P->rows * NX) * (int)sizeof(double2);
   P->smem_y = wig::padded_size(NY * P->yc) * (int)sizeof(double2);
   P->smem_z = wig::padded_size(4 * P->zc * NZ) * (int)sizeof(double2);
+  // ---- register-blocked passes (axes of at least 32 points; a tile override keeps the Stockham ones)
+  P->blk = NX >= 32 && NY >= 32 && NZ >= 32 && !getenv("WIG_D3_TILING") && !getenv("WIG_D3_RADIX") ? 1 : 0;
+  if (P->blk) {
+    const int n[3] = {NX, NY, NZ};
+    int v[9] = {0};
+    // WIG_D3_BTILING="xe,xc,xmb,ye,yc,ymb,ze,zc,zmb" overrides the tiles for tuning runs (0: default)
+    if (const char* t = getenv("WIG_D3_BTILING"))
+      sscanf(t, "%d,%d,%d,%d,%d,%d,%d,%d,%d", &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6], &v[7], &v[8]);
+    // x, z: 8 elements of four components a thread (255 registers), 4 on grids below 2^18 points
+    // (step, us: 128^3 307 / 330 with 8 / 4, 32^3 36 / 30; the Stockham passes 419 and 47); y: 16 of one
+    // component (8, 4 on shorter axes).  CTAs of up to 256 threads (at most 16 and 8 columns,
+    // y and z), as long as there are two tiles an SM: 128^3 307 / 367 us with 128- / 64-thread tiles.
+    const bool small = (long)NX * NY * NZ < (1L << 18);
+    const long lines[3] = {(long)NY * NZ, 4L * NZ * NX, (long)NY * NX};
+    const int least[3] = {1, std::min(4, NX), std::min(4, NX)}, most[3] = {std::min(NY * NZ, 64), 16, 8};
+    int nt[3];
+    for (int i = 0; i < 3; ++i) {
+      P->be[i] = v[3 * i] ? v[3 * i] : (i == 1 ? (n[i] >= 128 ? 16 : (small ? 4 : 8)) : (small ? 4 : 8));
+      const int T = n[i] / P->be[i];
+      int c = least[i];
+      while (c * T < 32) c *= 2;
+      while (c < most[i] && 2 * c * T <= 256 && lines[i] / (2 * c) >= 2 * 148) c *= 2;
+      P->bc[i] = v[3 * i + 1] ? v[3 * i + 1] : c;
+      nt[i] = P->bc[i] * T;
+      P->bmb[i] = v[3 * i + 2] ? v[3 * i + 2]
+                               : std::max(1, std::min(32, (i == 1 || P->be[i] == 4 ? 512 : 256) / nt[i]));
+      if (nt[i] > 1024 || nt[i] % 32 || (i > 0 && P->bc[i] > 32)) return fail(WIG_ERR_ARG, "WIG_D3_BTILING: tile of %d threads", nt[i]);
+    }
+    const auto pad = [](int n, int e) { return n + n / std::min(e, 8); };
+    P->xnt = nt[0];
+    P->ynt = nt[1];
+    P->znt = nt[2];
+    P->smem_x = P->bc[0] * 4 * pad(NX, P->be[0]) * (int)sizeof(double2);
+    P->smem_y = P->bc[1] * wig::blk_stride(pad(NY, P->be[1]), P->bc[1]) * (int)sizeof(double2);
+    P->smem_z = P->bc[2] * wig::blk_stride(4 * pad(NZ, P->be[2]), P->bc[2]) * (int)sizeof(double2);
+    P->gx = clampi(NY * NZ / P->bc[0], 1, 148 * P->bmb[0]);
+    P->gy = clampi(4 * NZ * (NX / P->bc[1]), 1, 148 * P->bmb[1]);
+    P->gz = clampi(NY * (NX / P->bc[2]), 1, 148 * P->bmb[2]);
+  }
   // GPU_Dirac3D.py:637-683
   P->dX = 2. * d->x_amplitude / (double)NX;
   P->dY = 2. * d->y_amplitude / (double)NY;
@@ -122,6 +165,13 @@ int d3_plan(const dirac3_desc* d, Dirac3Plan* P) {
            NX, NY, NZ, P->rows, P->xnt, P->yc, P->ynt, P->zc, P->znt, P->snt, P->xr, P->yr, P->zr, P->xmb,
            P->ymb, P->zmb);
   src += macros;
+  if (P->blk) {
+    snprintf(macros, sizeof(macros),
+             "#define D3_B 1\n#define D3_BXC %d\n#define D3_BXE %d\n#define D3_BXMB %d\n#define D3_BYC %d\n"
+             "#define D3_BYE %d\n#define D3_BYMB %d\n#define D3_BZC %d\n#define D3_BZE %d\n#define D3_BZMB %d\n",
+             P->bc[0], P->be[0], P->bmb[0], P->bc[1], P->be[1], P->bmb[1], P->bc[2], P->be[2], P->bmb[2]);
+    src += macros;
+  }
   src += kJitDirac3Source;
   P->src.swap(src);
   return WIG_OK;
@@ -181,21 +231,23 @@ extern "C" int dirac3_create(const dirac3_desc* d, dirac3_handle** out) {
   a.dPx = kval(P.dPx, cm); a.dPy = kval(P.dPy, cm); a.dPz = kval(P.dPz, cm);
   a.dX_e = P.dX; a.dY_e = P.dY; a.dZ_e = P.dZ; a.dPx_e = P.dPx; a.dPy_e = P.dPy; a.dPz_e = P.dPz;
   for (int i = 0; i < 8; ++i) a.coef[i] = d->coef[i];
-  std::vector<double2> twx = twiddles(NX), twy = twiddles(NY), twz = twiddles(NZ);
   const size_t npart_x = (size_t)(P.gx * wig::D3X > P.gn ? P.gx * wig::D3X : P.gn);
   const double init[2] = {1.0, 0.0};   // scale, s1
-  double2 *twx_d, *twy_d, *twz_d;
   double *px0, *px1, *pp, *sc;
   DevBuf& B = h->bufs;
-  rc = B.alloc(&twx_d, NX, twx.data());
-  if (!rc) rc = B.alloc(&twy_d, NY, twy.data());
-  if (!rc) rc = B.alloc(&twz_d, NZ, twz.data());
+  double2* tw_d[3] = {nullptr, nullptr, nullptr};
+  const int n[3] = {NX, NY, NZ};
+  for (int i = 0; i < 3 && !rc; ++i) {
+    const std::vector<double2> tw = P.blk ? block_twiddles(n[i], P.be[i]) : twiddles(n[i]);
+    rc = B.alloc(&tw_d[i], tw.size(), tw.data());
+  }
+  if (P.blk) { a.btw_x = tw_d[0]; a.btw_y = tw_d[1]; a.btw_z = tw_d[2]; }
+  else { a.tw_x = tw_d[0]; a.tw_y = tw_d[1]; a.tw_z = tw_d[2]; }
   if (!rc) rc = B.alloc(&px0, npart_x);
   if (!rc) rc = B.alloc(&px1, npart_x);
   if (!rc) rc = B.alloc(&pp, (size_t)P.gz * wig::D3P);
   if (!rc) rc = B.alloc(&sc, 2, init);
   if (rc) { B.free_all(); delete h; return rc; }
-  a.tw_x = twx_d; a.tw_y = twy_d; a.tw_z = twz_d;
   a.part_x[0] = px0; a.part_x[1] = px1; a.part_p = pp;
   a.scale = sc; a.s1 = sc + 1;
   a.n_x_cta = P.gx; a.n_z_cta = P.gz;
@@ -216,6 +268,7 @@ extern "C" int dirac3_run(dirac3_handle* h, void* psi_dev, int64_t t_index0, int
   const Dirac3Plan& P = h->P;
   double2* psi = (double2*)psi_dev;
   const double dt = h->d.dt;
+  const auto step = P.blk ? launch_after : launch;   // blocked passes: one x-pass CTA more (the sample)
   int normalise = (flags & WIG_RUN_CONTINUE) ? 0 : 1;
   if (normalise) {   // Normalize_GPU before the loop (:1323)
     long n = 4L * h->d.n_x * h->d.n_y * h->d.n_z;
@@ -231,19 +284,19 @@ extern "C" int dirac3_run(dirac3_handle* h, void* psi_dev, int64_t t_index0, int
     long long prev = 0;
     double* obs_prev = nullptr;
     void* args[] = {&h->a, &psi, &mode, &parity, &normalise, &tA, &tobs, &prev, &obs_prev};
-    if (int rc = launch(h->f_x, P.gx, P.xnt, P.smem_x, st, args)) return rc;
+    if (int rc = step(h->f_x, P.gx + P.blk, P.xnt, P.smem_x, st, args)) return rc;
   }
   for (int64_t k = 1; k <= n_steps; ++k) {
     void* cargs[] = {&h->a, &psi};
-    if (int rc = launch(h->f_yf, P.gy, P.ynt, P.smem_y, st, cargs)) return rc;
-    if (int rc = launch(h->f_z, P.gz, P.znt, P.smem_z, st, cargs)) return rc;
-    if (int rc = launch(h->f_yi, P.gy, P.ynt, P.smem_y, st, cargs)) return rc;
+    if (int rc = step(h->f_yf, P.gy, P.ynt, P.smem_y, st, cargs)) return rc;
+    if (int rc = step(h->f_z, P.gz, P.znt, P.smem_z, st, cargs)) return rc;
+    if (int rc = step(h->f_yi, P.gy, P.ynt, P.smem_y, st, cargs)) return rc;
     int mode = (k == n_steps) ? 2 : 1, parity = (int)(k & 1), nrm = 0;
     double tA = dt * (double)(t_index0 + k), tobs = dt * (double)(t_index0 + k + 1);
     long long prev = (long long)(t_index0 + k);
     double* obs_prev = h->obs + (size_t)(k - 1) * wig::D3NOBS;
     void* args[] = {&h->a, &psi, &mode, &parity, &nrm, &tA, &tobs, &prev, &obs_prev};
-    if (int rc = launch(h->f_x, P.gx, P.xnt, P.smem_x, st, args)) return rc;
+    if (int rc = step(h->f_x, P.gx + P.blk, P.xnt, P.smem_x, st, args)) return rc;
   }
   if (obs_host) {
     const size_t nobs = (size_t)n_steps * wig::D3NOBS;

@@ -42,6 +42,10 @@ struct Dirac3Args {
   double* scale;         // [1] factor of the initial Normalize_GPU
   int n_x_cta, n_z_cta;
   double coef[8];
+  // stage twiddles of the register-blocked passes (BlockFft); null when the plan uses the Stockham ones
+  const double2* btw_x;
+  const double2* btw_y;
+  const double2* btw_z;
 };
 
 __device__ __forceinline__ double d3_n2(double2 v) { return v.x * v.x + v.y * v.y; }
@@ -329,6 +333,235 @@ __device__ __forceinline__ void d3_norm_final(const Dirac3Args& a, int n_cta) {
     *a.scale = 1.0 / sqrt(red[0][0] * a.dX_e * a.dY_e * a.dZ_e);
     *a.s1 = 0.;
   }
+}
+
+// ---------------------------------------------------------------- register-blocked passes
+// As in wig_dirac.cuh: the x- and z-pass hold E elements of all four components of
+// a line per thread (BlockFft::run_many), the y-pass E elements of one component.
+// Persistent over their tiles, as the passes above, with the same partial sums.
+
+// The factors of d3_A at one point: exp(-i dt A0), cos, and m c^2 / 2, A1, A2, A3 times sin / F; A0(t_obs).
+constexpr int D3AF = 8;
+template <class Phys>
+__device__ __forceinline__ void d3_A_factors(const Dirac3Args& a, const Phys& ph, double t, double t_obs, double x,
+                                             double y, double z, double (&f)[D3AF]) {
+  const double A0 = ph.A0(t, x, y, z), A1 = ph.A1(t, x, y, z), A2 = ph.A2(t, x, y, z), A3 = ph.A3(t, x, y, z);
+  const double mc2 = 0.5 * a.mass * a.c * a.c;
+  const double F = sqrt(mc2 * mc2 + (A1 * A1 + A2 * A2 + A3 * A3));
+  double sv, cv, sF, cF;
+  sincos(-a.dt * A0, &sv, &cv);
+  sincos(a.dt * (F / a.hbar), &sF, &cF);
+  const double sf = sF / F;
+  f[0] = cv; f[1] = sv; f[2] = cF; f[3] = mc2 * sf;
+  f[4] = A1 * sf; f[5] = A2 * sf; f[6] = A3 * sf;
+  f[7] = ph.A0(t_obs, x, y, z);
+}
+__device__ __forceinline__ void d3_A_apply(const double (&f)[D3AF], double2& p1, double2& p2, double2& p3,
+                                           double2& p4) {
+  const double2 e = make_double2(f[0], f[1]);
+  const double2 U11 = make_double2(f[2], -f[3]), U33 = make_double2(f[2], f[3]);
+  const double2 U13 = make_double2(0., f[6]), U24 = make_double2(0., -f[6]);
+  const double2 U14 = make_double2(f[5], f[4]), U23 = make_double2(-f[5], f[4]);
+  const double2 q1 = cmul(e, cadd(cadd(cmul(U11, p1), cmul(U13, p3)), cmul(U14, p4)));
+  const double2 q2 = cmul(e, cadd(cadd(cmul(U11, p2), cmul(U23, p3)), cmul(U24, p4)));
+  const double2 q3 = cmul(e, cadd(cadd(cmul(U13, p1), cmul(U14, p2)), cmul(U33, p3)));
+  const double2 q4 = cmul(e, cadd(cadd(cmul(U23, p1), cmul(U24, p2)), cmul(U33, p4)));
+  p1 = q1; p2 = q2; p3 = q3; p4 = q4;
+}
+
+// x-pass (d3_xpass_body's modes), ROWS lines per tile.  The last CTA of the grid (block n_x_cta)
+// only records the previous sample.  Shared memory: per line four exchange regions.
+template <class Phys, int NX, int NY, int NZ, int ROWS, int E>
+__device__ __forceinline__ void d3_xpass_blk_body(const Dirac3Args& a, const Phys& ph, double2* __restrict__ psi,
+                                                  int mode, int parity, int normalise, double t_A, double t_obs,
+                                                  long long prev_tindex, double* obs_prev) {
+  typedef BlockFft<double2, NX, E> F;
+  constexpr int T = F::T, NT = ROWS * T, NROW = NY * NZ, NG = NROW / ROWS;
+  static_assert(NT % 32 == 0 && (T % 32 == 0 || 32 % T == 0), "x-pass lines per CTA");
+  static_assert(4 * F::REGION * 2 >= D3AF * NX, "the factors fit in the exchange regions");
+  extern __shared__ double2 sm[];
+  __shared__ double red[NT / 32][NACC];
+  grid_wait();
+  grid_launch_next();
+  if ((int)blockIdx.x == a.n_x_cta) {
+    if (mode != 0 && obs_prev != nullptr) d3_finalize_sample<NT>(a, a.part_x[parity ^ 1], prev_tindex, obs_prev);
+    return;
+  }
+  const int seq = threadIdx.x / T, t = threadIdx.x % T;
+  const size_t comp = (size_t)NX * NROW;
+  const double scale = (mode == 0 && normalise) ? *a.scale : 1.0;
+  double2* X = sm + seq * 4 * F::REGION;
+  double* fs = reinterpret_cast<double*>(X) + t;
+  const auto sync = SeqSync<T, ROWS>::make(seq);
+  double acc[NACC];
+#pragma unroll
+  for (int q = 0; q < NACC; ++q) acc[q] = 0.;
+  for (int g = blockIdx.x; g < NG; g += a.n_x_cta) {
+    const int row = g * ROWS + seq, iz = row / NY, iy = row - iz * NY;
+    double2* P = psi + (size_t)row * NX + t;
+    double2 v[4][E];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[c][m] = P[c * comp + T * m];
+    if (mode != 0) {
+      F::template run_many<true>(v, X, fresh(a.btw_x), t, sync);
+    } else if (normalise) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int m = 0; m < E; ++m) v[c][m] = cscale(v[c][m], scale);
+    }
+    sync();   // the regions have been read
+    const double y = d3_coord(a.dY, iy, NY), z = d3_coord(a.dZ, iz, NZ);
+#pragma unroll 1
+    for (int m = 0; m < E; ++m) {
+      const double x = d3_coord(a.dX, t + T * m, NX);
+      if (mode != 0) {
+        double f[D3AF];
+        d3_A_factors(a, ph, t_A, t_obs, x, y, z, f);
+#pragma unroll
+        for (int j = 0; j < D3AF; ++j) fs[j * NX + T * m] = f[j];
+      } else {
+        fs[(D3AF - 1) * NX + T * m] = ph.A0(t_obs, x, y, z);
+      }
+    }
+    double S = 0.;
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      double2 p1 = v[0][m], p2 = v[1][m], p3 = v[2][m], p4 = v[3][m];
+      if (mode != 0) {
+        double f[D3AF];
+#pragma unroll
+        for (int j = 0; j < D3AF; ++j) f[j] = fs[j * NX + T * m];
+        d3_A_apply(f, p1, p2, p3, p4);
+        v[0][m] = p1; v[1][m] = p2; v[2][m] = p3; v[3][m] = p4;
+      }
+      if (mode != 2) {
+        const double rho = d3_n2(p1) + d3_n2(p2) + d3_n2(p3) + d3_n2(p4);
+        S += rho;
+        acc[1] += rho * d3_coord(a.dX, t + T * m, NX);
+        acc[4] += d3_re(p4, p1) + d3_re(p3, p2);
+        acc[5] += d3_im(p1, p4) + d3_im(p3, p2);
+        acc[6] += d3_re(p3, p1) - d3_re(p4, p2);
+        acc[7] += fs[(D3AF - 1) * NX + T * m] * rho;
+      }
+    }
+    acc[0] += S;
+    acc[2] += S * y;
+    acc[3] += S * z;
+    if (mode != 2) F::template run_many<false>(v, X, fresh(a.btw_x), t, sync);
+    else sync();   // the factors have been read
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int m = 0; m < E; ++m) P[c * comp + T * m] = v[c][m];
+  }
+  if (mode != 2) {
+    acc[4] *= 2.;
+    acc[5] *= -2.;
+    acc[6] *= 2.;
+    block_sum<NT, NACC>(acc, red);
+    if (threadIdx.x < D3X) a.part_x[parity][(size_t)blockIdx.x * D3X + threadIdx.x] = red[0][threadIdx.x];
+  }
+}
+
+// y-pass: component m, plane z, C columns per tile (column = threadIdx.x % C).
+// Shared memory: C exchange regions.
+template <int NX, int NY, int NZ, int C, int E, bool INV>
+__device__ __forceinline__ void d3_ypass_blk_body(const Dirac3Args& a, double2* __restrict__ psi) {
+  typedef BlockFft<double2, NY, E> F;
+  constexpr int T = F::T, NT = C * T, RS = blk_stride(F::REGION, C), NCT = NX / C, NTILE = 4 * NZ * NCT;
+  static_assert(NT % 32 == 0, "y-pass columns per CTA");
+  extern __shared__ double2 sm[];
+  grid_wait();
+  grid_launch_next();
+  const int c = threadIdx.x % C, t = threadIdx.x / C;
+  double2* X = sm + c * RS;
+  const auto sync = SeqSync<NT, 1>::make(0);
+  for (int g = blockIdx.x; g < NTILE; g += gridDim.x) {
+    const int plane = g / NCT, x0 = (g - plane * NCT) * C;          // plane = m * NZ + z
+    double2* P = psi + (size_t)plane * NX * NY + x0 + c + (size_t)t * NX;
+    double2 v[E];
+#pragma unroll
+    for (int m = 0; m < E; ++m) v[m] = P[(size_t)(T * m) * NX];
+    F::template run<INV>(v, X, fresh(a.btw_y), t, sync);
+#pragma unroll
+    for (int m = 0; m < E; ++m) P[(size_t)(T * m) * NX] = v[m];
+  }
+}
+
+// z-pass: row y, C columns per tile, 4 components.  The mix factors are even in p_z: evaluated for
+// k <= N_z / 2, shared through the exchange regions.  Shared memory: per column four exchange regions.
+template <int NX, int NY, int NZ, int C, int E>
+__device__ __forceinline__ void d3_zpass_blk_body(const Dirac3Args& a, double2* __restrict__ psi) {
+  typedef BlockFft<double2, NZ, E> F;
+  constexpr int T = F::T, NT = C * T, RS = blk_stride(4 * F::REGION, C), NCT = NX / C, NTILE = NY * NCT;
+  static_assert(NT % 32 == 0, "z-pass columns per CTA");
+  extern __shared__ double2 sm[];
+  __shared__ double red[NT / 32][NACC];
+  grid_wait();
+  grid_launch_next();
+  const size_t comp = (size_t)NX * NY * NZ, plane = (size_t)NX * NY;
+  const double inv_n = 1.0 / ((double)NX * (double)NY * (double)NZ);
+  const double m_ = 0.5 * a.mass;
+  const int cc = threadIdx.x % C, t = threadIdx.x / C;
+  double2* X = sm + cc * RS;
+  const auto sync = SeqSync<NT, 1>::make(0);
+  double acc[NACC];
+#pragma unroll
+  for (int q = 0; q < NACC; ++q) acc[q] = 0.;
+  for (int g = blockIdx.x; g < NTILE; g += gridDim.x) {
+    const int iy = g / NCT, col = (g - iy * NCT) * C + cc;
+    double2* P = psi + (size_t)iy * NX + col + (size_t)t * plane;
+    double2 v[4][E];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[c][m] = P[c * comp + (size_t)(T * m) * plane];
+    F::template run_many<false>(v, X, fresh(a.btw_z), t, sync);
+    const double px = d3_coord(a.dPx, col, NX), py = d3_coord(a.dPy, iy, NY);
+    sync();
+#pragma unroll 2
+    for (int k = t; k <= NZ / 2; k += T) {
+      const double pz = d3_coord(a.dPz, k, NZ);
+      const double E_ = a.c * sqrt(px * px + py * py + pz * pz + m_ * a.c * (m_ * a.c));
+      double sn, cs;
+      sincos(E_ * a.dt / a.hbar, &sn, &cs);
+      X[k] = make_double2(cs * inv_n, a.c * sn / E_ * inv_n);
+    }
+    sync();
+    double S = 0.;
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      const int k = t + T * m;
+      const double2 q1 = v[0][m], q2 = v[1][m], q3 = v[2][m], q4 = v[3][m];
+      const double pz = d3_coord(a.dPz, k, NZ);
+      const double up = d3_n2(q1) + d3_n2(q2), dn = d3_n2(q3) + d3_n2(q4), r2 = up + dn;
+      S += r2;
+      acc[3] += r2 * pz;
+      acc[4] += a.mass * a.c * a.c * (up - dn) + 2. * a.c * px * (d3_re(q4, q1) + d3_re(q3, q2)) +
+                2. * a.c * py * (d3_im(q4, q1) + d3_im(q2, q3)) + 2. * a.c * pz * (d3_re(q3, q1) - d3_re(q4, q2));
+      const double2 f = X[k <= NZ / 2 ? k : NZ - k];
+      const double2 U11 = make_double2(f.x, -a.c * m_ * f.y), U33 = make_double2(f.x, a.c * m_ * f.y);
+      const double2 U13 = make_double2(0., -pz * f.y), U24 = make_double2(0., pz * f.y);
+      const double2 U14 = make_double2(-py * f.y, -px * f.y), U23 = make_double2(py * f.y, -px * f.y);
+      v[0][m] = cadd(cadd(cmul(U11, q1), cmul(U13, q3)), cmul(U14, q4));
+      v[1][m] = cadd(cadd(cmul(U11, q2), cmul(U23, q3)), cmul(U24, q4));
+      v[2][m] = cadd(cadd(cmul(U13, q1), cmul(U14, q2)), cmul(U33, q3));
+      v[3][m] = cadd(cadd(cmul(U23, q1), cmul(U24, q2)), cmul(U33, q4));
+    }
+    acc[0] += S;
+    acc[1] += S * px;
+    acc[2] += S * py;
+    F::template run_many<true>(v, X, fresh(a.btw_z), t, sync);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int m = 0; m < E; ++m) P[c * comp + (size_t)(T * m) * plane] = v[c][m];
+  }
+  block_sum<NT, NACC>(acc, red);
+  if (threadIdx.x < D3P) a.part_p[(size_t)blockIdx.x * D3P + threadIdx.x] = red[0][threadIdx.x];
 }
 
 }  // namespace wig

@@ -385,12 +385,20 @@ template <class C, int N, int E> struct BlockFft {
   // s: the sequence's exchange region; sync() orders the T threads' accesses to it.
   template <bool INV, class Sync>
   __device__ __forceinline__ static void run(C (&v)[E], C* s, const C* __restrict__ tw, int t, const Sync& sync) {
-    stage<1, INV>(v, s, tw, t, sync);
+    stage<1, INV, 1>(reinterpret_cast<C(&)[1][E]>(v), s, tw, t, sync);
+  }
+  // NC sequences held by the same T threads, transformed together (each stage's twiddles are
+  // loaded once, its boundary costs one pair of barriers); s: NC regions, one after another
+  template <bool INV, int NC, class Sync>
+  __device__ __forceinline__ static void run_many(C (&v)[NC][E], C* s, const C* __restrict__ tw, int t,
+                                                  const Sync& sync) {
+    stage<1, INV, NC>(v, s, tw, t, sync);
   }
 
   // the stage of sub-length NS: butterflies t + T q, q < E / R
-  template <int NS, bool INV, class Sync>
-  __device__ __forceinline__ static void stage(C (&v)[E], C* s, const C* __restrict__ tw, int t, const Sync& sync) {
+  template <int NS, bool INV, int NC, class Sync>
+  __device__ __forceinline__ static void stage(C (&v)[NC][E], C* s, const C* __restrict__ tw, int t,
+                                               const Sync& sync) {
     constexpr int R = radix(NS), Q = E / R;
     static_assert(T % NS == 0, "a stage's butterflies share their twiddles");
     const int k = t & (NS - 1);
@@ -402,7 +410,8 @@ template <class C, int N, int E> struct BlockFft {
         w1[a] = __ldg(tw + (3 + a) * NS + k);
         if (INV) { w4[a] = cconj(w4[a]); w1[a] = cconj(w1[a]); }
       }
-      dft16_tw<INV>(v, w4, w1);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) dft16_tw<INV>(v[c], w4, w1);
     } else {
       C w[R];
       if constexpr (NS > 1) {
@@ -413,27 +422,34 @@ template <class C, int N, int E> struct BlockFft {
         }
       }
 #pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        C u[R];
+      for (int c = 0; c < NC; ++c)
 #pragma unroll
-        for (int r = 0; r < R; ++r) u[r] = NS > 1 && r > 0 ? cmul(v[q + r * Q], w[r]) : v[q + r * Q];
-        dft_r<R, INV>(u);
+        for (int q = 0; q < Q; ++q) {
+          C u[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[q + r * Q] = u[r];
-      }
+          for (int r = 0; r < R; ++r) u[r] = NS > 1 && r > 0 ? cmul(v[c][q + r * Q], w[r]) : v[c][q + r * Q];
+          dft_r<R, INV>(u);
+#pragma unroll
+          for (int r = 0; r < R; ++r) v[c][q + r * Q] = u[r];
+        }
     }
     if constexpr (NS * R < N) {
       sync();   // the region's previous contents have been read
       C* d = s + slot<NS, R>((t - k) * R + k);
 #pragma unroll
-      for (int q = 0; q < Q; ++q)
+      for (int c = 0; c < NC; ++c)
 #pragma unroll
-        for (int r = 0; r < R; ++r) d[slot<NS, R>(T * q * R) + slot<NS, R>(r * NS)] = v[q + r * Q];
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            d[c * REGION + slot<NS, R>(T * q * R) + slot<NS, R>(r * NS)] = v[c][q + r * Q];
       sync();
       const C* g = s + slot<NS, R>(t);
 #pragma unroll
-      for (int m = 0; m < E; ++m) v[m] = g[slot<NS, R>(T * m)];
-      stage<NS * R, INV>(v, s, tw + (NS > 1 ? (R == 16 ? 6 : R - 1) * NS : 0), t, sync);
+      for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int m = 0; m < E; ++m) v[c][m] = g[c * REGION + slot<NS, R>(T * m)];
+      stage<NS * R, INV, NC>(v, s, tw + (NS > 1 ? (R == 16 ? 6 : R - 1) * NS : 0), t, sync);
     }
   }
 };

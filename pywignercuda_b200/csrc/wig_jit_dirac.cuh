@@ -16,16 +16,38 @@ __device__ __forceinline__ UserPhys user_phys(const wig::DiracArgs& a) {
   return ph;
 }
 
-extern "C" __global__ void __launch_bounds__(DIR_RNT, DIR_RMB)
+// DIR_B 1: the passes on the register-blocked transform, DIR_BROWS rows / DIR_BC columns a CTA,
+// DIR_BRE / DIR_BCE elements a thread, DIR_BRMB / DIR_BCMB CTAs per SM
+#ifndef DIR_B
+#define DIR_B 0
+#endif
+#if DIR_B
+#define DIR_ROW_BOUNDS __launch_bounds__(DIR_BROWS * (DIR_NX / DIR_BRE), DIR_BRMB)
+#define DIR_COL_BOUNDS __launch_bounds__(DIR_BC * (DIR_NY / DIR_BCE), DIR_BCMB)
+#else
+#define DIR_ROW_BOUNDS __launch_bounds__(DIR_RNT, DIR_RMB)
+#define DIR_COL_BOUNDS __launch_bounds__(DIR_CNT, DIR_CMB)
+#endif
+
+extern "C" __global__ void DIR_ROW_BOUNDS
 dirac_rowpass(wig::DiracArgs a, double2* psi, int mode, int parity, double t_step, double t_obs,
               double* obs_row) {
+#if DIR_B
+  wig::dirac_row_blk_body<UserPhys, DIR_NX, DIR_NY, DIR_BROWS, DIR_BRE>(a, user_phys(a), psi, mode, parity, t_step,
+                                                                        t_obs, obs_row);
+#else
   wig::dirac_row_body<UserPhys, DIR_NX, DIR_NY, DIR_ROWS, DIR_RNT>(
       a, user_phys(a), psi, mode, parity, t_step, t_obs, obs_row);
+#endif
 }
 
-extern "C" __global__ void __launch_bounds__(DIR_CNT, DIR_CMB)
+extern "C" __global__ void DIR_COL_BOUNDS
 dirac_colpass(wig::DiracArgs a, double2* psi) {
+#if DIR_B
+  wig::dirac_col_blk_body<DIR_NX, DIR_NY, DIR_BC, DIR_BCE>(a, psi);
+#else
   wig::dirac_col_body<DIR_NX, DIR_NY, DIR_C, DIR_CNT>(a, psi);
+#endif
 }
 
 extern "C" __global__ void __launch_bounds__(DIR_SNT)

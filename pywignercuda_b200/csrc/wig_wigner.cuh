@@ -764,6 +764,23 @@ __device__ __forceinline__ void odm_ppass_body(const WigArgs& a, double2* __rest
 // region and take the conjugate at N - k: half the sincos and half the
 // evaluations of the user's expressions.  k = N/2 is evaluated like the others.
 
+// The pending scale of `mode` alone (consume_partials without a sample).
+template <int NT>
+__device__ __forceinline__ double2 consume_scale(const WigArgs& a, int mode) {
+  __shared__ double red2[NT / 32][2];
+  double acc[2] = {0., 0.};
+  for (int i = threadIdx.x; i < a.n_partials; i += NT) {
+    const double* p = a.partials + (size_t)i * NACC;
+    acc[0] += p[0];
+    acc[1] += p[1];
+  }
+  block_sum<NT, 2>(acc, red2);
+  const double2 S = make_double2(red2[0][0], red2[0][1]);
+  if (mode == 1) return crecip(make_double2(S.x * a.dX * a.dP, S.y * a.dX * a.dP));
+  const double d = a.dX * a.dP;
+  return crecip(make_double2(S.x * d, S.y * d));
+}
+
 // factor(k) for this thread's elements t + T m, applied to v; s: the exchange region
 template <int N, int E, class Sync, class Factor>
 __device__ __forceinline__ void apply_odd_factor(double2 (&v)[E], double2* s, int t, const Sync& sync,
@@ -805,7 +822,7 @@ __device__ __forceinline__ void xpass_blk_body(const WigArgs& a, const Phys& ph,
 #pragma unroll
   for (int m = 0; m < E; ++m) v[m] = Wr[t + T * m];
   if (scale_mode != 0) {
-    const double2 s = consume_partials<NT>(a, scale_mode, nullptr, red);
+    const double2 s = consume_scale<NT>(a, scale_mode);
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = cmul(v[m], s);
   }
@@ -932,8 +949,7 @@ __device__ __forceinline__ void ppass_blk_body(const WigArgs& a, const Phys& ph,
 #pragma unroll
   for (int m = 0; m < E; ++m) v[m] = Wc[(size_t)(T * m) * NX];
   if (FINAL == 0 && scale_mode != 0) {
-    __shared__ double red2[NT / 32][NACC];
-    const double2 s = consume_partials<NT>(a, scale_mode, nullptr, red2);
+    const double2 s = consume_scale<NT>(a, scale_mode);
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = cmul(v[m], s);
   }
@@ -1205,7 +1221,6 @@ __device__ __forceinline__ void gp_phase_blk_body(const WigArgs& a, const double
   constexpr int T = F::T, NT = ROWS * T;
   static_assert(NT % 32 == 0 && (T % 32 == 0 || 32 % T == 0), "phase rows per CTA");
   extern __shared__ double2 sm[];
-  __shared__ double red[NT / 32][NACC];
   const int seq = threadIdx.x / T, t = threadIdx.x % T, row = blockIdx.x * ROWS + seq;
   double2* X = sm + seq * F::REGION;
   double* Ps = reinterpret_cast<double*>(sm + ROWS * F::REGION);
@@ -1213,7 +1228,7 @@ __device__ __forceinline__ void gp_phase_blk_body(const WigArgs& a, const double
   grid_wait();
   grid_launch_next();
   double2 s = make_double2(1., 0.);
-  if (scale_mode != 0) s = consume_partials<NT>(a, scale_mode, nullptr, red);
+  if (scale_mode != 0) s = consume_scale<NT>(a, scale_mode);
   double acc[1] = {0.};
   for (int x = threadIdx.x; x < NX; x += NT) {
     double2 c = make_double2(0., 0.);

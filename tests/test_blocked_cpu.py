@@ -1,5 +1,5 @@
-"""The complex128 Wigner2D passes on the register-blocked transform, executed on
-the host (tests/emu/blocked_emu.cpp), against the oracle, plain, under
+"""The complex128 Wigner2D and Dirac passes on the register-blocked transform,
+executed on the host (tests/emu/blocked_emu.cpp, the Dirac drivers), against the oracle, plain, under
 ThreadSanitizer (a missing barrier between two threads' uses of an exchange
 region is a reported race) and under AddressSanitizer (an index past a launch's
 shared memory).  Tiles: sequences within a warp, of one and of
@@ -73,3 +73,96 @@ def test_blocked_passes_match_oracle(staged, n_x, n_p, x, p, form, sanitize):  #
     scale = np.maximum(np.abs(ref_obs[:, :10]).max(axis=0), 1e-3)
     assert np.all(np.abs(obs[:, :10] - ref_obs[:, :10]) / scale < 1e-10), (obs[:, :10] - ref_obs[:, :10]) / scale
     assert np.all(np.abs(obs[:, 10] - ref_obs[:, 10]) < 1e-12), obs[:, 10] - ref_obs[:, 10]
+
+
+def _driver(staged, name, edits):
+    """tests/emu/<name>.cpp with the register-blocked launch shapes and tables, as <name>_blocked.cpp."""
+    with open(os.path.join(E.EMU, name + '.cpp')) as f:
+        src = f.read()
+    for old, new in edits:
+        assert old in src, old
+        src = src.replace(old, new)
+    with open(os.path.join(staged, name + '_blocked.cpp'), 'w') as f:
+        f.write(src)
+    return name + '_blocked.cpp'
+
+
+DIRAC2D = (
+    ('const int n_row = NY / DIR_ROWS, n_col = NX / DIR_C;', 'const int n_row = NY / DIR_BROWS, n_col = NX / DIR_BC;\n'
+     '  const auto pad = [](int n, int e) { return n + n / std::min(e, 8); };'),
+    ('(size_t)wig::padded_size(4 * DIR_ROWS * NX) * sizeof(double2)',
+     '(size_t)DIR_BROWS * 4 * pad(NX, DIR_BRE) * sizeof(double2)'),
+    ('(size_t)wig::padded_size(4 * DIR_C * NY) * sizeof(double2)',
+     '(size_t)DIR_BC * wig::blk_stride(4 * pad(NY, DIR_BCE), DIR_BC) * sizeof(double2)'),
+    ('emu_launch(n_row, DIR_RNT', 'emu_launch(n_row + 1, DIR_BROWS * (NX / DIR_BRE)'),
+    ('emu_launch(n_col, DIR_CNT', 'emu_launch(n_col, DIR_BC * (NY / DIR_BCE)'),
+    ('a.n_row_cta = n_row;', 'a.n_row_cta = n_row;\n  const std::vector<double2> bx2 = wighost::block_twiddles(NX, '
+     'DIR_BRE), by2 = wighost::block_twiddles(NY, DIR_BCE);\n  a.btw_x = bx2.data(); a.btw_y = by2.data();'),
+    ('#include <cstdlib>', '#include "wig_batch_host.h"\n#include <algorithm>\n#include <cstdlib>'))
+
+DIRAC3D = (
+    ('NY * NZ / D3_ROWS', 'NY * NZ / D3_BXC'), ('NX / D3_YC', 'NX / D3_BYC'), ('NX / D3_ZC', 'NX / D3_BZC'),
+    ('(size_t)wig::padded_size(4 * D3_ROWS * NX)', '(size_t)D3_BXC * 4 * pad(NX, D3_BXE)'),
+    ('(size_t)wig::padded_size(NY * D3_YC)', '(size_t)D3_BYC * wig::blk_stride(pad(NY, D3_BYE), D3_BYC)'),
+    ('(size_t)wig::padded_size(4 * D3_ZC * NZ)', '(size_t)D3_BZC * wig::blk_stride(4 * pad(NZ, D3_BZE), D3_BZC)'),
+    ('emu_launch(gx, D3_XNT', 'emu_launch(gx + 1, D3_BXC * (NX / D3_BXE)'),
+    ('emu_launch(gy, D3_YNT', 'emu_launch(gy, D3_BYC * (NY / D3_BYE)'),
+    ('emu_launch(gz, D3_ZNT', 'emu_launch(gz, D3_BZC * (NZ / D3_BZE)'),
+    ('  // d3_plan / dirac3_create', '  const auto pad = [](int n, int e) { return n + n / std::min(e, 8); };\n  // d3_plan'),
+    ('a.n_z_cta = gz;', 'a.n_z_cta = gz;\n  const std::vector<double2> bx = wighost::block_twiddles(NX, D3_BXE), by = '
+     'wighost::block_twiddles(NY, D3_BYE), bz = wighost::block_twiddles(NZ, D3_BZE);\n  a.btw_x = bx.data(); '
+     'a.btw_y = by.data(); a.btw_z = bz.data();'),
+    ('#include "wig_jit_dirac3.cuh"', '#include "wig_jit_dirac3.cuh"\n#include "wig_batch_host.h"\n#include <algorithm>'))
+
+
+@pytest.mark.parametrize('n_x,n_y,row,col,sanitize', [(64, 128, (2, 4), (1, 4), 'address'), (128, 64, (4, 8), (4, 8), None),
+                                                      (64, 64, (4, 8), (2, 4), 'thread')])
+def test_blocked_dirac2d_passes_match_oracle(staged, n_x, n_y, row, col, sanitize):  # noqa: F811
+    from oracle.dirac2d import DiracOracle, DiracParams, spinor_particle_spin_up
+    exe = E.build(staged, _driver(staged, 'dirac2d_emu', DIRAC2D),
+                  dict(DIR_NX=n_x, DIR_NY=n_y, DIR_ROWS=1, DIR_RNT=32, DIR_RMB=1, DIR_C=1, DIR_CNT=32, DIR_CMB=1,
+                       DIR_SNT=64, DIR_B=1, DIR_BROWS=row[0], DIR_BRE=row[1], DIR_BRMB=1, DIR_BC=col[0],
+                       DIR_BCE=col[1], DIR_BCMB=1), sanitize)
+    prm = DiracParams(n_x, n_y, E.XA, E.YA, E.DT, mass=E.MASS, c=E.C, A0=E.A[0], A1=E.A[1], A2=E.A[2], A3=E.A[3],
+                      constants='exact')
+    psi0 = spinor_particle_spin_up(prm, (2., 1.), lambda x, y: np.exp(-(x * x + y * y) / 4.))
+    psi0 = np.ascontiguousarray(psi0, dtype=np.complex128)
+    steps = 2
+    fin, fout, fobs = (os.path.join(staged, n) for n in ('bd_in.bin', 'bd_out.bin', 'bd_obs.bin'))
+    psi0.tofile(fin)
+    r = subprocess.run([exe, fin, fout, fobs, str(steps)] + [repr(v) for v in (E.XA, E.YA, E.DT, E.MASS, E.C)],
+                       capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stderr[-2000:]
+    ref_obs, ref = DiracOracle(prm).run(psi0, steps)
+    got, obs = np.fromfile(fout, dtype=np.complex128).reshape(4, n_y, n_x), np.fromfile(fobs).reshape(steps, 10)
+    assert rel_l2(got, ref) < 1e-12
+    scale = np.maximum(np.abs(ref_obs).max(axis=0), 1e-3)
+    assert np.all(np.abs(obs - ref_obs) / scale < 1e-10), (obs - ref_obs) / scale
+
+
+@pytest.mark.parametrize('dims,x,y,z,cap,sanitize', [((32, 64, 32), (8, 8), (8, 16), (8, 8), 3, 'address'),
+                                                     ((64, 32, 32), (4, 4), (4, 4), (4, 4), 5, 'thread')])
+def test_blocked_dirac3d_passes_match_oracle(staged, dims, x, y, z, cap, sanitize):  # noqa: F811
+    """`cap` CTAs a pass: each takes several tiles, so a tile's loads follow the previous tile's exchange."""
+    from oracle.dirac3d import Dirac3DOracle, Dirac3DParams, spinor_particle_spin_up_3d
+    n_x, n_y, n_z = dims
+    macros = dict(D3_NX=n_x, D3_NY=n_y, D3_NZ=n_z, D3_ROWS=1, D3_XNT=32, D3_YC=2, D3_YNT=32, D3_ZC=1, D3_ZNT=32,
+                  D3_SNT=64, D3_XR=8, D3_YR=8, D3_ZR=8, D3_XMB=1, D3_YMB=1, D3_ZMB=1, D3_B=1)
+    for axis, (lines, e) in zip('XYZ', (x, y, z)):
+        macros.update({'D3_B%sC' % axis: lines, 'D3_B%sE' % axis: e, 'D3_B%sMB' % axis: 1})
+    exe = E.build(staged, _driver(staged, 'dirac3d_emu', DIRAC3D), macros, sanitize)
+    prm = Dirac3DParams(n_x, n_y, n_z, *E.D3A, E.D3DT, mass=1., c=137.036, A0=E.D3POT[0], A1=E.D3POT[1],
+                        A2=E.D3POT[2], A3=E.D3POT[3], constants='exact')
+    psi0 = spinor_particle_spin_up_3d(prm, (2., 0.5, 1.), lambda x, y, z: np.exp(-(x * x + y * y + z * z) / 4.))
+    psi0 = np.ascontiguousarray(psi0, dtype=np.complex128)
+    steps = 2
+    fin, fout, fobs = (os.path.join(staged, n) for n in ('b3_in.bin', 'b3_out.bin', 'b3_obs.bin'))
+    psi0.tofile(fin)
+    r = subprocess.run([exe, fin, fout, fobs, str(steps)] + [repr(v) for v in E.D3A + (E.D3DT, 1., 137.036)] + [str(cap)],
+                       capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stderr[-2000:]
+    ref_obs, ref = Dirac3DOracle(prm).run(psi0, steps)
+    got, obs = np.fromfile(fout, dtype=np.complex128).reshape(ref.shape), np.fromfile(fobs).reshape(steps, 12)
+    assert rel_l2(got, ref) < 1e-12
+    scale = np.maximum(np.abs(ref_obs).max(axis=0), 1e-3)
+    assert np.all(np.abs(obs - ref_obs) / scale < 1e-10), (obs - ref_obs) / scale

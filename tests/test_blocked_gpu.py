@@ -46,3 +46,34 @@ def test_blocked_passes_match_oracle(n_x, n_p, form):
     assert obs_close(got[:, :9], obs[:3, 1:10], TOL) < TOL
     # the negative area sums the points below zero: those within rounding of zero enter one sum and not the other
     assert np.max(np.abs(got[:, 9] - obs[:3, 10])) < 1e-10
+
+
+@pytest.mark.parametrize('n_x,n_y', [(64, 64), (128, 256), (64, 2048), (2048, 64), (512, 256), (1024, 512), (512, 1024)])
+def test_blocked_dirac2d_passes_match_oracle(n_x, n_y):
+    """4 elements a thread below 2^17 points, 8 from there; one to four columns a CTA."""
+    from instances import dirac_instance, dirac_obs
+    from oracle.dirac2d import DiracOracle, DiracParams, spinor_particle_spin_up
+    prm = DiracParams(n_x, n_y, 12., 8., 1e-4, mass=1., c=137.036, A0='-1./sqrt(x*x+y*y+0.5) + 3.*t*x', A1='-0.5*y',
+                      A2='0.5*x', A3='0.1*x')
+    psi0 = spinor_particle_spin_up(prm, (3., 1.), lambda x, y: np.exp(-(x * x + y * y) / 2.))
+    inst = dirac_instance(prm, psi0, 3)
+    inst.Run()
+    obs, psi = DiracOracle(prm).run(psi0, 3)
+    assert rel_l2(inst.Psi_end, psi) < TOL
+    assert obs_close(dirac_obs(inst), obs[:, :7], TOL) < TOL
+    assert obs_close(np.stack([inst.Px_average, inst.Py_average, inst.NormKept_average], 1), obs[:, 7:10], TOL) < TOL
+
+
+@pytest.mark.parametrize('dims', [(32, 32, 32), (64, 32, 128), (32, 128, 64), (128, 64, 64), (512, 32, 64), (32, 64, 512)])
+def test_blocked_dirac3d_passes_match_oracle(dims):
+    """4 elements a thread below 2^18 points, 8 from there (the y-pass 4, 8 or 16)."""
+    from instances import dirac3d_instance, dirac3d_obs
+    from oracle.dirac3d import Dirac3DOracle, Dirac3DParams, spinor_particle_spin_up_3d
+    prm = Dirac3DParams(*dims, 10., 8., 9., 1e-4, mass=1., c=137.036, A0='-1./sqrt(x*x+y*y+z*z+0.5) + 2.*t*z',
+                        A1='-0.5*y', A2='0.5*x', A3='0.1*z')
+    psi0 = spinor_particle_spin_up_3d(prm, (3., 1., 0.5), lambda x, y, z: np.exp(-(x * x + y * y + z * z) / 4.))
+    inst = dirac3d_instance(prm, psi0, 3)
+    inst.Run()
+    obs, psi = Dirac3DOracle(prm).run(psi0, 3)
+    assert rel_l2(inst.Psi_end, psi) < TOL
+    assert obs_close(dirac3d_obs(inst), obs, TOL) < TOL
