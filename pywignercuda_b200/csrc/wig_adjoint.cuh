@@ -49,6 +49,9 @@ struct AArgs {
   const double* ths;      // [n_p] theta / n_p
   double2* pend;          // [1] pending normalisation 1/s of the state (damped forward)
   double2* coef;          // [2] (1/conj(s), -conj(beta)) of the adjoint step being run
+  // stage twiddles of the register-blocked complex128 passes (BlockFft); null for complex64
+  const double2* btw_x;
+  const double2* btw_p;
 };
 
 template <class C> struct CScalar;
@@ -99,7 +102,9 @@ __device__ __forceinline__ int adj_col(int warp, int grp) {
 // x-pass, one warp per CTA, rf_spw(NX) rows per warp: out = K (s in) (sgn = +1)
 // or K^H in (sgn = -1), s = *pend when use_pend, else 1; in and out may alias.
 // The spectrum is staged in natural order in the row's exchange region and the
-// kinetic factor applied there in a rolled loop (one copy of the factor code).
+// kinetic factor applied there, eight frequencies at a time: a lone warp per SM runs a
+// one-by-one loop at the latency of its table load and sincospi (complex64 256^2 gradient
+// of 60 steps: 4.39 -> 3.24 ms, bit for bit the same).
 template <class C, int NX, int NP>
 __device__ __forceinline__ void adj_xpass(const AArgs& a, const C* in, C* out, double sgn, int use_pend) {
   typedef RegFft<C, NX> F;
@@ -111,6 +116,8 @@ __device__ __forceinline__ void adj_xpass(const AArgs& a, const C* in, C* out, d
   const int lane = threadIdx.x & 31, grp = lane / G, g = lane % G;
   const int row = blockIdx.x * SPW + grp;
   WIG_BOUNDS_CHECK("adjoint x-pass row", row, NP);
+  grid_wait();
+  grid_launch_next();
   const C* src = in + (size_t)row * NX;
   const C s = use_pend ? cmk<C>(a.pend->x, a.pend->y) : cmk<C>(1., 0.);
   C v[E];
@@ -123,7 +130,7 @@ __device__ __forceinline__ void adj_xpass(const AArgs& a, const C* in, C* out, d
   for (int e = 0; e < E; ++e) x.put(g * Q + e / G + E * (e % G), v[e]);
   __syncwarp();
   const double cq = a.dt * a.dp * a.dlambda * (double)ashift(row, NP) / (a.mass * 6.283185307179586477);
-#pragma unroll 1
+#pragma unroll 8
   for (int k = g; k < NX; k += G) x.put(k, cmul(x.get(k), adj_turn<C>(cq * (double)ashift(k, NX), __ldg(a.rtab + k), sgn)));
   __syncwarp();
 #pragma unroll
@@ -146,6 +153,7 @@ __device__ __forceinline__ void moyal_coeffs(const AArgs& a, double x, double ep
 // Coalesced load / store of a CT x NP tile of columns [col0, col0 + CT) (swizzled tile).
 template <class C, int NP, int CT, int NT>
 __device__ __forceinline__ void adj_tile_load(C* tile, const C* src, int nx, int col0) {
+#pragma unroll 8
   for (int e = threadIdx.x; e < CT * NP; e += NT) {
     const int k = e / CT, c = e & (CT - 1);
     WIG_BOUNDS_CHECK("adjoint tile column", col0 + c, nx);
@@ -154,6 +162,7 @@ __device__ __forceinline__ void adj_tile_load(C* tile, const C* src, int nx, int
 }
 template <class C, int NP, int CT, int NT>
 __device__ __forceinline__ void adj_tile_store(const C* tile, C* dst, int nx, int col0) {
+#pragma unroll 8
   for (int e = threadIdx.x; e < CT * NP; e += NT) {
     const int k = e / CT, c = e & (CT - 1);
     WIG_BOUNDS_CHECK("adjoint tile column", col0 + c, nx);
@@ -224,6 +233,8 @@ __device__ __forceinline__ void adj_ppass(const AArgs& a, const C* in, C* out, C
   C* t1 = t0 + CT * NP;
   const C* tw = reinterpret_cast<const C*>(a.tw_p);
   const int col0 = blockIdx.x * CT;
+  grid_wait();
+  grid_launch_next();
   adj_tile_load<C, NP, CT, NT>(t0, in, NX, col0);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / G, g = lane % G;
@@ -242,7 +253,7 @@ __device__ __forceinline__ void adj_ppass(const AArgs& a, const C* in, C* out, C
   double al, be;
   moyal_coeffs(a, a.dx * (double)ashift(col, NX), eps, &al, &be);
   const double mm = __ldg(a.mm + col);
-#pragma unroll 1
+#pragma unroll 8
   for (int k = g; k < NP; k += G) {
     const double j = (double)ashift(k, NP);
     x0.put(k, cmul(x0.get(k), adj_turn<C>(j * fma(be, j * j, al), __ldg(a.rth + k) * mm, 1.)));
@@ -295,6 +306,8 @@ __device__ __forceinline__ void adj_ppass_T(const AArgs& a, C* lam, const C* Y, 
   C* t1 = t0 + CT * NP;
   const C* tw = reinterpret_cast<const C*>(a.tw_p);
   const int col0 = blockIdx.x * CT;
+  grid_wait();
+  grid_launch_next();
   adj_tile_load<C, NP, CT, NT>(t0, lam, NX, col0);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / G, g = lane % G;
@@ -349,7 +362,7 @@ __device__ __forceinline__ void adj_ppass_T(const AArgs& a, C* lam, const C* Y, 
   const double mm = __ldg(a.mm + col);
   const double h = 0.5 * a.hbar * a.dtheta;   // u = h j
   double gq[3] = {0., 0., 0.};
-#pragma unroll 1
+#pragma unroll 8
   for (int k = g; k < NP; k += G) {
     const double j = (double)ashift(k, NP);
     const C d = adj_turn<C>(j * fma(be, j * j, al), __ldg(a.rth + k) * mm, 1.);
@@ -376,6 +389,261 @@ __device__ __forceinline__ void adj_ppass_T(const AArgs& a, C* lam, const C* Y, 
   adj_block_sum<NT, 3>(gq, part + 3 * blockIdx.x);
   __syncthreads();
   adj_tile_store<C, NP, CT, NT>(t0, lam, NX, col0);
+}
+
+// ------------------------------------------------------------------ register-blocked complex128 passes
+// One 512^2 grid on the passes above is 256 single-warp CTAs (x) or 128 two-warp CTAs (p) of 32
+// elements a thread: about two warps per SM, 30 and 44 us a pass, and a damped step has one (forward)
+// or three (adjoint) single-warp launches besides for its sums.  Here a thread holds 4 or 8 elements
+// (BlockFft), and each sum is taken by the kernel that needs it:
+//   forward   x-pass: scales its input by the previous step's 1/s from the p-pass's CTA partials (the
+//             last CTA of the grid records s); p-pass.
+//   adjoint   p-pass: forms its two scalars from the dot partials; x-pass: leaves the dot partials
+//             of the next step's U, and its last CTA sums the gradient partials.
+
+// sum over i < n of part[NV i + q] (q < NV) to every thread
+template <int NT, int NV>
+__device__ __forceinline__ void adj_collect(const double* part, int n, double (&out)[NV]) {
+  __shared__ double red[NT / 32][NV];
+  double v[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) v[q] = 0.;
+  for (int i = threadIdx.x; i < n; i += NT)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] += part[(size_t)NV * i + q];
+  block_sum<NT, NV>(v, red);
+#pragma unroll
+  for (int q = 0; q < NV; ++q) out[q] = red[0][q];
+}
+
+// this CTA's share of sum conj(v) U into dot[2 blockIdx.x ..]; U: the thread's first element
+template <int E, int T, int NT>
+__device__ __forceinline__ void adj_dot_rows(const double2 (&v)[E], const double2* U, double* dot) {
+  __shared__ double red[NT / 32][2];
+  double d[2] = {0., 0.};
+#pragma unroll
+  for (int m = 0; m < E; ++m) {
+    const double2 u = U[T * m];
+    d[0] = fma(v[m].x, u.x, fma(v[m].y, u.y, d[0]));
+    d[1] = fma(v[m].x, u.y, fma(-v[m].y, u.x, d[1]));
+  }
+  block_sum<NT, 2>(d, red);
+  if (threadIdx.x < 2) dot[2 * blockIdx.x + threadIdx.x] = red[0][threadIdx.x];
+}
+
+// x-pass: out = K (in / s) or K^H in, ROWS rows per CTA.  part (may be null): 2 n_part doubles, the
+// partials of the sum behind s (s_out[step], when given, records it).  U (may be null): plane of the
+// next adjoint step, whose dot partials with out go to dot[2 blockIdx.x ..].  gpart (may be null):
+// 3 n_g gradient partials, summed into grad[3 step ..].  Shared memory: ROWS exchange regions.
+template <int NX, int NP, int ROWS, int E>
+__device__ __forceinline__ void adj_xpass_blk(const AArgs& a, const double2* in, double2* out, double sgn,
+                                              const double* part, int n_part, double2* s_out, long long step,
+                                              const double2* U, double* dot, const double* gpart, int n_g,
+                                              double* grad) {
+  typedef BlockFft<double2, NX, E> F;
+  constexpr int T = F::T, NT = ROWS * T;
+  static_assert(NT % 32 == 0 && (T % 32 == 0 || 32 % T == 0), "x-pass rows per CTA");
+  extern __shared__ double2 smd[];
+  grid_wait();
+  grid_launch_next();
+  if (blockIdx.x == NP / ROWS) {
+    if (part != nullptr && s_out != nullptr) {
+      double S[2];
+      adj_collect<NT, 2>(part, n_part, S);
+      if (threadIdx.x == 0) s_out[step] = make_double2(S[0] * a.dx * a.dp, S[1] * a.dx * a.dp);
+    }
+    if (gpart != nullptr) {
+      double g[3];
+      adj_collect<NT, 3>(gpart, n_g, g);
+      if (threadIdx.x < 3) grad[3 * step + threadIdx.x] = threadIdx.x == 0 ? g[0] : (threadIdx.x == 1 ? g[1] : g[2]);
+    }
+    return;
+  }
+  const int seq = threadIdx.x / T, t = threadIdx.x % T, row = blockIdx.x * ROWS + seq;
+  WIG_BOUNDS_CHECK("adjoint x-pass row", row, NP);
+  const size_t base = (size_t)row * NX + t;
+  double2 v[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) v[m] = in[base + T * m];
+  if (part != nullptr) {
+    double S[2];
+    adj_collect<NT, 2>(part, n_part, S);
+    const double2 sc = crecip(make_double2(S[0] * a.dx * a.dp, S[1] * a.dx * a.dp));
+#pragma unroll
+    for (int m = 0; m < E; ++m) v[m] = cmul(v[m], sc);
+  }
+  double2* X = smd + seq * F::REGION;
+  const auto sync = SeqSync<T, ROWS>::make(seq);
+  F::template run<false>(v, X, a.btw_x, t, sync);
+  const double cq = a.dt * a.dp * a.dlambda * (double)ashift(row, NP) / (a.mass * 6.283185307179586477);
+  apply_odd_factor<NX, E>(v, X, t, sync, [&](int k) {
+    return adj_turn<double2>(cq * (double)ashift(k, NX), __ldg(a.rtab + k), sgn);
+  });
+  F::template run<true>(v, X, a.btw_x, t, sync);
+#pragma unroll
+  for (int m = 0; m < E; ++m) out[base + T * m] = v[m];
+  if (U != nullptr) adj_dot_rows<E, T, NT>(v, U + base, dot);
+}
+
+// the same dot partials, of a lam that no x-pass has just left (a sweep's first step): the rows and the
+// order of adj_xpass_blk, so that a sweep equals its steps bit for bit
+template <int NX, int NP, int ROWS, int E>
+__device__ __forceinline__ void adj_dot_blk(const double2* lam, const double2* U, double* dot) {
+  constexpr int T = NX / E, NT = ROWS * T;
+  grid_wait();
+  grid_launch_next();
+  const size_t base = (size_t)(blockIdx.x * ROWS + threadIdx.x / T) * NX + threadIdx.x % T;
+  double2 v[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) v[m] = lam[base + T * m];
+  adj_dot_rows<E, T, NT>(v, U + base, dot);
+}
+
+// the Moyal factor of column x for every frequency, through the exchange region (apply_odd_factor)
+template <int NP>
+__device__ __forceinline__ double2 adj_moyal(const AArgs& a, double al, double be, double mm, int k) {
+  const double j = (double)ashift(k, NP);
+  return adj_turn<double2>(j * fma(be, j * j, al), __ldg(a.rth + k) * mm, 1.);
+}
+
+// forward p-pass (adj_ppass), C columns per CTA; damped: out holds U and part the CTA's share of its sum.
+template <int NX, int NP, int C, int E>
+__device__ __forceinline__ void adj_ppass_blk(const AArgs& a, const double2* in, double2* out, double eps,
+                                              double* part) {
+  typedef BlockFft<double2, NP, E> F;
+  constexpr int T = F::T, NT = C * T, RS = blk_stride(F::REGION, C);
+  static_assert(NT % 32 == 0 && C <= 32, "p-pass columns per CTA");
+  extern __shared__ double2 smd[];
+  const int c = threadIdx.x % C, t = threadIdx.x / C, col = blockIdx.x * C + c;
+  WIG_BOUNDS_CHECK("adjoint p-pass column", col, NX);
+  const size_t base = (size_t)t * NX + col;
+  double2 v[E], A[E];
+#pragma unroll
+  for (int m = 0; m < E; ++m) v[m] = in[base + (size_t)(T * m) * NX];
+  double2* X = smd + c * RS;
+  const auto sync = SeqSync<NT, 1>::make(0);
+  double al, be;
+  moyal_coeffs(a, a.dx * (double)ashift(col, NX), eps, &al, &be);
+  const double mm = __ldg(a.mm + col);
+  const int n_it = a.damped ? 4 : 1;
+#pragma unroll 1
+  for (int it = 0; it < n_it; ++it) {
+    if (it > 0) {
+      const double* sfp = fresh(a.sfp + t);
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[m] = cscale(v[m], __ldg(sfp + T * m));
+    }
+    F::template run<false>(v, X, fresh(a.btw_p), t, sync);
+    if (it == 0) {
+      apply_odd_factor<NP, E>(v, X, t, sync, [&](int k) { return adj_moyal<NP>(a, al, be, mm, k); });
+    } else {
+      const double* ths = fresh(a.ths + t);
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[m] = cscale(v[m], __ldg(ths + T * m));
+    }
+    F::template run<true>(v, X, fresh(a.btw_p), t, sync);
+    if (it == 0) {
+#pragma unroll
+      for (int m = 0; m < E; ++m) A[m] = v[m];
+    } else {
+      const double ci = it == 1 ? a.cl1 : (it == 2 ? a.cl2 : a.cl3);
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[m] = make_double2(A[m].x - ci * v[m].y, A[m].y + ci * v[m].x);
+    }
+  }
+  double su[2] = {0., 0.};
+#pragma unroll
+  for (int m = 0; m < E; ++m) {
+    out[base + (size_t)(T * m) * NX] = v[m];
+    su[0] += v[m].x;
+    su[1] += v[m].y;
+  }
+  if (a.damped) {
+    __shared__ double red[NT / 32][2];
+    block_sum<NT, 2>(su, red);
+    if (threadIdx.x < 2) part[2 * blockIdx.x + threadIdx.x] = red[0][threadIdx.x];
+  }
+}
+
+// adjoint p-pass (adj_ppass_T), C columns per CTA: the scalars of N^H from the 2 n_dot dot partials
+// and s_in[step] (damped), the gradient partials into part[3 blockIdx.x ..].
+template <int NX, int NP, int C, int E>
+__device__ __forceinline__ void adj_ppass_T_blk(const AArgs& a, double2* lam, const double2* Y, double eps,
+                                                double* part, const double* dot, int n_dot, const double2* s_in,
+                                                long long step) {
+  typedef BlockFft<double2, NP, E> F;
+  constexpr int T = F::T, NT = C * T, RS = blk_stride(2 * F::REGION, C);
+  static_assert(NT % 32 == 0 && C <= 32, "p-pass columns per CTA");
+  extern __shared__ double2 smd[];
+  const int c = threadIdx.x % C, t = threadIdx.x / C, col = blockIdx.x * C + c;
+  WIG_BOUNDS_CHECK("adjoint p-pass column", col, NX);
+  const size_t base = (size_t)t * NX + col;
+  double2 w[2][E];   // [0] lam, [1] the Horner base of C^H, then Y
+#pragma unroll
+  for (int m = 0; m < E; ++m) w[0][m] = lam[base + (size_t)(T * m) * NX];
+  double2* X = smd + c * RS;
+  const auto sync = SeqSync<NT, 1>::make(0);
+  if (a.damped) {
+    double r[2];
+    adj_collect<NT, 2>(dot, n_dot, r);
+    const double2 s = s_in[step];
+    const double2 beta = cmul(make_double2(r[0] * a.dx * a.dp, r[1] * a.dx * a.dp), crecip(cmul(s, s)));
+    const double2 c1 = crecip(cconj(s)), c0 = make_double2(-beta.x, beta.y);
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      w[0][m] = cadd(cmul(w[0][m], c1), c0);
+      w[1][m] = w[0][m];
+    }
+#pragma unroll 1
+    for (int it = 0; it < 3; ++it) {
+      F::template run<false>(w[0], X, fresh(a.btw_p), t, sync);
+      const double* ths = fresh(a.ths + t);
+#pragma unroll
+      for (int m = 0; m < E; ++m) w[0][m] = cscale(w[0][m], __ldg(ths + T * m));
+      F::template run<true>(w[0], X, fresh(a.btw_p), t, sync);
+      const double ci = -(it == 0 ? a.cl1 : (it == 1 ? a.cl2 : a.cl3));   // conj(i c) = -i c
+      const double* sfp = fresh(a.sfp + t);
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        const double f = ci * __ldg(sfp + T * m);
+        w[0][m] = make_double2(w[1][m].x - f * w[0][m].y, w[1][m].y + f * w[0][m].x);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < E; ++m) w[1][m] = Y[base + (size_t)(T * m) * NX];
+  F::template run_many<false>(w, X, fresh(a.btw_p), t, sync);
+  const double xc = a.dx * (double)ashift(col, NX);
+  double al, be;
+  moyal_coeffs(a, xc, eps, &al, &be);
+  const double mm = __ldg(a.mm + col);
+  const double h = 0.5 * a.hbar * a.dtheta;   // u = h j
+  sync();
+#pragma unroll 2
+  for (int k = t; k <= NP / 2; k += T) X[k] = adj_moyal<NP>(a, al, be, mm, k);
+  sync();
+  double gq[3] = {0., 0., 0.};
+#pragma unroll
+  for (int m = 0; m < E; ++m) {
+    const int k = t + T * m;
+    const double2 d = k <= NP / 2 ? X[k] : cconj(X[NP - k]);
+    const double2 U = w[0][m], yd = cmul(w[1][m], d);
+    const double re = U.y * yd.x - U.x * yd.y;   // Re(i conj(U) yd)
+    const double j = (double)ashift(k, NP), u = h * j;
+    gq[0] += j * re;
+    gq[1] += xc * u * (xc * xc + u * u) * re;
+    gq[2] += xc * u * re;
+    w[0][m] = cmul(U, cconj(d));
+  }
+  gq[0] *= a.dt * a.dtheta;
+  gq[1] *= 8. * a.dt / a.hbar;
+  gq[2] *= 4. * a.dt / a.hbar;
+  F::template run<true>(w[0], X, fresh(a.btw_p), t, sync);
+#pragma unroll
+  for (int m = 0; m < E; ++m) lam[base + (size_t)(T * m) * NX] = w[0][m];
+  __shared__ double red[NT / 32][3];
+  block_sum<NT, 3>(gq, red);
+  if (threadIdx.x < 3) part[3 * blockIdx.x + threadIdx.x] = red[0][threadIdx.x];
 }
 
 }  // namespace wig

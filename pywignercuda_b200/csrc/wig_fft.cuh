@@ -377,6 +377,13 @@ template <class C, int N, int E> struct BlockFft {
     const int at = N <= E * E ? 1 : E;   // the short stage's sub-length
     return ns == at ? shrt : E;
   }
+  // entries of the twiddle table
+  __host__ __device__ static constexpr int table() {
+    int n = 0;
+    for (int ns = 1; ns < N; ns *= radix(ns))
+      if (ns > 1) n += (radix(ns) == 16 ? 6 : radix(ns) - 1) * ns;
+    return n;
+  }
   template <int NS, int R> __device__ __forceinline__ static int slot(int i) {
     if (NS >= 8 || (NS > 1 && R < 4)) return i;
     return NS * R < 8 ? i + (i >> 3) : i + NS * (i / (NS * R));   // at most N / min(R, 8) pads

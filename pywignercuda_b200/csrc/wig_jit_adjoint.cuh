@@ -15,6 +15,54 @@ typedef double2 WigaC;
 typedef float2 WigaC;
 #endif
 
+// WIGA_B 1 (complex128): the passes on the register-blocked transform: WIGA_BXR rows / WIGA_BPC columns
+// a CTA, WIGA_BXE / WIGA_BPE elements a thread, WIGA_BXMB / WIGA_BPMB CTAs per SM
+#ifndef WIGA_B
+#define WIGA_B 0
+#endif
+#if WIGA_B
+extern "C" __global__ void __launch_bounds__(WIGA_BXR * (WIGA_NX / WIGA_BXE), WIGA_BXMB)
+wiga_bx(wig::AArgs a, const double2* in, double2* out, double sgn, const double* part, int n_part, double2* s_out,
+        long long step, const double2* U, double* dot, const double* gpart, int n_g, double* grad) {
+  wig::adj_xpass_blk<WIGA_NX, WIGA_NP, WIGA_BXR, WIGA_BXE>(a, in, out, sgn, part, n_part, s_out, step, U, dot, gpart,
+                                                            n_g, grad);
+}
+
+extern "C" __global__ void __launch_bounds__(WIGA_BPC * (WIGA_NP / WIGA_BPE), WIGA_BPMB)
+wiga_bp(wig::AArgs a, const double2* in, double2* out, const double* eps, long long step, double* part) {
+  wig::grid_wait();
+  wig::grid_launch_next();
+  wig::adj_ppass_blk<WIGA_NX, WIGA_NP, WIGA_BPC, WIGA_BPE>(a, in, out, eps[step], part);
+}
+
+extern "C" __global__ void __launch_bounds__(WIGA_BPC * (WIGA_NP / WIGA_BPE), WIGA_BPMB)
+wiga_bpt(wig::AArgs a, double2* lam, const double2* Y, const double* eps, long long step, double* part,
+         const double* dot, int n_dot, const double2* s_in) {
+  wig::grid_wait();
+  wig::grid_launch_next();
+  wig::adj_ppass_T_blk<WIGA_NX, WIGA_NP, WIGA_BPC, WIGA_BPE>(a, lam, Y, eps[step], part, dot, n_dot, s_in, step);
+}
+
+extern "C" __global__ void __launch_bounds__(WIGA_BXR * (WIGA_NX / WIGA_BXE))
+wiga_bdot(const double2* lam, const double2* U, double* dot) {
+  wig::adj_dot_blk<WIGA_NX, WIGA_NP, WIGA_BXR, WIGA_BXE>(lam, U, dot);
+}
+
+// the end of a damped forward sweep: W = in / s, s from the last p-pass's partials (recorded in s_out[step])
+extern "C" __global__ void __launch_bounds__(256)
+wiga_bscale(wig::AArgs a, const double2* in, double2* W, long long n, const double* part, int n_part, double2* s_out,
+            long long step) {
+  wig::grid_wait();
+  wig::grid_launch_next();
+  double S[2];
+  wig::adj_collect<256, 2>(part, n_part, S);
+  const double2 s = make_double2(S[0] * a.dx * a.dp, S[1] * a.dx * a.dp), sc = wig::crecip(s);
+  if (s_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) s_out[step] = s;
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (long long)gridDim.x * 256)
+    W[i] = wig::cmul(in[i], sc);
+}
+#else
+
 // x-pass: one warp per CTA (rf_spw(n_x) rows).  sgn = +1: K, -1: K^H; use_pend:
 // scale the input by the pending normalisation on load.
 extern "C" __global__ void __launch_bounds__(32)
@@ -34,6 +82,8 @@ wiga_ppass(wig::AArgs a, const WigaC* in, WigaC* out, WigaC* U_out, const double
 // normalisation 1/s, and s into s_out[step] (when given).  One warp.
 extern "C" __global__ void __launch_bounds__(32)
 wiga_fwd_finalize(wig::AArgs a, const double* part, int n, double2* s_out, long long step) {
+  wig::grid_wait();
+  wig::grid_launch_next();
   double re = 0., im = 0.;
   for (int i = threadIdx.x; i < n; i += 32) { re += part[2 * i]; im += part[2 * i + 1]; }
 #pragma unroll
@@ -61,22 +111,12 @@ wiga_reset_pend(wig::AArgs a) {
   if (threadIdx.x == 0) *a.pend = make_double2(1., 0.);
 }
 
-// CTA partials of sum conj(lam) U (FP64), grid-stride over the plane
-extern "C" __global__ void __launch_bounds__(256)
-wiga_dot(const WigaC* lam, const WigaC* U, long long n, double* part) {
-  double v[2] = {0., 0.};
-  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
-    const WigaC l = lam[i], u = U[i];
-    v[0] += (double)l.x * (double)u.x + (double)l.y * (double)u.y;
-    v[1] += (double)l.x * (double)u.y - (double)l.y * (double)u.x;
-  }
-  wig::adj_block_sum<256, 2>(v, part + 2 * blockIdx.x);
-}
-
 // The adjoint of the normalisation of step `step`: lam_U = coef[0] lam + coef[1]
 // with coef[0] = 1 / conj(s), coef[1] = -conj(dX dP r / s^2), r = sum conj(lam) U.  One warp.
 extern "C" __global__ void __launch_bounds__(32)
 wiga_adj_coef(wig::AArgs a, const double* part, int n, const double2* s_in, long long step) {
+  wig::grid_wait();
+  wig::grid_launch_next();
   double re = 0., im = 0.;
   for (int i = threadIdx.x; i < n; i += 32) { re += part[2 * i]; im += part[2 * i + 1]; }
 #pragma unroll
@@ -103,6 +143,11 @@ wiga_ppass_T(wig::AArgs a, WigaC* lam, const WigaC* Y, const double* eps, long l
 // q = 0: dL/d eps_step, 1: dL/dv4 share, 2: dL/dv2 share
 extern "C" __global__ void __launch_bounds__(32)
 wiga_grad_finalize(const double* part, int n, double* grad, long long step) {
+  // one CTA per step of a chunk: CTA i sums the partials of step `step` - i
+  wig::grid_wait();
+  wig::grid_launch_next();
+  part += (size_t)blockIdx.x * 3 * n;
+  step -= blockIdx.x;
   double s[3] = {0., 0., 0.};
   for (int i = threadIdx.x; i < n; i += 32)
 #pragma unroll
@@ -115,3 +160,18 @@ wiga_grad_finalize(const double* part, int n, double* grad, long long step) {
 #pragma unroll
     for (int q = 0; q < 3; ++q) grad[3 * step + q] = s[q];
 }
+
+// CTA partials of sum conj(lam) U (FP64), grid-stride over the plane
+extern "C" __global__ void __launch_bounds__(256)
+wiga_dot(const WigaC* lam, const WigaC* U, long long n, double* part) {
+  wig::grid_wait();
+  wig::grid_launch_next();
+  double v[2] = {0., 0.};
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+    const WigaC l = lam[i], u = U[i];
+    v[0] += (double)l.x * (double)u.x + (double)l.y * (double)u.y;
+    v[1] += (double)l.x * (double)u.y - (double)l.y * (double)u.x;
+  }
+  wig::adj_block_sum<256, 2>(v, part + 2 * blockIdx.x);
+}
+#endif

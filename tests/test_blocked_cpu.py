@@ -114,6 +114,61 @@ DIRAC3D = (
      'a.btw_y = by.data(); a.btw_z = bz.data();'),
     ('#include "wig_jit_dirac3.cuh"', '#include "wig_jit_dirac3.cuh"\n#include "wig_batch_host.h"\n#include <algorithm>'))
 
+ADJOINT_LAUNCHES = """
+  // wiga_forward and wiga_adjoint_sweep (csrc/wig_adjoint.cu: forward_blk, adjoint_blk)
+  const auto pad = [](int n, int e) { return n + n / std::min(e, 8); };
+  const std::vector<double2> bx = wighost::block_twiddles(nx, WIGA_BXE), bp = wighost::block_twiddles(np, WIGA_BPE);
+  a.btw_x = bx.data(); a.btw_p = bp.data();
+  const int bxn = np / WIGA_BXR, bxt = WIGA_BXR * (nx / WIGA_BXE), bpn = nx / WIGA_BPC, bpt = WIGA_BPC * (np / WIGA_BPE);
+  const size_t sbx = (size_t)WIGA_BXR * pad(nx, WIGA_BXE) * 16;
+  const size_t sbp = (size_t)WIGA_BPC * wig::blk_stride(pad(np, WIGA_BPE), WIGA_BPC) * 16;
+  const size_t sbt = (size_t)WIGA_BPC * wig::blk_stride(2 * pad(np, WIGA_BPE), WIGA_BPC) * 16;
+  std::vector<double> bpart(3 * bpn), dot(2 * bxn);
+  double* part_p = bpart.data();
+  const double2* cur = W.data();
+  for (long n = 0; n < n_steps; ++n) {
+    double2* Yn = Y.data() + (size_t)n * plane;
+    double2* out = damped ? U.data() + (size_t)n * plane : W.data();
+    const bool pend = damped && n > 0;
+    emu_launch(bxn + 1, bxt, [&] { wiga_bx(a, cur, Yn, 1., pend ? part_p : nullptr, bpn, pend ? s.data() : nullptr,
+                                           (long long)(n - 1), nullptr, nullptr, nullptr, 0, nullptr); }, sbx);
+    emu_launch(bpn, bpt, [&] { wiga_bp(a, Yn, out, eps.data(), (long long)n, part_p); }, sbp);
+    cur = out;
+  }
+  if (damped) emu_launch(4, 256, [&] { wiga_bscale(a, cur, W.data(), (long long)plane, part_p, bpn, s.data(),
+                                                   (long long)(n_steps - 1)); });
+  for (long n = n_steps - 1; n >= 0; --n) {
+    const double2* Yn = Y.data() + (size_t)n * plane;
+    if (damped && n == n_steps - 1)
+      emu_launch(bxn, bxt, [&] { wiga_bdot(lam.data(), U.data() + (size_t)n * plane, dot.data()); });
+    emu_launch(bpn, bpt, [&] { wiga_bpt(a, lam.data(), Yn, eps.data(), (long long)n, part_p, dot.data(), bxn, s.data()); }, sbt);
+    const double2* Un = damped && n > 0 ? U.data() + (size_t)(n - 1) * plane : nullptr;
+    emu_launch(bxn + 1, bxt, [&] { wiga_bx(a, lam.data(), lam.data(), -1., nullptr, 0, nullptr, (long long)n, Un,
+                                           dot.data(), part_p, bpn, grad.data()); }, sbx);
+  }
+  if (!write_all(argv[4]"""
+
+
+def _adjoint_driver(staged):
+    """tests/emu/adjoint_emu.cpp with the launches of the register-blocked complex128 passes."""
+    with open(os.path.join(E.EMU, 'adjoint_emu.cpp')) as f:
+        head, rest = f.read().split('  // wiga_forward with the records kept')
+    tail = rest.split('  if (!write_all(argv[4]')[1]
+    src = head.replace('#include <cstdlib>', '#include <algorithm>\n#include <cstdlib>') + ADJOINT_LAUNCHES + tail
+    with open(os.path.join(staged, 'adjoint_emu_blocked.cpp'), 'w') as f:
+        f.write(src)
+    return 'adjoint_emu_blocked.cpp'
+
+
+@pytest.mark.parametrize('x,p,gamma,sanitize', [((1, 4), (2, 4), 0.1, 'address'), ((4, 8), (4, 8), 0.1, 'thread'),
+                                                ((2, 4), (4, 8), 0., None)])
+def test_blocked_adjoint_matches_twin(staged, monkeypatch, x, p, gamma, sanitize):  # noqa: F811
+    """The complex128 forward and adjoint sweeps against the twin, by test_emu_cpu's test with this driver."""
+    macros = dict(WIGA_B=1, WIGA_BXR=x[0], WIGA_BXE=x[1], WIGA_BXMB=1, WIGA_BPC=p[0], WIGA_BPE=p[1], WIGA_BPMB=1)
+    build = E.build
+    monkeypatch.setattr(E, 'build', lambda dst, source, m: build(dst, _adjoint_driver(dst), dict(m, **macros), sanitize))
+    E.test_adjoint_device_code_matches_twin(staged, 1, gamma)
+
 
 @pytest.mark.parametrize('n_x,n_y,row,col,sanitize', [(64, 128, (2, 4), (1, 4), 'address'), (128, 64, (4, 8), (4, 8), None),
                                                       (64, 64, (4, 8), (2, 4), 'thread')])
