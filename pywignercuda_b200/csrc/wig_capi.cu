@@ -530,8 +530,8 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
   // ---- register-blocked passes (BlockFft)
   {
     const bool stockham = P->rf || getenv("WIG_TILING") || getenv("WIG_RADIX");   // tile overrides of the other forms
-    P->bx = !stockham && NX >= 64 ? 1 : 0;
-    P->bp = !stockham && NP >= 64 ? 1 : 0;
+    P->bx = !stockham && NX >= 32 ? 1 : 0;
+    P->bp = !stockham && NP >= 32 ? 1 : 0;
     // Elements a thread: as many as the grid leaves threads for.  16 (two stage boundaries in
     // shared memory up to 4096 points, 128 registers, 16 warps per SM) from 2^19 points, 8 from
     // 2^17, below that 4, where the step is a chain of latencies and more warps shorten it.
@@ -1415,12 +1415,12 @@ static int dirac_plan(const dirac_desc* d, DiracPlan* P) {
   P->n_col = NX / P->cc;
   P->smem_row = wig::padded_size(4 * P->rows * NX) * (int)sizeof(double2);
   P->smem_col = wig::padded_size(4 * P->cc * NY) * (int)sizeof(double2);
-  // ---- register-blocked passes (axes of at least 64 points; a tile override keeps the Stockham ones):
+  // ---- register-blocked passes (axes of at least 32 points; a tile override keeps the Stockham ones):
   // 8 elements of four components a thread (255 registers, 8 warps per SM), 4 on grids below 2^17
   // points, where more warps shorten the chains (step, us: 512^2 38 / 47 with 8 / 4, 256^2 24 / 20,
   // 128 x 64 19 / 14; the Stockham passes 68 at 512^2).  Column tiles of 4 where the grid is wide
   // enough and the tile fits (512^2: 36.8 / 38.4 / 44.9 us with 4 / 2 / 1).
-  P->blk = NX >= 64 && NY >= 64 && !getenv("WIG_DIRAC_TILING") ? 1 : 0;
+  P->blk = NX >= 32 && NY >= 32 && !getenv("WIG_DIRAC_TILING") ? 1 : 0;
   if (P->blk) {
     const int e = (long)NX * NY >= (1L << 17) ? 8 : 4;
     P->bre = P->bce = e;

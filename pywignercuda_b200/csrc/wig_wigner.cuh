@@ -754,7 +754,7 @@ __device__ __forceinline__ void odm_ppass_body(const WigArgs& a, double2* __rest
 }
 
 // ------------------------------------------------------------------ register-blocked passes
-// The passes of axes of at least 64 points on BlockFft (wig_fft.cuh): a thread
+// The passes of axes of at least 32 points on BlockFft (wig_fft.cuh): a thread
 // holds E elements of its row or column from the global load to the global
 // store; shared memory carries only the transforms' stage boundaries.
 //

@@ -27,6 +27,7 @@ CASES = [
     (64, 64, (2, 4), (4, 4), 'odm', 'thread'),
     (64, 128, (2, 4), (1, 4), 'gp', 'thread'),
     (64, 64, (4, 8), (4, 8), 'gp', None),
+    (32, 32, (8, 8), (4, 4), 'cl', 'thread'),
 ]
 
 

@@ -1,7 +1,7 @@
 """The register-blocked complex128 Wigner2D passes on the GPU against the oracle,
-over the tiles that the planner picks: axes from 64 to 4096 points, 4, 8 and 16
-elements a thread (grids below 2^18, 2^19 points and above; the last with the
-Caldeira-Leggett base in tensor memory), one axis of 32 points left to the
+over the tiles that the planner picks: axes from 32 to 4096 points, 4, 8 and 16
+elements a thread (grids below 2^17, 2^19 points and above; the last with the
+Caldeira-Leggett base in tensor memory), one axis of 16 points left to the
 Stockham passes.  Bars: those of the other complex128 paths (relative L2 1e-10,
 observables 1e-10 of their scale)."""
 import numpy as np
@@ -17,7 +17,8 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-10
 POT, DPOT = '0.05*pow(x,4) - pow(x,2) + 0.1*x*sin(3.*t)', '0.2*pow(x,3) - 2.*x + 0.1*sin(3.*t)'
 
-CASES = [(64, 64, 'cl'), (128, 64, 'none'), (64, 256, 'odm2'), (512, 32, 'cl'), (32, 512, 'odm'), (2048, 64, 'kvn'),
+CASES = [(32, 32, 'cl'), (32, 64, 'gp'), (64, 32, 'odm2'), (32, 4096, 'cl'), (16, 64, 'none'), (512, 16, 'odm'),
+         (64, 64, 'cl'), (128, 64, 'none'), (64, 256, 'odm2'), (512, 32, 'cl'), (32, 512, 'odm'), (2048, 64, 'kvn'),
          (64, 2048, 'cl'), (4096, 64, 'cl'), (64, 4096, 'cl'), (512, 512, 'cl'), (1024, 256, 'odm'),
          (512, 1024, 'cl'), (1024, 1024, 'kvn'), (256, 2048, 'none'), (2048, 512, 'odm2'), (256, 4096, 'cl'),
          (64, 64, 'gp'), (256, 64, 'gp'), (512, 1024, 'gp'), (64, 128, 'gpodm')]
@@ -48,7 +49,8 @@ def test_blocked_passes_match_oracle(n_x, n_p, form):
     assert np.max(np.abs(got[:, 9] - obs[:3, 10])) < 1e-10
 
 
-@pytest.mark.parametrize('n_x,n_y', [(64, 64), (128, 256), (64, 2048), (2048, 64), (512, 256), (1024, 512), (512, 1024)])
+@pytest.mark.parametrize('n_x,n_y', [(32, 32), (16, 64), (64, 64), (128, 256), (64, 2048), (2048, 64), (512, 256),
+                                     (1024, 512), (512, 1024)])
 def test_blocked_dirac2d_passes_match_oracle(n_x, n_y):
     """4 elements a thread below 2^17 points, 8 from there; one to four columns a CTA."""
     from instances import dirac_instance, dirac_obs
