@@ -2,11 +2,12 @@
 // sizes advanced together, one x-pass launch and one p-pass launch per step
 // over a work list that spans every instance (x-items: blocks of rows, p-items:
 // blocks of columns).  Every sequence (a row in the x-pass, a column in the
-// p-pass) is transformed by the register-resident FFT of wig_rfft.cuh: rf_g(N)
-// lanes of a warp hold its N elements in registers, so the whole p-pass --
+// p-pass) is held in registers from load to store, so the whole p-pass --
 // forward FFT, Moyal factor, inverse FFT, the three Caldeira-Leggett dissipator
 // applications (six more FFTs), observables -- runs on registers, with shared
-// memory only for the coalescing tile and one exchange per FFT.
+// memory only for the coalescing tile and the exchanges of the FFTs.  FP32
+// sequences are transformed by rf_g(N) lanes of a warp (wig_rfft.cuh), FP64 ones
+// by a thread group of 8 or 16 elements a thread (BlockFft, wig_fft.cuh).
 //
 // Storage: W is the real Wigner function, FP32, one float per grid point
 // (instance i a row-major (n_p, n_x) block at its offset); two real rows or
@@ -97,7 +98,12 @@ __host__ __device__ constexpr int bx_rows(int n, int warps) { return 2 * warps *
 // Caldeira-Leggett part (see batch_p_item): an item is BP_PACK column groups.
 constexpr int BP_PACK = 2;
 __host__ __device__ constexpr int bp_cols(int n, int warps) { return BP_PACK * warps * rf_spw(n); }
-__host__ __device__ constexpr int bp_smem(int n, int warps) { return BP_PACK * warps * rf_spw(n) * n; }
+// FP32 form: a float2 tile; mixed: a float tile, then the exchange regions of the FP64 sequences in
+// flight or of all the FP32 ones, whichever is larger
+__host__ __device__ constexpr int bd_exch(int n, int warps);
+__host__ __device__ constexpr int bp_smem(int n, int warps, int prec = WIGB_PREC) {
+  return prec == 1 ? bp_cols(n, warps) * n / 2 + bd_exch(n, warps) : BP_PACK * warps * rf_spw(n) * n;
+}
 
 // p-pass: column of the CT-wide tile owned by group `grp` of warp `warp`.
 // With 8-lane groups two sequences share a half-warp; pairing columns c and
@@ -278,6 +284,77 @@ __device__ __forceinline__ int next_item(unsigned* ticket, int n_items) {
 // it, Re IFFT[f A], only sees Re f there, so the split uses Re fa, Re fb at
 // k = N/2: the same real result, and a contraction.
 
+// ------------------------------------------------------------------ FP64 sequences (WIGB_PREC 1)
+// The mixed form's FP64 transforms run on BlockFft (wig_fft.cuh): 16 elements a
+// thread from 512 points, 8 below (the FP64 dissipator keeps a second set), so a
+// CTA works through an item's packed sequences in rounds of bd_seqs(n).  A lane
+// group of the register FFT holds 32 double2 of a 1024-point sequence, which 168
+// registers spill to local memory (1.1 KB a thread), and its lanes' strided
+// exchange conflicts on the banks.  64-instance mixed batch, B200: x-pass 214 ->
+// 120 us, p-pass 488 -> 374 us,
+// against ~150 us a step of FP64 issue.
+__host__ __device__ constexpr int bd_e(int n) { return n >= 512 ? 16 : 8; }
+__host__ __device__ constexpr int bd_t(int n) { return n / bd_e(n); }
+__host__ __device__ constexpr int bd_seqs(int n, int warps) { return 32 * warps / bd_t(n); }
+__host__ __device__ constexpr int bd_region(int n) { return n + n / 8; }        // BlockFft::REGION
+// region of one FP32 sequence of the mixed p-pass (float2), and the exchange area (float2)
+__host__ __device__ constexpr int bs_region(int n) { return n + (rf_g(n) == 8 ? 8 : 0); }
+__host__ __device__ constexpr int bd_exch(int n, int warps) {
+  const int d = 2 * bd_seqs(n, warps) * bd_region(n), f = warps * rf_spw(n) * bs_region(n);
+  return d > f ? d : f;
+}
+
+// The random words of a sequence's points, as SrStream hands them to lane g = i mod G of the
+// register FFT (two words a point i, the packed pair's): thread t holds i = t + T m, so its words
+// are every rho-th pair of lane t mod G's stream, rho = T / G, from pair t / G on.
+__host__ __device__ constexpr unsigned sr_pow(unsigned n) {        // 1664525^n mod 2^32
+  unsigned a = 1u;
+  for (unsigned i = 0; i < n; ++i) a *= 1664525u;
+  return a;
+}
+__host__ __device__ constexpr unsigned sr_sum(unsigned n) {        // the constant after n LCG steps
+  unsigned c = 0u;
+  for (unsigned i = 0; i < n; ++i) c = c * 1664525u + 1013904223u;
+  return c;
+}
+template <int N> struct PairWords {
+  static constexpr int G = rf_g(N), RHO = bd_t(N) / G;
+  static_assert(bd_t(N) % G == 0, "a thread's points belong to one lane of the register FFT");
+  SrStream rs;
+  __device__ __forceinline__ explicit PairWords(unsigned seed, int t) : rs{seed} {
+    for (int i = 0; i < 2 * (t / G); ++i) rs.next();
+  }
+  __device__ __forceinline__ void skip() { rs.s = rs.s * sr_pow(2 * (RHO - 1)) + sr_sum(2 * (RHO - 1)); }
+};
+
+// Mirror split of a packed spectrum held by the sequence's threads (v[m] = Z(t + T m)), through
+// the exchange region s:  Z'(k) = Z(k) S(k) + conj Z(N - k) D(k),  S = fa + fb, D = fa - fb, the two
+// sequences' factors with the 1/2 folded in.  fab(k) gives fa, fb for k <= N/2; both factors are odd
+// in the phase, so at N - k they are the conjugates: one evaluation per mirror pair.
+template <int N, int E, class Sync, class Fab>
+__device__ __forceinline__ void mirror_split_blk(double2 (&v)[E], double2* s, int t, const Sync& sync, const Fab& fab) {
+  constexpr int T = N / E;
+  sync();   // the region's previous contents have been read
+#pragma unroll
+  for (int m = 0; m < E; ++m) s[t + T * m] = v[m];
+  sync();
+#pragma unroll 2
+  for (int q = t; q <= N / 2; q += T) {
+    const int km = (N - q) & (N - 1);
+    const double2 Z = s[q], P = s[km];
+    double2 fa, fb;
+    fab(q, &fa, &fb);
+    if (q == N / 2) { fa.y = 0.; fb.y = 0.; }       // Nyquist: see nyquist_real
+    const double2 S = cadd(fa, fb), D = csub(fa, fb);
+    // every pair is one thread's own: no other thread reads what it rewrites
+    s[q] = cadd(cmul(Z, S), cmul(cconj(P), D));
+    if (km != q) s[km] = cadd(cmul(P, cconj(S)), cmul(cconj(Z), cconj(D)));
+  }
+  sync();
+#pragma unroll
+  for (int m = 0; m < E; ++m) v[m] = s[t + T * m];
+}
+
 // ------------------------------------------------------------------ x-pass
 // Item: bx_rows(N) consecutive rows; lane group `pair` carries rows ra = row0 +
 // 2 pair and rb = ra + 1 packed into z = W(ra) + i W(rb) (W is real), lane g
@@ -314,7 +391,7 @@ __device__ __forceinline__ void mirror_split(const X& x, int g, const Fab& fab) 
   }
 }
 
-// The precision of an x-pass: its complex type's twiddle and factor tables.
+// The FP32 x-pass's twiddle and factor tables.
 template <class C> struct XPrec;
 template <> struct XPrec<float2> {
   __device__ __forceinline__ static const float2* tw(const BArgs& A, const BInst& I) { return A.tw + I.tw_x; }
@@ -327,18 +404,7 @@ template <> struct XPrec<float2> {
     return make_float2(__ldg(gt + 2 * k), __ldg(gt + 2 * k + 1));
   }
 };
-template <> struct XPrec<double2> {
-  __device__ __forceinline__ static const double2* tw(const BArgs& A, const BInst& I) { return A.tw64 + I.tw_x; }
-  __device__ __forceinline__ static double2 fa(const BArgs& A, const BInst& I, double t, int k) {
-    return turn_factor64(t, 0.5 * __ldg(A.fd + I.fd_x + k));
-  }
-  __device__ __forceinline__ static double2 g(const BArgs& A, const BInst& I, int N, int k) {
-    return __ldg(reinterpret_cast<const double2*>(A.fd + I.fd_x + 2 * N) + k);
-  }
-};
-
-// One x-item in the arithmetic of C (float2: FP32; double2: FP64, rounded to
-// FP32 once on store).  rows: the item's bx_rows(N) rows of W (in global memory
+// One x-item in FP32 (C = float2).  rows: the item's bx_rows(N) rows of W (in global memory
 // or staged in shared memory); after_load() runs once every lane holds its two
 // rows in registers (the caller may then reuse the staging buffer).  The
 // spectrum is staged in natural order in the pair's exchange region (N
@@ -395,16 +461,55 @@ __device__ __forceinline__ void batch_x_item_t(const BArgs& A, int inst, const B
   }
 }
 
-#if WIGB_PREC == 1
-typedef double2 XC;
-#else
-typedef float2 XC;
-#endif
+// The same item in FP64 (WIGB_PREC 1): rounds of bd_seqs(N) row pairs, one thread group of bd_t(N)
+// each; after_load() runs once the last round's rows are in registers.
+template <int N, class After>
+__device__ __forceinline__ void batch_x_item_d(const BArgs& A, int inst, const BInst& I, int row0, const float* rows,
+                                               const After& after_load) {
+  constexpr int E = bd_e(N), T = bd_t(N), NS = bd_seqs(N, WIGB_WARPS), PAIRS = bx_rows(N, WIGB_WARPS) / 2;
+  typedef BlockFft<double2, N, E> F;
+  static_assert(F::REGION == bd_region(N) && PAIRS % NS == 0, "x-item rounds");
+  extern __shared__ float2 smb[];
+  const int seq = threadIdx.x / T, t = threadIdx.x % T;
+  double2* X = reinterpret_cast<double2*>(smb) + seq * F::REGION;
+  const auto sync = SeqSync<T, NS>::make(seq);
+  const double2* tw = A.tw64 + I.tw_x;
+  const double* rl = A.fd + I.fd_x;
+  const double2* gt = reinterpret_cast<const double2*>(rl + 2 * N);
+  const double sc = A.scale[inst];
+#pragma unroll 1
+  for (int p0 = 0; p0 < PAIRS; p0 += NS) {
+    const int pair = p0 + seq, ra = row0 + 2 * pair;
+    WIG_BOUNDS_CHECK("batched x-pass row", ra + 1, I.n_p);
+    const float* Ra = rows + (size_t)(2 * pair) * N + t;
+    double2 v[E];
+#pragma unroll
+    for (int m = 0; m < E; ++m) v[m] = make_double2((double)Ra[T * m] * sc, (double)Ra[N + T * m] * sc);
+    if (p0 + NS == PAIRS) after_load();
+    F::template run<false>(v, X, fresh(tw), t, sync);
+    // kinetic factor of row a, exp(-i dt lambda p / m), in turns; row b's is its product with the pair ratio
+    const double cq = I.dt * I.dp * I.dlambda * (double)shifted(ra, I.n_p) / (I.mass * 6.283185307179586477);
+    mirror_split_blk<N, E>(v, X, t, sync, [&](int k, double2* fa, double2* fb) {
+      const int lj = k < N / 2 ? k : k - N;
+      *fa = turn_factor64(cq * (double)lj, 0.5 * __ldg(rl + k));
+      *fb = cmul(*fa, __ldg(gt + k));
+    });
+    F::template run<true>(v, X, fresh(tw), t, sync);
+    float* Wa = A.W + I.off + (size_t)ra * N + t;
+    PairWords<N> words(sr_word(sr_key(A.step, 0), (long long)I.off + (long long)ra * N + t % rf_g(N)), t);
+#pragma unroll
+    for (int m = 0; m < E; ++m) {
+      Wa[T * m] = store_round(v[m].x, words.rs.next());
+      Wa[N + T * m] = store_round(v[m].y, words.rs.next());
+      words.skip();
+    }
+  }
+}
 
-// The x-pass's exchange regions (elements of float2: an FP64 region of N double2
-// spans 2 N of them) and staging buffer (floats) of one item of size class N.
+// The x-pass's exchange regions (elements of float2: a double2 spans two) and staging buffer (floats) of one
+// item of size class N.
 __host__ __device__ constexpr int bx_exch(int n, int warps, int prec) {
-  return warps * rf_spw(n) * (n + (rf_g(n) == 8 ? 8 : 0)) * (prec == 1 ? 2 : 1);
+  return prec == 1 ? 2 * bd_seqs(n, warps) * bd_region(n) : warps * rf_spw(n) * (n + (rf_g(n) == 8 ? 8 : 0));
 }
 __host__ __device__ constexpr int bx_stage(int n, int warps) { return bx_rows(n, warps) * n; }
 
@@ -476,84 +581,15 @@ __device__ __forceinline__ void batch_p_item(const BArgs& A, int inst, const BIn
   const bool damped = I.damp == 1;
   const int n_it = damped ? 4 : 1;
   float2 w[E];
-#if WIGB_PREC == 1
-  // FP64 Moyal pair: the packed columns are widened, transformed, split with
-  // the spectrum's mirror and multiplied by the FP64 factors in place (the
-  // exchange and the staged spectrum use c1's and c2's slots as doubles, PairX),
-  // transformed back and rounded to FP32 once; the dissipator pairs below run
-  // in FP32 from there.
-  constexpr int it0 = 1;
-  {
-    typedef RegFft<double2, N> F64;
-    const double2* tf64 = A.tw64 + I.tw_p;
-    const double2* ti64 = tf64 + N;
-    const double* rth64 = A.fd + I.fd_p;
-    const double mma64 = __ldg(A.fd + I.fd_x + nx + col0 + c1), mmb64 = __ldg(A.fd + I.fd_x + nx + col0 + c2);
-    double2 z[E];
-#pragma unroll
-    for (int m = 0; m < E; ++m) z[m] = make_double2((double)tile[sl1(g + G * m)].x, (double)tile[sl2(g + G * m)].x);
-    const PairX<TileSlot<CT2>> px{reinterpret_cast<double*>(tile), sl1, sl2};
-    F64::fwdx(z, px, tf64, g);
-    __syncwarp();
-#pragma unroll
-    for (int e = 0; e < E; ++e) px.put(g * Q + e / G + E * (e % G), z[e]);
-    __syncwarp();
-    mirror_split<N, G, double2>(px, g, [&](int k, double2* fa, double2* fb) {
-      const double j = (double)(k < N / 2 ? k : k - N);
-      const double r = 0.5 * __ldg(rth64 + k);
-      *fa = turn_factor64(j * fma(bea, j * j, ala), r * mma64);
-      *fb = turn_factor64(j * fma(beb, j * j, alb), r * mmb64);
-    });
-    __syncwarp();
-#pragma unroll
-    for (int e = 0; e < E; ++e) z[e] = px.get(g * Q + e / G + E * (e % G));
-    F64::invx(z, px, ti64, g);
-    if constexpr (N <= WIGB_DISS64_MAXN) {
-      // the dissipator in FP64 as well (coarse grids): A kept in registers, D through PairX
-      if (damped) {
-        const double* sfp64 = rth64 + N;   // sign(p) f(p)
-        const double* ths64 = sfp64 + N;   // theta / N
-        double2 A[E];
-#pragma unroll
-        for (int m = 0; m < E; ++m) A[m] = z[m];
-#pragma unroll 1
-        for (int it = 0; it < 3; ++it) {
-#pragma unroll
-          for (int m = 0; m < E; ++m) z[m] = cscale(z[m], __ldg(sfp64 + g + G * m));
-          F64::fwdx(z, px, tf64, g);
-#pragma unroll
-          for (int i = 0; i < Q; ++i)
-#pragma unroll
-            for (int b = 0; b < G; ++b) z[i * G + b] = cscale(z[i * G + b], __ldg(ths64 + g * Q + i + E * b));
-          F64::invx(z, px, ti64, g);
-          const double cf = it == 0 ? I.cl_k1 : (it == 1 ? I.cl_k12 : I.cl_c3);
-#pragma unroll
-          for (int m = 0; m < E; ++m) z[m] = make_double2(A[m].x - cf * z[m].y, A[m].y + cf * z[m].x);
-        }
-      }
-    }
-    // rounded to FP32 stochastically (the lane's stream: seeded at its first point of column c1)
-    SrStream rs{sr_word(sr_key(A.step, 1), (long long)I.off + (long long)g * nx + col0 + c1)};
-#pragma unroll
-    for (int m = 0; m < E; ++m) {
-      const float a = store_round(z[m].x, rs.next());
-      w[m] = make_float2(a, store_round(z[m].y, rs.next()));
-    }
-  }
-  const int n_it_run = N <= WIGB_DISS64_MAXN ? 1 : n_it;
-#else
-  constexpr int it0 = 0;
-  const int n_it_run = n_it;
 #pragma unroll
   for (int m = 0; m < E; ++m) {
     const float2 a = tile[sl1(g + G * m)], b = tile[sl2(g + G * m)];
     w[m] = make_float2(a.x, b.x);                  // z = Re W(c1) + i Re W(c2)
   }
-#endif
   // One transform pair per pass through this loop (kept rolled so the kernel
   // holds a single copy of each FFT); the exchange runs in c2's slots.
 #pragma unroll 1
-  for (int it = it0; it < n_it_run; ++it) {
+  for (int it = 0; it < n_it; ++it) {
     __syncwarp();   // the previous transform's exchange reads are done before slots change
     if (it == 1) {
 #pragma unroll
@@ -666,6 +702,195 @@ __device__ __forceinline__ void batch_p_item(const BArgs& A, int inst, const BIn
     const int e = threadIdx.x + r * NT, k = e / CT2, cc = e & (CT2 - 1);
     WIG_BOUNDS_CHECK("batched p-pass store column", col0 + cc, nx);
     Wi[(size_t)k * nx + col0 + cc] = tile[k * CT2 + (cc ^ tile_sw<CT2>(k))].x;
+  }
+  batch_item_done<NT>(A, inst, I, item, acc, I.damp ? 1 : 0, sample);
+}
+
+// The mixed form's item (WIGB_PREC 1), the same columns and packed pairs:
+//   1. rounds of bd_seqs(N) pairs: FP64 Moyal pair (and, up to WIGB_DISS64_MAXN points, the
+//      dissipator) on BlockFft, rounded to FP32 stochastically into the tile;
+//   2. longer damped columns: the three FP32 dissipator pairs on the register FFT, the base read from
+//      the tile;
+//   3. the tile's rows to global memory, with the columns' FP64 moments (a thread's points lie in one
+//      column).
+// Element (k, c) of the float tile at k CT2 + (c ^ bt_sw(k)): consecutive rows of a column on distinct banks.
+template <int CT2> __device__ __forceinline__ int bt_sw(int k) {
+  return CT2 >= 32 ? (k & 31) : ((k / (32 / CT2)) & (CT2 - 1));
+}
+template <int N>
+__device__ __forceinline__ void batch_p_item_d(const BArgs& A, int inst, const BInst& I, int col0, int item,
+                                               int sample) {
+  constexpr int CT = WIGB_WARPS * rf_spw(N), CT2 = BP_PACK * CT, NT = WIGB_NT;
+  constexpr int E = bd_e(N), T = bd_t(N), NS = bd_seqs(N, WIGB_WARPS);
+  constexpr bool DISS64 = N <= WIGB_DISS64_MAXN;
+  typedef BlockFft<double2, N, E> D;
+  static_assert(CT % NS == 0 && NT % CT2 == 0, "p-item rounds");
+  extern __shared__ float2 smb[];
+  float* tile = reinterpret_cast<float*>(smb);
+  double2* X0 = reinterpret_cast<double2*>(tile + CT2 * N);
+  const int nx = I.n_x;
+  float* Wi = A.W + I.off + col0 + threadIdx.x % CT2;
+  constexpr int PER = CT2 * N / NT, ROWS = NT / CT2;   // rows of the tile a load covers
+  const int kr = threadIdx.x / CT2, cr = threadIdx.x % CT2;
+  WIG_BOUNDS_CHECK("batched p-pass tile column", col0 + cr, nx);
+  constexpr int LB = PER < 16 ? PER : 16;
+#pragma unroll 1
+  for (int r0 = 0; r0 < PER; r0 += LB) {
+    float buf[LB];
+#pragma unroll
+    for (int r = 0; r < LB; ++r) buf[r] = Wi[(size_t)(kr + (r0 + r) * ROWS) * nx];
+#pragma unroll
+    for (int r = 0; r < LB; ++r) {
+      const int k = kr + (r0 + r) * ROWS;
+      tile[k * CT2 + (cr ^ bt_sw<CT2>(k))] = buf[r];
+    }
+  }
+  __syncthreads();
+  const bool damped = I.damp == 1;
+  const double* rth = A.fd + I.fd_p;   // exp(-D_theta theta^2 dt), then sign(p) f(p), then theta / N
+  const double2* tw = A.tw64 + I.tw_p;
+  {
+    const int seq = threadIdx.x / T, t = threadIdx.x % T;
+    double2* X = X0 + seq * D::REGION;
+    const auto sync = SeqSync<T, NS>::make(seq);
+    // Moyal factor as in batch_p_item
+    const double h = 0.5 * I.hbar * I.dtheta;
+    const double kk = -I.dt * h / (3.141592653589793238 * I.hbar);
+#pragma unroll 1
+    for (int p0 = 0; p0 < CT; p0 += NS) {
+      const int c1 = p0 + seq, c2 = c1 + CT;
+      double2 z[E];
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        const int k = t + T * m;
+        z[m] = make_double2((double)tile[k * CT2 + (c1 ^ bt_sw<CT2>(k))], (double)tile[k * CT2 + (c2 ^ bt_sw<CT2>(k))]);
+      }
+      D::template run<false>(z, X, fresh(tw), t, sync);
+      const double xa = I.dx * (double)shifted(col0 + c1, nx), xb = I.dx * (double)shifted(col0 + c2, nx);
+      const double ala = kk * ((4. * I.v4 * xa * xa + 2. * I.v2) * xa + I.v1);
+      const double alb = kk * ((4. * I.v4 * xb * xb + 2. * I.v2) * xb + I.v1);
+      const double bea = kk * h * h * (4. * I.v4 * xa), beb = kk * h * h * (4. * I.v4 * xb);
+      const double mma = __ldg(A.fd + I.fd_x + nx + col0 + c1), mmb = __ldg(A.fd + I.fd_x + nx + col0 + c2);
+      mirror_split_blk<N, E>(z, X, t, sync, [&](int k, double2* fa, double2* fb) {
+        const double j = (double)(k < N / 2 ? k : k - N);
+        const double r = 0.5 * __ldg(rth + k);
+        *fa = turn_factor64(j * fma(bea, j * j, ala), r * mma);
+        *fb = turn_factor64(j * fma(beb, j * j, alb), r * mmb);
+      });
+      D::template run<true>(z, X, fresh(tw), t, sync);
+      if constexpr (DISS64) {
+        if (damped) {
+          double2 B[E];
+#pragma unroll
+          for (int m = 0; m < E; ++m) B[m] = z[m];
+#pragma unroll 1
+          for (int it = 0; it < 3; ++it) {
+            const double* sf = fresh(rth + N + t);
+#pragma unroll
+            for (int m = 0; m < E; ++m) z[m] = cscale(z[m], __ldg(sf + T * m));
+            D::template run<false>(z, X, fresh(tw), t, sync);
+            const double* th = fresh(rth + 2 * N + t);
+#pragma unroll
+            for (int m = 0; m < E; ++m) z[m] = cscale(z[m], __ldg(th + T * m));
+            D::template run<true>(z, X, fresh(tw), t, sync);
+            const double cf = it == 0 ? I.cl_k1 : (it == 1 ? I.cl_k12 : I.cl_c3);
+#pragma unroll
+            for (int m = 0; m < E; ++m) z[m] = make_double2(B[m].x - cf * z[m].y, B[m].y + cf * z[m].x);
+          }
+        }
+      }
+      // rounded to FP32 stochastically (the words of the register FFT's lanes, seeded at column c1)
+      PairWords<N> words(sr_word(sr_key(A.step, 1), (long long)I.off + (long long)(t % rf_g(N)) * nx + col0 + c1), t);
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        const int k = t + T * m;
+        tile[k * CT2 + (c1 ^ bt_sw<CT2>(k))] = store_round(z[m].x, words.rs.next());
+        tile[k * CT2 + (c2 ^ bt_sw<CT2>(k))] = store_round(z[m].y, words.rs.next());
+        words.skip();
+      }
+    }
+  }
+  __syncthreads();
+  if constexpr (!DISS64) {
+    if (damped) {
+      typedef RegFft<float2, N> F;
+      constexpr int FE = F::E, G = F::G, Q = F::Q;
+      const float2* tf = A.tw + I.tw_p;
+      const float2* ti = tf + N;
+      const float* sfp = A.ft + I.ft_p + N;   // sign(p) f(p)
+      const float* ths = sfp + N;             // theta / N
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / G, g = lane % G;
+      const int c1 = rf_col<N>(warp, grp), c2 = c1 + CT;
+      float2* Xf = reinterpret_cast<float2*>(X0);
+      const PlainSlot sl{(warp * rf_spw(N) + grp) * bs_region(N)};
+      float2 w[FE];
+#pragma unroll
+      for (int m = 0; m < FE; ++m) {
+        const int k = g + G * m;
+        w[m] = make_float2(tile[k * CT2 + (c1 ^ bt_sw<CT2>(k))], tile[k * CT2 + (c2 ^ bt_sw<CT2>(k))]);
+      }
+#pragma unroll 1
+      for (int it = 1; it < 4; ++it) {
+        __syncwarp();   // the previous transform's exchange reads are done before slots change
+        const float* sf = fresh(sfp + g);
+#pragma unroll
+        for (int m = 0; m < FE; ++m) w[m] = cscale(w[m], __ldg(sf + G * m));
+        F::fwd(w, Xf, sl, fresh(tf), g);
+        const float* th = fresh(ths);
+#pragma unroll
+        for (int i = 0; i < Q; ++i)
+#pragma unroll
+          for (int b = 0; b < G; ++b) w[i * G + b] = cscale(w[i * G + b], __ldg(th + g * Q + i + FE * b));
+        F::inv(w, Xf, sl, fresh(ti), g);
+        const float cf = (float)(it == 1 ? I.cl_k1 : (it == 2 ? I.cl_k12 : I.cl_c3));
+#pragma unroll
+        for (int m = 0; m < FE; ++m) {
+          const int k = g + G * m;
+          const float2 a = make_float2(tile[k * CT2 + (c1 ^ bt_sw<CT2>(k))], tile[k * CT2 + (c2 ^ bt_sw<CT2>(k))]);
+          w[m] = make_float2(a.x - cf * w[m].y, a.y + cf * w[m].x);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < FE; ++m) {
+        const int k = g + G * m;
+        tile[k * CT2 + (c1 ^ bt_sw<CT2>(k))] = w[m].x;
+        tile[k * CT2 + (c2 ^ bt_sw<CT2>(k))] = w[m].y;
+      }
+      __syncthreads();
+    }
+  }
+  // store, with the column's moments sum W, sum W p_j, sum W p_j^2 and the negative part (FP64)
+  double s0 = 0., s1 = 0., s2 = 0., sn = 0.;
+#pragma unroll 8
+  for (int r = 0; r < PER; ++r) {
+    const int k = kr + r * ROWS;
+    const float v = tile[k * CT2 + (cr ^ bt_sw<CT2>(k))];
+    Wi[(size_t)k * nx] = v;
+    const double wr = (double)v, pj = (double)shifted(k, N), wp = wr * pj;
+    s0 += wr;
+    s1 += wp;
+    s2 = fma(wp, pj, s2);
+    sn += fmin(wr, 0.);
+  }
+  double acc[NACC];
+#pragma unroll
+  for (int v = 0; v < NACC; ++v) acc[v] = 0.;
+  {
+    const double x = I.dx * (double)shifted(col0 + cr, nx);
+    const double dV = (4. * I.v4 * x * x + 2. * I.v2) * x + I.v1;
+    const double V = ((I.v4 * x * x + I.v2) * x + I.v1) * x + I.v0;
+    const double M1 = s1 * I.dp, M2 = s2 * (I.dp * I.dp);
+    acc[0] = s0;
+    acc[2] = s0 * x;
+    acc[3] = s0 * x * x;
+    acc[4] = M1;
+    acc[5] = M2;
+    acc[6] = M1 * x;
+    acc[7] = s0 * dV;
+    acc[8] = M1 * dV;
+    acc[9] = s0 * x * dV;
+    acc[10] = M2 / (2. * I.mass) + s0 * V;
+    acc[11] = sn;
   }
   batch_item_done<NT>(A, inst, I, item, acc, I.damp ? 1 : 0, sample);
 }

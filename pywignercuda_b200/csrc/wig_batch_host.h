@@ -160,13 +160,16 @@ void batch_instance_setup(const D& d, wig::BInst& b, std::vector<float>* ft, std
   for (double v : th) fd->push_back(v);
 }
 
-// Twiddle tables of every size class (float and double, same offsets).
+// Twiddle tables of every size class at common offsets, 2 n entries each: the register FFT's
+// in float; in double the stage twiddles of BlockFft<double2, n, bd_e(n)>, filled up with zeros.
 inline void batch_twiddles(const std::vector<int>& classes, std::vector<float2>* tw, std::vector<double2>* tw64,
                            std::map<int, int>* off) {
   for (int n : classes) {
     (*off)[n] = (int)tw->size();
     rf_twiddles(n, tw);
-    rf_twiddles64(n, tw64);
+    const std::vector<double2> b = block_twiddles(n, wig::bd_e(n));
+    tw64->insert(tw64->end(), b.begin(), b.end());
+    tw64->resize(tw->size(), double2{0., 0.});
   }
 }
 

@@ -1740,7 +1740,7 @@ int batch_smem_x(const std::vector<int>& classes, int warps, int prec, int xstag
   }
   return ex * (int)sizeof(float2) + (xstage ? st * (int)sizeof(float) : 0);
 }
-int batch_smem_p(int n, int warps) { return wig::bp_smem(n, warps) * (int)sizeof(float2); }
+int batch_smem_p(int n, int warps, int prec) { return wig::bp_smem(n, warps, prec) * (int)sizeof(float2); }
 
 }  // namespace
 
@@ -1777,15 +1777,11 @@ struct wigb_handle {
 static std::string wigb_source(const std::vector<int>& classes, int warps, int precision, int xstage) {
   // Register caps, as the warps per SM each pass must allow (8-warp tiles run one
   // CTA per SM, 255 registers).  Measured on the 64-instance batch (B200, CUDA events):
-  //   mixed x-pass 12 (168 registers, the same 72 B of spill as at 255): 253 -> 220 us
-  //     against 8 warps per SM;
-  //   mixed p-pass 12 (168 registers, ~1 KB of spill to L1-cached local memory; the
-  //     1024-point FP64 Moyal pair holds 32 double2 per lane): 535 -> 487 us against 8;
-  //   FP32 x-pass 16 (128 registers, no spill): 173 -> 164 us against 12;
-  //   FP32 p-pass 12 (168 registers): 16 measured slower (347 -> 379 us).
+  //   x-pass 16 (128 registers): mixed 120 us against 127 at 12, FP32 164 against 173;
+  //   p-pass 12 (168 registers): mixed 374 us, FP32 346; 16 spills more and is slower
+  //   (FP32 347 -> 379 us when it was measured), 8 leaves too few warps to cover latency.
   char head[512];
-  const bool mixed = precision == WIGB_PREC_MIXED;
-  const int xwps = mixed ? 12 : 16, pwps = 12;
+  const int xwps = 16, pwps = 12;
   int xminb = warps == 8 ? 1 : std::max(1, xwps / warps), pminb = warps == 8 ? 1 : std::max(1, pwps / warps);
   // tuning override (read per compile): WIG_BATCH_WPS=x,p sets the x- and p-pass register
   // caps by the warps per SM they must allow (e.g. 12,8); 0 keeps the default
@@ -1847,7 +1843,7 @@ static int wigb_compile(wigb_handle* h, int warps, BVariant* v) {
   const int xstage = batch_xstage(h->precision);
   const std::string src = wigb_source(h->classes, warps, h->precision, xstage);
   int smx = batch_smem_x(h->classes, warps, h->precision, xstage), smp = 0;
-  for (int n : h->classes) smp = std::max(smp, batch_smem_p(n, warps));
+  for (int n : h->classes) smp = std::max(smp, batch_smem_p(n, warps, h->precision));
   if (smx > 227 * 1024 || smp > 227 * 1024)
     return fail(WIG_ERR_ARG, "batched tile of %d warps needs %d / %d bytes of shared memory", warps, smx, smp);
   CUmodule mod;

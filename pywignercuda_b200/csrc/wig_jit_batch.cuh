@@ -30,8 +30,17 @@
 #endif
 template <int N> __device__ WIGB_CASE_INLINE void wigb_p_case(const wig::BArgs& A, int inst, const wig::BInst& I, int col0,
                                                           int item, int sample) {
+#if WIGB_PREC == 1
+  wig::batch_p_item_d<N>(A, inst, I, col0, item, sample);
+#else
   wig::batch_p_item<N>(A, inst, I, col0, item, sample);
+#endif
 }
+#if WIGB_PREC == 1
+#define WIGB_X_ITEM(N) wig::batch_x_item_d<N>
+#else
+#define WIGB_X_ITEM(N) wig::batch_x_item_t<float2, N>
+#endif
 #define WIGB_P_CASE(N) case N: wigb_p_case<N>(A, it.x, sI, it.y, item, sample); break;
 #define WIGB_R_CASE(N) case N: wig::batch_reduce_item<N>(A, it.x, sI, it.y, item, mode, sample); break;
 #define WIGB_S_CASE(N) case N: wig::batch_scale_item<N>(A, it.x, sI, it.y); break;
@@ -118,7 +127,7 @@ __device__ __forceinline__ void wigb_stage_wait(unsigned long long*, unsigned, u
 #endif
 
 #if WIGB_XSTAGE
-#define WIGB_X_CASE(N) case N: wig::batch_x_item_t<wig::XC, N>(A, sIn[buf], sI[buf], sRow[buf], stage, after); break;
+#define WIGB_X_CASE(N) case N: WIGB_X_ITEM(N)(A, sIn[buf], sI[buf], sRow[buf], stage, after); break;
 
 // Shared memory: the exchange regions (wigb_xexch_max() float2), then the
 // staging buffer (wigb_xstage_max() floats).
@@ -179,7 +188,7 @@ wigb_xpass(wig::BArgs A, int n_items) {
 #else
 #define WIGB_X_CASE(N)                                                                              \
   case N:                                                                                           \
-    wig::batch_x_item_t<wig::XC, N>(A, it.x, sI, it.y, A.W + sI.off + (size_t)it.y * N, [] {}); \
+    WIGB_X_ITEM(N)(A, it.x, sI, it.y, A.W + sI.off + (size_t)it.y * N, [] {}); \
     break;
 
 // Shared memory: the exchange regions (wigb_xexch_max() float2).

@@ -222,3 +222,16 @@ def test_blocked_dirac3d_passes_match_oracle(staged, dims, x, y, z, cap, sanitiz
     assert rel_l2(got, ref) < 1e-12
     scale = np.maximum(np.abs(ref_obs).max(axis=0), 1e-3)
     assert np.all(np.abs(obs - ref_obs) / scale < 1e-10), (obs - ref_obs) / scale
+
+
+@pytest.mark.parametrize('warps,sanitize', [(2, 'address'), (4, 'thread')])
+def test_mixed_batch_long_axes_match_oracle(staged, monkeypatch, warps, sanitize):  # noqa: F811
+    """The mixed batched form's sequences of 16 elements a thread (512 points): a 64 x 512 and a
+    512 x 64 instance beside an undamped 64 x 64 one, by test_emu_cpu's test with these shapes."""
+    monkeypatch.setattr(E, 'BSIZES', ())
+    monkeypatch.setattr(E, 'BSHAPES', ((64, 512, 10., 8.), (512, 64, 8., 10.), (64, 64, 10., 10.)))
+    monkeypatch.setattr(E, 'BEXTRA', {})
+    build = E.build
+    monkeypatch.setattr(E, 'build', lambda dst, source, m: build(dst, source, dict(m, **{'WIGB_CASES(F)': 'F(64) F(512)'}),
+                                                                 sanitize))
+    E.test_batch_device_code_matches_oracle(staged, warps, 3, 1, 0)
