@@ -291,7 +291,7 @@ __device__ __forceinline__ int next_item(unsigned* ticket, int n_items) {
 // group of the register FFT holds 32 double2 of a 1024-point sequence, which 168
 // registers spill to local memory (1.1 KB a thread), and its lanes' strided
 // exchange conflicts on the banks.  64-instance mixed batch, B200: x-pass 214 ->
-// 120 us, p-pass 488 -> 374 us,
+// 120 us, p-pass 488 -> 374 us (354 with WIG_PACKED_F32 for its FP32 dissipator),
 // against ~150 us a step of FP64 issue.
 __host__ __device__ constexpr int bd_e(int n) { return n >= 512 ? 16 : 8; }
 __host__ __device__ constexpr int bd_t(int n) { return n / bd_e(n); }

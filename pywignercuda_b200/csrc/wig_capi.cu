@@ -1777,8 +1777,8 @@ struct wigb_handle {
 static std::string wigb_source(const std::vector<int>& classes, int warps, int precision, int xstage) {
   // Register caps, as the warps per SM each pass must allow (8-warp tiles run one
   // CTA per SM, 255 registers).  Measured on the 64-instance batch (B200, CUDA events):
-  //   x-pass 16 (128 registers): mixed 120 us against 127 at 12, FP32 164 against 173;
-  //   p-pass 12 (168 registers): mixed 374 us, FP32 346; 16 spills more and is slower
+  //   x-pass 16 (128 registers): mixed 120 us against 127 at 12, FP32 145 against 163;
+  //   p-pass 12 (168 registers): mixed 354 us, FP32 334; 16 spills more and is slower
   //   (FP32 347 -> 379 us when it was measured), 8 leaves too few warps to cover latency.
   char head[512];
   const int xwps = 16, pwps = 12;

@@ -58,14 +58,39 @@ template <bool INV, class C> __device__ __forceinline__ C mul_mi(C a) {
   return r;
 }
 
+// Complex sum and difference; with WIG_PACKED_F32 one packed instruction for float2
+// (both components rounded as by the two scalar ones: the batched FP32 transforms are
+// bound by issue slots; 64-instance batch, step 522 -> 499 us, bit for bit the same).
+// Used where neither operand is a free swap or sign change of another value.
+template <class C> __device__ __forceinline__ C padd(C a, C b) { return cadd(a, b); }
+template <class C> __device__ __forceinline__ C psub(C a, C b) { return csub(a, b); }
+#if defined(__CUDA_ARCH__) && defined(WIG_PACKED_F32)
+template <> __device__ __forceinline__ float2 padd<float2>(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 c, a, b;\n"
+      " mov.b64 {%0, %1}, c;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+template <> __device__ __forceinline__ float2 psub<float2>(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n sub.rn.f32x2 c, a, b;\n"
+      " mov.b64 {%0, %1}, c;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+#endif
+
 // ---------------------------------------------------------------- R-point DFTs
 template <bool INV, class C> __device__ __forceinline__ void dft2(C& a, C& b) {
-  C t = a; a = cadd(t, b); b = csub(t, b);
+  C t = a; a = padd(t, b); b = psub(t, b);
 }
 
 template <bool INV, class C> __device__ __forceinline__ void dft4(C& v0, C& v1, C& v2, C& v3) {
-  C a0 = cadd(v0, v2), a1 = csub(v0, v2), a2 = cadd(v1, v3), a3 = mul_mi<INV>(csub(v1, v3));
-  v0 = cadd(a0, a2); v2 = csub(a0, a2); v1 = cadd(a1, a3); v3 = csub(a1, a3);
+  C a0 = padd(v0, v2), a1 = psub(v0, v2), a2 = padd(v1, v3), a3 = mul_mi<INV>(psub(v1, v3));
+  v0 = padd(a0, a2); v2 = psub(a0, a2); v1 = cadd(a1, a3); v3 = csub(a1, a3);
 }
 
 template <bool INV, class C> __device__ __forceinline__ void dft8(C* v) {
@@ -158,7 +183,7 @@ __device__ __forceinline__ C twc32(C v, int j) {
 template <bool INV, class C> __device__ __forceinline__ void dft8c(C* v) {
   C a[4], b[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) { a[k] = cadd(v[k], v[k + 4]); b[k] = csub(v[k], v[k + 4]); }
+  for (int k = 0; k < 4; ++k) { a[k] = padd(v[k], v[k + 4]); b[k] = psub(v[k], v[k + 4]); }
   b[1] = twc32<INV>(b[1], 4);
   b[2] = mul_mi<INV>(b[2]);
   b[3] = twc32<INV>(b[3], 12);
@@ -222,8 +247,8 @@ template <bool INV, class C> __device__ __forceinline__ void dft32(C* v) {
 #pragma unroll
   for (int k = 0; k < 16; ++k) {
     const C t = twc32<INV>(o[k], k);
-    v[k] = cadd(e[k], t);
-    v[k + 16] = csub(e[k], t);
+    v[k] = padd(e[k], t);
+    v[k + 16] = psub(e[k], t);
   }
 }
 

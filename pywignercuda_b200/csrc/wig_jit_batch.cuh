@@ -8,6 +8,7 @@
 // from a ticket counter, the one-off reduce / scale kernels take items
 // b, b + gridDim.x, ...
 #pragma once
+#define WIG_PACKED_F32 1
 #include "wig_batch.cuh"
 
 #ifndef WIGB_XMINB
