@@ -359,7 +359,7 @@ struct wig_handle {
   int64_t psq_n = 0;
   cudaStream_t last_stream = nullptr;
   int odm = 0, smem_odm_x = 0, smem_odm_p = 0;
-  double2* odm_T = nullptr;                    // 5 planes of ODM intermediates
+  double2* odm_T = nullptr;                    // ODM intermediates: 5 planes, 2 on the blocked passes
   double odm_coef[2] = {0., 0.}, odm_sign[2] = {1., -1.};
   // launch shapes of the x- and p-pass; blocked ones (BlockFft) start with programmatic serialisation, and
   // their x-pass and first-half p-pass have one CTA more (the sample)
@@ -778,7 +778,7 @@ extern "C" int wig_create(const wig_desc* d, wig_handle** out) {
                                            : shifted_range(dLambda * NX / 2., NX);
   double* lam_d = nullptr;
   if (!rc) rc = B.alloc(&lam_d, NX, lt.data());
-  if (!rc && h->odm) rc = B.alloc(&h->odm_T, (h->odm2 ? 3 : 5) * (size_t)NX * NP);
+  if (!rc && h->odm) rc = B.alloc(&h->odm_T, (h->odm2 ? 2 : 5) * (size_t)NX * NP);
   double2 *bx_d = nullptr, *bp_d = nullptr, *box_d = nullptr, *bop_d = nullptr, *c2_d = nullptr, *ct_d = nullptr;
   const auto upload_tw = [&](double2** dst, int n, int e) {
     const std::vector<double2> tw = block_twiddles(n, e);
@@ -943,7 +943,7 @@ static int wig_odm_term(wig_handle* h, WigRunState* S, double coef, double sign,
     a.btw_p = h->btw_op;
     void* xargs[] = {&a, &S->W, &h->odm_T, &sign};
     if (int rc = launch_after(h->f_ox, h->gox, h->gox_nt, h->smem_odm_x, st, xargs)) return rc;
-    void* pargs[] = {&a, &S->W, &h->odm_T, &coef};
+    void* pargs[] = {&a, &S->W, &h->odm_T, &coef, &sign};
     if (int rc = launch_after(h->f_op, h->gop, h->gop_nt, h->smem_odm_p, st, pargs)) return rc;
     S->a.n_partials = h->gop;
     return WIG_OK;

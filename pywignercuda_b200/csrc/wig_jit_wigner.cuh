@@ -212,8 +212,8 @@ wig_odm_xpass(wig::WigArgs a, const double2* W, double2* R, double sign) {
 }
 
 extern "C" __global__ void __launch_bounds__(WIG_OPC * (WIG_NP / WIG_OE), WIG_OPMB)
-wig_odm_ppass(wig::WigArgs a, double2* W, const double2* R, double coef) {
-  wig::odm_ppass_blk_body<WIG_NX, WIG_NP, WIG_OPC, WIG_OE>(a, W, R, coef);
+wig_odm_ppass(wig::WigArgs a, double2* W, const double2* R, double coef, double sign) {
+  wig::odm_ppass_blk_body<WIG_NX, WIG_NP, WIG_OPC, WIG_OE>(a, W, R, coef, sign);
 }
 #elif WIG_ODM == 1
 extern "C" __global__ void __launch_bounds__(WIG_XNT)

@@ -1060,9 +1060,12 @@ __device__ __forceinline__ void ppass_blk_body(const WigArgs& a, const Phys& ph,
 // a + b = 2 X, a - b = hbar Theta: with T_k = IFFT_x[FFT_x(W) G_k] / n_x the sum is
 //   cos(2X)/2 (T0 - T3) + i s sin(2X)/2 (T1 - T2) + T4           a function of x: R0
 //   + cos(hbar Theta) (T0 + T3)/2 + sin(hbar Theta) i s (T1 + T2)/2     R1, R2
-// so the x-pass leaves three planes instead of five and the p-pass transforms
-// three columns instead of five.  g(p + hbar lambda / 2) is evaluated once per
-// point (g(p - hbar lambda / 2) is its value at -lambda) instead of twice per term.
+// G1 + G2 = g g (sgn(p-) + sgn(p+)) is sgn(p) times G0 + G3 = g g (1 + sgn(p+) sgn(p-)),
+// p+- = p +- hbar lambda / 2, at every point (both are 0 where p+ and p- have opposite signs), so
+// R2 = i s sgn(p) R1: the x-pass does four inverse transforms instead of five and leaves two
+// planes instead of five, the p-pass transforms three columns instead of five.
+// g(p + hbar lambda / 2) is evaluated once per point (g(p - hbar lambda / 2) is its value at
+// -lambda) instead of twice per term.
 // Shared memory of the x-pass: ROWS regions, then ROWS (NX + 1) doubles (g).
 template <class Phys, int NX, int NP, int ROWS, int E>
 __device__ __forceinline__ void odm_xpass_blk_body(const WigArgs& a, const Phys& ph, const double2* __restrict__ W,
@@ -1089,9 +1092,9 @@ __device__ __forceinline__ void odm_xpass_blk_body(const WigArgs& a, const Phys&
   F::template run<false>(f, X, a.btw_x, t, sync);
   const double inv_n = 1.0 / (double)NX;
   sync();   // g is complete
-  // term 0: G1 - G2, 1: G0 - G3, 2: G4, 3: G0 + G3, 4: G1 + G2
+  // term 0: G1 - G2, 1: G0 - G3, 2: G4, 3: G0 + G3
 #pragma unroll 1
-  for (int term = 0; term < 5; ++term) {
+  for (int term = 0; term < 4; ++term) {
 #pragma unroll
     for (int m = 0; m < E; ++m) {
       const int k = t + T * m;
@@ -1101,8 +1104,7 @@ __device__ __forceinline__ void odm_xpass_blk_body(const WigArgs& a, const Phys&
       if (term == 0) q = gg * (sn - sp);
       else if (term == 1) q = gg * (1. - sp * sn);
       else if (term == 2) q = -0.5 * gp * gp - 0.5 * gm * gm;
-      else if (term == 3) q = gg * (1. + sp * sn);
-      else q = gg * (sn + sp);
+      else q = gg * (1. + sp * sn);
       v[m] = cscale(f[m], q * inv_n);
     }
     F::template run<true>(v, X, fresh(a.btw_x), t, sync);
@@ -1117,21 +1119,18 @@ __device__ __forceinline__ void odm_xpass_blk_body(const WigArgs& a, const Phys&
         r0[m] = make_double2(r0[m].x + 0.5 * cs.x * v[m].x, r0[m].y + 0.5 * cs.x * v[m].y);
       } else if (term == 2) {
         R[base + t + T * m] = cadd(r0[m], v[m]);
-      } else if (term == 3) {
-        R[plane + base + t + T * m] = cscale(v[m], 0.5);
       } else {
-        const double h = 0.5 * sign;
-        R[2 * plane + base + t + T * m] = make_double2(-h * v[m].y, h * v[m].x);
+        R[plane + base + t + T * m] = cscale(v[m], 0.5);
       }
     }
   }
 }
 
-// W <- W + coef IFFT_p[FFT_p(R0) + cos(hbar Theta) FFT_p(R1) + sin(hbar Theta) FFT_p(R2)], then the
-// observable sums with their imaginary parts.  Shared memory: C exchange regions.
+// W <- W + coef IFFT_p[FFT_p(R0) + cos(hbar Theta) FFT_p(R1) + sin(hbar Theta) FFT_p(R2)], R2 = i sign
+// sgn(p) R1, then the observable sums with their imaginary parts.  Shared memory: C exchange regions.
 template <int NX, int NP, int C, int E>
 __device__ __forceinline__ void odm_ppass_blk_body(const WigArgs& a, double2* __restrict__ W,
-                                                   const double2* __restrict__ R, double coef) {
+                                                   const double2* __restrict__ R, double coef, double sign) {
   typedef BlockFft<double2, NP, E> F;
   constexpr int T = F::T, NT = C * T, RS = blk_stride(F::REGION, C);
   static_assert(NT % 32 == 0 && C <= 32, "ODM p-pass columns per CTA");
@@ -1147,9 +1146,17 @@ __device__ __forceinline__ void odm_ppass_blk_body(const WigArgs& a, double2* __
   double2 acc[E], v[E];
 #pragma unroll 1
   for (int q = 0; q < 3; ++q) {
-    const double2* Rc = R + q * plane + col;
+    const double2* Rc = R + (q == 0 ? 0 : plane) + col;
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = Rc[(size_t)(th + T * m) * NX];
+    if (q == 2) {
+      const double* pt = fresh(a.p_tab + th);
+#pragma unroll
+      for (int m = 0; m < E; ++m) {
+        const double h = sign * sgn(__ldg(pt + T * m));
+        v[m] = make_double2(-h * v[m].y, h * v[m].x);
+      }
+    }
     F::template run<false>(v, X, fresh(a.btw_p), th, sync);
     const double2* ct = fresh(a.csth + th);
 #pragma unroll

@@ -59,7 +59,7 @@ int main(int argc, char** argv) {
   emu_launch(n_cta_r, WIG_RNT, [&] { wig_reduce(a, Wp); });
   a.n_partials = n_cta_r;
 #if WIG_ODM == 2
-  std::vector<double2> c2x(NX), cth(NP), R(3 * npts);
+  std::vector<double2> c2x(NX), cth(NP), R(2 * npts);
   for (int k = 0; k < NX; ++k) c2x[k] = make_double2(cos(2. * xt[k]), sin(2. * xt[k]));
   for (int k = 0; k < NP; ++k) cth[k] = make_double2(cos(hBar * ths[k] * NP), sin(hBar * ths[k] * NP));
   a.cs2x = c2x.data();
@@ -105,7 +105,7 @@ int main(int argc, char** argv) {
     for (int j = 0; j < odm; ++j) {
       const double coef = dt * 2 * gamma * weight[j] * (1.0 / (double)NP);
       emu_launch(gox, oxnt, [&] { wig_odm_xpass(ao, Wp, R.data(), sign[j]); }, smox);
-      emu_launch(gop, opnt, [&] { wig_odm_ppass(ao, Wp, R.data(), coef); }, smop);
+      emu_launch(gop, opnt, [&] { wig_odm_ppass(ao, Wp, R.data(), coef, sign[j]); }, smop);
     }
     a.n_partials = gop;
 #endif
