@@ -1237,12 +1237,22 @@ __device__ __forceinline__ void gp_phase_blk_body(const WigArgs& a, const double
   double2 s = make_double2(1., 0.);
   if (scale_mode != 0) s = consume_scale<NT>(a, scale_mode);
   double acc[1] = {0.};
-  for (int x = threadIdx.x; x < NX; x += NT) {
-    double2 c = make_double2(0., 0.);
-    for (int q = 0; q < n_chunks; ++q) c = cadd(c, chunks[(size_t)q * NX + x]);
-    const double px = a.dP * (s.x * c.x - s.y * c.y);
-    Ps[x] = px;
-    acc[0] += px * px;
+  constexpr int PX = NT < NX ? NX / NT : 1;   // the loads of a chunk row are in flight together
+  double2 cs[PX];
+#pragma unroll
+  for (int i = 0; i < PX; ++i) cs[i] = make_double2(0., 0.);
+  if (threadIdx.x < NX) {
+#pragma unroll 2
+    for (int q = 0; q < n_chunks; ++q) {
+#pragma unroll
+      for (int i = 0; i < PX; ++i) cs[i] = cadd(cs[i], chunks[(size_t)q * NX + threadIdx.x + NT * i]);
+    }
+#pragma unroll
+    for (int i = 0; i < PX; ++i) {
+      const double px = a.dP * (s.x * cs[i].x - s.y * cs[i].y);
+      Ps[threadIdx.x + NT * i] = px;
+      acc[0] += px * px;
+    }
   }
   __syncthreads();
   if (psq != nullptr && blockIdx.x == 0) {
