@@ -575,11 +575,12 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
       return fail(WIG_ERR_ARG, "WIG_BTILING: tiles of %d / %d threads", nt, ntp);
     P->gx = NP / P->bxr + 1;
     P->gx_nt = nt;
-    P->gx_smem = P->bxr * pad(NX, P->bxe) * (int)sizeof(double2);
+    P->gx_smem = P->bxr * (pad(NX, P->bxe) + wig::blk_pre_slots(NX, P->bxe)) * (int)sizeof(double2);
     P->gp_n = NX / P->bpc;
     P->gp_nt = ntp;
-    P->gph_smem = P->bpc * wig::blk_stride(pad(NP, P->bpe), P->bpc) * (int)sizeof(double2);
-    P->gp_smem = P->gph_smem;
+    P->gp_smem = P->bpc * (wig::blk_stride(pad(NP, P->bpe), P->bpc) + wig::blk_pre_slots(NP, P->bpe)) *
+                 (int)sizeof(double2);
+    P->gph_smem = P->gp_smem;
     if (!P->bx) { P->gx = P->n_cta_x; P->gx_nt = P->xnt; P->gx_smem = P->smem_x; }
     if (!P->bp) { P->gp_n = P->n_cta_p; P->gp_nt = P->pnt; P->gp_smem = P->smem_p; P->gph_smem = P->smem_ph; }
     P->odm2 = P->odm && P->bx && P->bp ? 1 : 0;

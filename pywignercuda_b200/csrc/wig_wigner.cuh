@@ -798,9 +798,34 @@ __device__ __forceinline__ void apply_odd_factor(double2 (&v)[E], double2* s, in
   }
 }
 
+// With at most 8 elements a thread (grids below 2^19 points, where a CTA of the next pass is resident
+// beside the current one) the factors, which do not depend on W, are evaluated before the wait for the
+// preceding pass, into their own N / 2 + 1 slots a sequence (blk_pre_slots).  Steps, us, before /
+// after: 256^2 9.4 / 7.8, 128 x 64 damped 12.8 / 10.1, 512^2 16.4 / 13.2, 512^2 damped 26.0 / 21.8,
+// 4096 x 64 damped 31.9 / 26.7, Gross-Pitaevskii 512^2 (phases and the sines of the mean field) 61.4 /
+// 56.0.  With 16 elements the slots take the shared memory of resident CTAs of the same pass: 1024^2
+// damped 64.6 / 69.4, 2048 x 256 damped 39.6 / 64.4, so those evaluate them in place.
+__host__ __device__ constexpr bool blk_pre(int e) { return e <= 8; }
+__host__ __device__ constexpr int blk_pre_slots(int n, int e) { return blk_pre(e) ? n / 2 + 1 : 0; }
+template <int N, int E, class Factor>
+__device__ __forceinline__ void odd_factor_pre(double2* pf, int t, const Factor& factor) {
+#pragma unroll 1
+  for (int k = t; k <= N / 2; k += N / E) pf[k] = factor(k);
+}
+// ... and applied after at least one stage boundary of the sequence
+template <int N, int E>
+__device__ __forceinline__ void apply_odd_factor_pre(double2 (&v)[E], const double2* pf, int t) {
+#pragma unroll
+  for (int m = 0; m < E; ++m) {
+    const int k = t + (N / E) * m;
+    v[m] = cmul(v[m], k <= N / 2 ? pf[k] : cconj(pf[N - k]));
+  }
+}
+
 // x-pass: ROWS rows per CTA, NX / E threads per row; the last CTA of the grid
 // (block NP / ROWS) only records the previous pass's sample, so that no row's
-// CTA waits for that reduction.  Shared memory: ROWS exchange regions.
+// CTA waits for that reduction.  Shared memory: ROWS exchange regions, then ROWS
+// times blk_pre_slots(NX, E).
 template <class Phys, int NX, int NP, int ROWS, int E, bool KIN_STRING>
 __device__ __forceinline__ void xpass_blk_body(const WigArgs& a, const Phys& ph, double2* __restrict__ W,
                                                int scale_mode, double* obs_row) {
@@ -809,13 +834,30 @@ __device__ __forceinline__ void xpass_blk_body(const WigArgs& a, const Phys& ph,
   static_assert(NT % 32 == 0 && (T % 32 == 0 || 32 % T == 0), "x-pass rows per CTA");
   extern __shared__ double2 sm[];
   __shared__ double red[NT / 32][NACC];
+  const int seq = threadIdx.x / T, t = threadIdx.x % T, row = blockIdx.x * ROWS + seq;
+  const auto factor = [&](int k) {
+    const int ii = (row + NP / 2) % NP, jj = (k + NX / 2) % NX;
+    const double p = a.dp * (ii - 0.5 * NP);
+    const double lambda = a.dlambda * (jj - 0.5 * NX);
+    double phase;
+    if (KIN_STRING)
+      phase = a.dt * ((ph.KineticEnergy(p + a.hbar * lambda / 2.) -
+                       ph.KineticEnergy(p - a.hbar * lambda / 2.)) / a.hbar);
+    else
+      phase = a.dt * lambda * p / a.mass;
+    const double rr = __ldg(a.r_lambda + k) * (1.0 / (double)NX);
+    double sn, cs;
+    sincos(phase, &sn, &cs);
+    return make_double2(rr * cs, -rr * sn);
+  };
+  double2* pf = sm + ROWS * F::REGION + seq * blk_pre_slots(NX, E);
+  if (blk_pre(E) && blockIdx.x < NP / ROWS) odd_factor_pre<NX, E>(pf, t, factor);
   grid_wait();
   grid_launch_next();
   if (blockIdx.x == NP / ROWS) {
     if (obs_row != nullptr) consume_partials<NT>(a, scale_mode, obs_row, red);
     return;
   }
-  const int seq = threadIdx.x / T, t = threadIdx.x % T, row = blockIdx.x * ROWS + seq;
   WIG_BOUNDS_CHECK("x-pass row", row, NP);
   double2* Wr = W + (size_t)row * NX;
   double2 v[E];
@@ -829,23 +871,8 @@ __device__ __forceinline__ void xpass_blk_body(const WigArgs& a, const Phys& ph,
   double2* X = sm + seq * F::REGION;
   const auto sync = SeqSync<T, ROWS>::make(seq);
   F::template run<false>(v, X, a.btw_x, t, sync);
-  const int ii = (row + NP / 2) % NP;
-  const double p = a.dp * (ii - 0.5 * NP);
-  const double inv_n = 1.0 / (double)NX;
-  apply_odd_factor<NX, E>(v, X, t, sync, [&](int k) {
-    const int jj = (k + NX / 2) % NX;
-    const double lambda = a.dlambda * (jj - 0.5 * NX);
-    double phase;
-    if (KIN_STRING)
-      phase = a.dt * ((ph.KineticEnergy(p + a.hbar * lambda / 2.) -
-                       ph.KineticEnergy(p - a.hbar * lambda / 2.)) / a.hbar);
-    else
-      phase = a.dt * lambda * p / a.mass;
-    const double rr = __ldg(a.r_lambda + k) * inv_n;
-    double sn, cs;
-    sincos(phase, &sn, &cs);
-    return make_double2(rr * cs, -rr * sn);
-  });
+  if constexpr (blk_pre(E)) apply_odd_factor_pre<NX, E>(v, pf, t);
+  else apply_odd_factor<NX, E>(v, X, t, sync, factor);
   F::template run<true>(v, X, a.btw_x, t, sync);
 #pragma unroll
   for (int m = 0; m < E; ++m) Wr[t + T * m] = v[m];
@@ -920,7 +947,8 @@ __device__ __forceinline__ double column_observable(const WigArgs& a, double (*r
 // ppass_body; OBS 0 leaves the partial sums out (plans whose damping passes
 // write them).  The Caldeira-Leggett base A is kept in registers (TM 0) or, where a
 // thread's E elements leave no room for a second set, in tensor memory (TM 1).
-// Shared memory: C exchange regions.  gp_phase rows theta <= N_p / 2 are read (odd in theta).
+// Shared memory: C exchange regions, then C times blk_pre_slots(NP, E).
+// gp_phase rows theta <= N_p / 2 are read (odd in theta).
 // With scale_mode or obs_row (Strang) the last CTA (block NX / C) only records
 // the sample, as in the x-pass.
 template <class Phys, int NX, int NP, int C, int E, int DAMP, int KVN = 0, int HALF = 0, int FINAL = 1, int TM = 0,
@@ -931,8 +959,32 @@ __device__ __forceinline__ void ppass_blk_body(const WigArgs& a, const Phys& ph,
                                                const double* __restrict__ gp_phase = nullptr) {
   typedef BlockFft<double2, NP, E> F;
   constexpr int T = F::T, NT = C * T, RS = blk_stride(F::REGION, C);
+  constexpr bool PRE = blk_pre(E);
   static_assert(NT % 32 == 0 && C <= 32, "p-pass columns per CTA");
   extern __shared__ double2 sm[];
+  const int c = threadIdx.x % C, th = threadIdx.x / C, col = blockIdx.x * C + c;
+  const int jj = (col + NX / 2) % NX;
+  const double x = a.dx * (jj - 0.5 * NX);
+  // phase of the factor without the mean field, and its modulus
+  const auto polar = [&](int k, double mask) {
+    const int ii = (k + NP / 2) % NP;
+    const double theta = a.dtheta * (ii - 0.5 * NP);
+    const double phase = KVN ? a.dt * (-ph.DPotential(t, x) * theta)
+                             : (HALF ? 0.5 * a.dt : a.dt) * ((ph.Potential(t, x - a.hbar * theta / 2.) -
+                                                              ph.Potential(t, x + a.hbar * theta / 2.)) / a.hbar);
+    return make_double2(phase, __ldg((HALF ? a.r_theta_half : a.r_theta) + k) * mask);
+  };
+  const auto factor = [&](int k, double2 pr) {
+    if (HALF && gp_phase != nullptr) pr.x -= gp_phase[(size_t)k * NX + col];
+    double sn, cs;
+    sincos(pr.x, &sn, &cs);
+    return make_double2(pr.y * cs, -pr.y * sn);
+  };
+  double2* pf = sm + C * RS + c * blk_pre_slots(NP, E);
+  if (PRE && (FINAL || blockIdx.x < NX / C)) {
+    const double mask = a.mask1[col] * a.mask2s[col];
+    odd_factor_pre<NP, E>(pf, th, [&](int k) { return HALF ? polar(k, mask) : factor(k, polar(k, mask)); });
+  }
   grid_wait();
   grid_launch_next();
   if (FINAL == 0) {
@@ -942,7 +994,6 @@ __device__ __forceinline__ void ppass_blk_body(const WigArgs& a, const Phys& ph,
       return;
     }
   }
-  const int c = threadIdx.x % C, th = threadIdx.x / C, col = blockIdx.x * C + c;
   WIG_BOUNDS_CHECK("p-pass tile column", col, NX);
   double2* Wc = W + (size_t)th * NX + col;
   double2 v[E];
@@ -953,11 +1004,10 @@ __device__ __forceinline__ void ppass_blk_body(const WigArgs& a, const Phys& ph,
 #pragma unroll
     for (int m = 0; m < E; ++m) v[m] = cmul(v[m], s);
   }
+  if (PRE && HALF) odd_factor_pre<NP, E>(pf, th, [&](int k) { return factor(k, pf[k]); });   // the thread's own slots
   double2* X = sm + c * RS;
   const auto sync = SeqSync<NT, 1>::make(0);
-  const int jj = (col + NX / 2) % NX;
-  const double x = a.dx * (jj - 0.5 * NX);
-  const double mask = a.mask1[col] * a.mask2s[col];
+  const double mask = PRE ? 0. : a.mask1[col] * a.mask2s[col];
   double2 A[E];   // unused with TM
   // it 0: the potential factor; 1..3 (Caldeira-Leggett): A + c3 D(A + c12 D(A + c1 D A)),
   // D = IFFT_p[theta FFT_p(sign(p) f(p) .)] / n_p, the c's imaginary.  One rolled loop, so the
@@ -977,18 +1027,8 @@ __device__ __forceinline__ void ppass_blk_body(const WigArgs& a, const Phys& ph,
     }
     F::template run<false>(v, X, fresh(a.btw_p), th, sync);
     if (it == 0) {
-      apply_odd_factor<NP, E>(v, X, th, sync, [&](int k) {
-        const int ii = (k + NP / 2) % NP;
-        const double theta = a.dtheta * (ii - 0.5 * NP);
-        double phase = KVN ? a.dt * (-ph.DPotential(t, x) * theta)
-                           : (HALF ? 0.5 * a.dt : a.dt) * ((ph.Potential(t, x - a.hbar * theta / 2.) -
-                                                            ph.Potential(t, x + a.hbar * theta / 2.)) / a.hbar);
-        if (HALF && gp_phase != nullptr) phase -= gp_phase[(size_t)k * NX + col];
-        const double r = __ldg((HALF ? a.r_theta_half : a.r_theta) + k) * mask;
-        double sn, cs;
-        sincos(phase, &sn, &cs);
-        return make_double2(r * cs, -r * sn);
-      });
+      if constexpr (PRE) apply_odd_factor_pre<NP, E>(v, pf, th);
+      else apply_odd_factor<NP, E>(v, X, th, sync, [&](int k) { return factor(k, polar(k, mask)); });
     } else {
       const double* ths = fresh(a.theta_s + th);
 #pragma unroll
@@ -1219,7 +1259,7 @@ __device__ __forceinline__ void colsum_blk_body(const double2* __restrict__ W, d
 // Gross-Pitaevskii phase rows theta <= N_p / 2 (gp_phase_body; the phase is odd in theta): the
 // marginal P(x) from the chunk sums with the pending normalisation of scale_mode, its spectrum
 // once per row group, and per row one inverse transform.  psq (may be null) as gp_marginal_body.
-// Shared memory: ROWS exchange regions, then N_x doubles.
+// Shared memory: ROWS exchange regions, N_x doubles, then ROWS times blk_pre_slots(NX, E) doubles.
 template <int NX, int NP, int ROWS, int E>
 __device__ __forceinline__ void gp_phase_blk_body(const WigArgs& a, const double2* __restrict__ chunks, int n_chunks,
                                                   int scale_mode, double* __restrict__ phase_out,
@@ -1232,6 +1272,14 @@ __device__ __forceinline__ void gp_phase_blk_body(const WigArgs& a, const double
   double2* X = sm + seq * F::REGION;
   double* Ps = reinterpret_cast<double*>(sm + ROWS * F::REGION);
   const auto sync = SeqSync<T, ROWS>::make(seq);
+  // sin(lambda theta / 2) is odd in lambda: as apply_odd_factor, one value per pair
+  const double th = a.theta_s[row <= NP / 2 ? row : 0] * (double)NP;    // exact shifted Theta
+  double* fs = blk_pre(E) ? Ps + NX + seq * blk_pre_slots(NX, E) : reinterpret_cast<double*>(X);
+  const auto sines = [&]() {
+#pragma unroll 1
+    for (int k = t; k <= NX / 2; k += T) fs[k] = 2. * sin(0.5 * a.lambda_tab[k] * th);
+  };
+  if (blk_pre(E)) sines();
   grid_wait();
   grid_launch_next();
   double2 s = make_double2(1., 0.);
@@ -1264,13 +1312,11 @@ __device__ __forceinline__ void gp_phase_blk_body(const WigArgs& a, const double
 #pragma unroll
   for (int m = 0; m < E; ++m) v[m] = make_double2(Ps[t + T * m], 0.);
   F::template run<false>(v, X, a.btw_x, t, sync);
-  const double th = a.theta_s[row <= NP / 2 ? row : 0] * (double)NP;    // exact shifted Theta
-  // sin(lambda theta / 2) is odd in lambda: as apply_odd_factor, one value per pair
-  double* fs = reinterpret_cast<double*>(X);
-  sync();
-#pragma unroll 2
-  for (int k = t; k <= NX / 2; k += T) fs[k] = 2. * sin(0.5 * a.lambda_tab[k] * th);
-  sync();
+  if (!blk_pre(E)) {
+    sync();
+    sines();
+    sync();
+  }
 #pragma unroll
   for (int m = 0; m < E; ++m) {
     const int k = t + T * m;

@@ -27,8 +27,8 @@ int main(int argc, char** argv) {
   if (!read_all(argv[1], W.data(), npts * sizeof(double2))) return 4;
   const auto pad = [](int n, int e) { return n + n / std::min(e, 8); };
   const int gx = NP / WIG_BXR, xnt = WIG_BXR * (NX / WIG_BXE), gp = NX / WIG_BPC, pnt = WIG_BPC * (NP / WIG_BPE);
-  const size_t smx = (size_t)WIG_BXR * pad(NX, WIG_BXE) * sizeof(double2);
-  const size_t smp = (size_t)WIG_BPC * wig::blk_stride(pad(NP, WIG_BPE), WIG_BPC) * sizeof(double2);
+  const size_t smx = (size_t)WIG_BXR * (pad(NX, WIG_BXE) + wig::blk_pre_slots(NX, WIG_BXE)) * sizeof(double2);
+  const size_t smp = (size_t)WIG_BPC * (wig::blk_stride(pad(NP, WIG_BPE), WIG_BPC) + wig::blk_pre_slots(NP, WIG_BPE)) * sizeof(double2);
   const int n_cta_r = clampi(NX * NP / (4 * WIG_RNT), 1, 296);
   wig::WigArgs a{};
   a.dt = dt; a.dx = dx; a.dp = dp; a.dtheta = dtheta; a.dlambda = dlambda; a.mass = mass; a.hbar = hBar;
