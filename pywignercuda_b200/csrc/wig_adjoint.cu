@@ -148,9 +148,9 @@ extern "C" int wiga_create(const wiga_desc* d, wiga_handle** out) {
     h->bp_n = nx / b.pc;
     h->bp_nt = b.pc * (np / b.e);
     const int rx = nx + nx / std::min(b.e, 8), rp = np + np / std::min(b.e, 8);   // BlockFft::REGION
-    h->bx_smem = b.xr * rx * 16;
-    h->bp_smem = b.pc * wig::blk_stride(rp, b.pc) * 16;
-    h->bpt_smem = b.pc * wig::blk_stride(2 * rp, b.pc) * 16;
+    h->bx_smem = b.xr * (rx + wig::blk_pre_slots(nx, b.e)) * 16;
+    h->bp_smem = b.pc * (wig::blk_stride(rp, b.pc) + wig::blk_pre_slots(np, b.e)) * 16;
+    h->bpt_smem = b.pc * (wig::blk_stride(2 * rp, b.pc) + wig::blk_pre_slots(np, b.e)) * 16;
     const std::vector<double2> twx = block_twiddles(nx, b.e), twp = block_twiddles(np, b.e);
     double2 *x_d = nullptr, *p_d = nullptr;
     rc = h->bufs.alloc(&x_d, twx.size(), twx.data());
@@ -291,7 +291,9 @@ int adjoint_blk(wiga_handle* h, double2* lam, const double2* Y_dev, const double
       if (int rc = launch_after(h->fdot, h->bx_n, h->bx_nt, 0, st, da)) return rc;
     }
     void* pa[] = {&h->a, &lam, (void*)&Y, (void*)&eps, &step, &h->part, &h->dot, &n_dot, (void*)&s_dev};
-    if (int rc = launch_after(h->fbpt, h->bp_n, h->bp_nt, h->bpt_smem, st, pa)) return rc;
+    // reads eps before its wait (adj_moyal_pre): as the sweep's first launch it takes the stream's order
+    const bool first = !damped && k == n_steps - 1;
+    if (int rc = (first ? launch : launch_after)(h->fbpt, h->bp_n, h->bp_nt, h->bpt_smem, st, pa)) return rc;
     const double2* U = damped && k > 0 ? U_dev + (size_t)(k - 1) * plane : nullptr;
     void* xa[] = {&h->a, (void*)&lc, &lam, &sgn, (void*)&none, &zero, &nos, &step, (void*)&U, &h->dot, &h->part, &n_g, &grad};
     if (int rc = launch_after(h->fbx, h->bx_n + 1, h->bx_nt, h->bx_smem, st, xa)) return rc;
@@ -352,9 +354,10 @@ extern "C" int wiga_forward(wiga_handle* h, void* W_dev, const double* eps_dev, 
 namespace {
 
 // The launches of adjoint step `step` but the sum of its gradient partials, left in slot `slot` of
-// h->gpart (arguments checked by the caller).
+// h->gpart (arguments checked by the caller).  first: the call's first step, whose p-pass (which reads
+// eps before its wait, adj_moyal_pre) takes the stream's order unless the damped sums precede it.
 int adjoint_step_launch(wiga_handle* h, char* lam, const void* Y_dev, const void* U_dev, const void* s_dev,
-                        const double* eps_dev, long long s, int slot, cudaStream_t st) {
+                        const double* eps_dev, long long s, int slot, bool first, cudaStream_t st) {
   if (h->a.damped) {
     long long n = (long long)h->d.n_x * h->d.n_p;
     const char* lc = lam;
@@ -366,7 +369,8 @@ int adjoint_step_launch(wiga_handle* h, char* lam, const void* Y_dev, const void
   }
   double* gp = h->gpart + (size_t)slot * 3 * h->grid_p;
   void* pa[] = {&h->a, &lam, (void*)&Y_dev, (void*)&eps_dev, &s, &gp};
-  if (int rc = launch_after(h->fpt, h->grid_p, h->pw * 32, h->smem_p, st, pa)) return rc;
+  first = first && !h->a.damped;
+  if (int rc = (first ? launch : launch_after)(h->fpt, h->grid_p, h->pw * 32, h->smem_p, st, pa)) return rc;
   const char* lc = lam;
   double sgn = -1.;
   int use_pend = 0;
@@ -406,7 +410,7 @@ extern "C" int wig_step_adjoint(wiga_handle* h, void* lam_dev, const void* Y_dev
   if (h->blk)
     return adjoint_blk(h, (double2*)lam_dev, (const double2*)Y_dev, (const double2*)U_dev, (const double2*)s_dev,
                        eps_dev, step, 1, grad_dev, (cudaStream_t)stream);
-  if (int rc = adjoint_step_launch(h, (char*)lam_dev, Y_dev, U_dev, s_dev, eps_dev, (long long)step, 0,
+  if (int rc = adjoint_step_launch(h, (char*)lam_dev, Y_dev, U_dev, s_dev, eps_dev, (long long)step, 0, true,
                                    (cudaStream_t)stream))
     return rc;
   return grad_finalize_launch(h, grad_dev, (long long)step, 1, (cudaStream_t)stream);
@@ -426,7 +430,8 @@ extern "C" int wiga_adjoint_sweep(wiga_handle* h, void* lam_dev, const void* Y_d
   for (int64_t k = n_steps - 1, slot = 0; k >= 0; --k) {
     const char* Yk = (const char*)Y_dev + (size_t)k * plane;
     const char* Uk = U_dev ? (const char*)U_dev + (size_t)k * plane : nullptr;
-    if (int rc = adjoint_step_launch(h, (char*)lam_dev, Yk, Uk, s_dev, eps_dev, (long long)(step0 + k), (int)slot, st))
+    if (int rc = adjoint_step_launch(h, (char*)lam_dev, Yk, Uk, s_dev, eps_dev, (long long)(step0 + k), (int)slot,
+                                     k == n_steps - 1, st))
       return rc;
     if (++slot == kGradChunk || k == 0) {
       if (int rc = grad_finalize_launch(h, grad_dev, (long long)(step0 + k + slot - 1), (int)slot, st)) return rc;

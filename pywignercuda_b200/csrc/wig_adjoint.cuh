@@ -116,6 +116,11 @@ __device__ __forceinline__ void adj_xpass(const AArgs& a, const C* in, C* out, d
   const int lane = threadIdx.x & 31, grp = lane / G, g = lane % G;
   const int row = blockIdx.x * SPW + grp;
   WIG_BOUNDS_CHECK("adjoint x-pass row", row, NP);
+  // the kinetic factors do not depend on the state: evaluated before the wait for the preceding pass
+  __shared__ C pf[SPW * NX];
+  const double cq = a.dt * a.dp * a.dlambda * (double)ashift(row, NP) / (a.mass * 6.283185307179586477);
+#pragma unroll 8
+  for (int k = g; k < NX; k += G) pf[grp * NX + k] = adj_turn<C>(cq * (double)ashift(k, NX), __ldg(a.rtab + k), sgn);
   grid_wait();
   grid_launch_next();
   const C* src = in + (size_t)row * NX;
@@ -129,9 +134,8 @@ __device__ __forceinline__ void adj_xpass(const AArgs& a, const C* in, C* out, d
 #pragma unroll
   for (int e = 0; e < E; ++e) x.put(g * Q + e / G + E * (e % G), v[e]);
   __syncwarp();
-  const double cq = a.dt * a.dp * a.dlambda * (double)ashift(row, NP) / (a.mass * 6.283185307179586477);
 #pragma unroll 8
-  for (int k = g; k < NX; k += G) x.put(k, cmul(x.get(k), adj_turn<C>(cq * (double)ashift(k, NX), __ldg(a.rtab + k), sgn)));
+  for (int k = g; k < NX; k += G) x.put(k, cmul(x.get(k), pf[grp * NX + k]));   // the lane's own factors
   __syncwarp();
 #pragma unroll
   for (int e = 0; e < E; ++e) v[e] = x.get(g * Q + e / G + E * (e % G));
@@ -148,6 +152,23 @@ __device__ __forceinline__ void moyal_coeffs(const AArgs& a, double x, double ep
   const double kk = -a.dt * h / (3.141592653589793238 * a.hbar);
   *al = kk * ((4. * a.v4 * x * x + 2. * a.v2) * x + eps);
   *be = kk * h * h * (4. * a.v4 * x);
+}
+
+// Moyal factors of column col at the frequencies g, g + G, .. of its lane group, for the same lanes to
+// apply: they depend on eps_n alone, so the p-passes evaluate them before the wait for the preceding
+// pass (60-step gradients, B200: complex128 512^2 4.47 -> 4.16 ms, complex64 256^2 2.08 -> 1.70 ms with
+// the x-pass's factors; the complex64 bits stay).  eps_n may come from a kernel of the caller; a sweep's first launch therefore waits for the
+// stream in full (launch, not launch_after) or is a pass that does not read it.
+template <class C, int NP, int G>
+__device__ __forceinline__ void adj_moyal_pre(const AArgs& a, C* pf, int col, double eps, int g) {
+  double al, be;
+  moyal_coeffs(a, a.dx * (double)ashift(col, a.n_x), eps, &al, &be);
+  const double mm = __ldg(a.mm + col);
+#pragma unroll 8
+  for (int k = g; k < NP; k += G) {
+    const double j = (double)ashift(k, NP);
+    pf[k] = adj_turn<C>(j * fma(be, j * j, al), __ldg(a.rth + k) * mm, 1.);
+  }
 }
 
 // Coalesced load / store of a CT x NP tile of columns [col0, col0 + CT) (swizzled tile).
@@ -218,6 +239,13 @@ __device__ __forceinline__ void adj_block_sum(double (&v)[NV], double* out) {
   }
 }
 
+// v f with the products' order of contraction fixed (float2: the rounding of each component does not
+// depend on how the surrounding code is compiled)
+__device__ __forceinline__ double2 cmul_fma(double2 v, double2 f) { return cmul(v, f); }
+__device__ __forceinline__ float2 cmul_fma(float2 v, float2 f) {
+  return make_float2(fmaf(v.x, f.x, -(v.y * f.y)), fmaf(v.x, f.y, v.y * f.x));
+}
+
 // Forward p-pass: out = P(eps) in (undamped) or U = C P(eps) in (damped, and
 // this CTA's share of sum U into part[2 blockIdx.x .. + 1]); U_out (may be
 // null) receives a copy of the output.  in and out may alias.  Tiles: T0 (the
@@ -233,12 +261,14 @@ __device__ __forceinline__ void adj_ppass(const AArgs& a, const C* in, C* out, C
   C* t1 = t0 + CT * NP;
   const C* tw = reinterpret_cast<const C*>(a.tw_p);
   const int col0 = blockIdx.x * CT;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / G, g = lane % G;
+  const int c = adj_col<NP, WARPS>(warp, grp);
+  __shared__ C pf[CT * NP];
+  adj_moyal_pre<C, NP, G>(a, pf + (threadIdx.x / G) * NP, col0 + c, eps, g);
   grid_wait();
   grid_launch_next();
   adj_tile_load<C, NP, CT, NT>(t0, in, NX, col0);
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / G, g = lane % G;
-  const int c = adj_col<NP, WARPS>(warp, grp);
   const TileSlot<CT> sl{c};
   const SlotX<C, TileSlot<CT>> x0{t0, sl}, x1{t1, sl};
   C w[E];
@@ -249,15 +279,9 @@ __device__ __forceinline__ void adj_ppass(const AArgs& a, const C* in, C* out, C
 #pragma unroll
   for (int e = 0; e < E; ++e) x0.put(g * Q + e / G + E * (e % G), w[e]);
   __syncwarp();
-  const int col = col0 + c;
-  double al, be;
-  moyal_coeffs(a, a.dx * (double)ashift(col, NX), eps, &al, &be);
-  const double mm = __ldg(a.mm + col);
+  const C* pk = pf + (threadIdx.x / G) * NP;
 #pragma unroll 8
-  for (int k = g; k < NP; k += G) {
-    const double j = (double)ashift(k, NP);
-    x0.put(k, cmul(x0.get(k), adj_turn<C>(j * fma(be, j * j, al), __ldg(a.rth + k) * mm, 1.)));
-  }
+  for (int k = g; k < NP; k += G) x0.put(k, cmul_fma(x0.get(k), pk[k]));
   __syncwarp();
 #pragma unroll
   for (int e = 0; e < E; ++e) w[e] = x0.get(g * Q + e / G + E * (e % G));
@@ -306,12 +330,14 @@ __device__ __forceinline__ void adj_ppass_T(const AArgs& a, C* lam, const C* Y, 
   C* t1 = t0 + CT * NP;
   const C* tw = reinterpret_cast<const C*>(a.tw_p);
   const int col0 = blockIdx.x * CT;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / G, g = lane % G;
+  const int c = adj_col<NP, WARPS>(warp, grp);
+  __shared__ C pf[CT * NP];
+  adj_moyal_pre<C, NP, G>(a, pf + (threadIdx.x / G) * NP, col0 + c, eps, g);
   grid_wait();
   grid_launch_next();
   adj_tile_load<C, NP, CT, NT>(t0, lam, NX, col0);
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / G, g = lane % G;
-  const int c = adj_col<NP, WARPS>(warp, grp);
   const TileSlot<CT> sl{c};
   const SlotX<C, TileSlot<CT>> x0{t0, sl}, x1{t1, sl};
   C w[E];
@@ -355,17 +381,14 @@ __device__ __forceinline__ void adj_ppass_T(const AArgs& a, C* lam, const C* Y, 
 #pragma unroll
   for (int e = 0; e < E; ++e) x0.put(g * Q + e / G + E * (e % G), w[e]);
   __syncwarp();
-  const int col = col0 + c;
-  const double xc = a.dx * (double)ashift(col, NX);
-  double al, be;
-  moyal_coeffs(a, xc, eps, &al, &be);
-  const double mm = __ldg(a.mm + col);
+  const double xc = a.dx * (double)ashift(col0 + c, NX);
   const double h = 0.5 * a.hbar * a.dtheta;   // u = h j
+  const C* pk = pf + (threadIdx.x / G) * NP;
   double gq[3] = {0., 0., 0.};
 #pragma unroll 8
   for (int k = g; k < NP; k += G) {
     const double j = (double)ashift(k, NP);
-    const C d = adj_turn<C>(j * fma(be, j * j, al), __ldg(a.rth + k) * mm, 1.);
+    const C d = pk[k];
     const C yd = cmul(x1.get(k), d);
     const C U = x0.get(k);
     // Re(i conj(U) yd) = U.y yd.x - U.x yd.y
@@ -434,7 +457,8 @@ __device__ __forceinline__ void adj_dot_rows(const double2 (&v)[E], const double
 // x-pass: out = K (in / s) or K^H in, ROWS rows per CTA.  part (may be null): 2 n_part doubles, the
 // partials of the sum behind s (s_out[step], when given, records it).  U (may be null): plane of the
 // next adjoint step, whose dot partials with out go to dot[2 blockIdx.x ..].  gpart (may be null):
-// 3 n_g gradient partials, summed into grad[3 step ..].  Shared memory: ROWS exchange regions.
+// 3 n_g gradient partials, summed into grad[3 step ..].  Shared memory: ROWS exchange regions, then
+// ROWS times blk_pre_slots(NX, E) (the factors, before the wait).
 template <int NX, int NP, int ROWS, int E>
 __device__ __forceinline__ void adj_xpass_blk(const AArgs& a, const double2* in, double2* out, double sgn,
                                               const double* part, int n_part, double2* s_out, long long step,
@@ -444,6 +468,14 @@ __device__ __forceinline__ void adj_xpass_blk(const AArgs& a, const double2* in,
   constexpr int T = F::T, NT = ROWS * T;
   static_assert(NT % 32 == 0 && (T % 32 == 0 || 32 % T == 0), "x-pass rows per CTA");
   extern __shared__ double2 smd[];
+  const int seq = threadIdx.x / T, t = threadIdx.x % T, row = blockIdx.x * ROWS + seq;
+  double2* pf = smd + ROWS * F::REGION + seq * blk_pre_slots(NX, E);
+  if (blockIdx.x < NP / ROWS) {
+    const double cq = a.dt * a.dp * a.dlambda * (double)ashift(row, NP) / (a.mass * 6.283185307179586477);
+    odd_factor_pre<NX, E>(pf, t, [&](int k) {
+      return adj_turn<double2>(cq * (double)ashift(k, NX), __ldg(a.rtab + k), sgn);
+    });
+  }
   grid_wait();
   grid_launch_next();
   if (blockIdx.x == NP / ROWS) {
@@ -459,7 +491,6 @@ __device__ __forceinline__ void adj_xpass_blk(const AArgs& a, const double2* in,
     }
     return;
   }
-  const int seq = threadIdx.x / T, t = threadIdx.x % T, row = blockIdx.x * ROWS + seq;
   WIG_BOUNDS_CHECK("adjoint x-pass row", row, NP);
   const size_t base = (size_t)row * NX + t;
   double2 v[E];
@@ -475,10 +506,7 @@ __device__ __forceinline__ void adj_xpass_blk(const AArgs& a, const double2* in,
   double2* X = smd + seq * F::REGION;
   const auto sync = SeqSync<T, ROWS>::make(seq);
   F::template run<false>(v, X, a.btw_x, t, sync);
-  const double cq = a.dt * a.dp * a.dlambda * (double)ashift(row, NP) / (a.mass * 6.283185307179586477);
-  apply_odd_factor<NX, E>(v, X, t, sync, [&](int k) {
-    return adj_turn<double2>(cq * (double)ashift(k, NX), __ldg(a.rtab + k), sgn);
-  });
+  apply_odd_factor_pre<NX, E>(v, pf, t);
   F::template run<true>(v, X, a.btw_x, t, sync);
 #pragma unroll
   for (int m = 0; m < E; ++m) out[base + T * m] = v[m];
@@ -499,14 +527,20 @@ __device__ __forceinline__ void adj_dot_blk(const double2* lam, const double2* U
   adj_dot_rows<E, T, NT>(v, U + base, dot);
 }
 
-// the Moyal factor of column x for every frequency, through the exchange region (apply_odd_factor)
-template <int NP>
-__device__ __forceinline__ double2 adj_moyal(const AArgs& a, double al, double be, double mm, int k) {
-  const double j = (double)ashift(k, NP);
-  return adj_turn<double2>(j * fma(be, j * j, al), __ldg(a.rth + k) * mm, 1.);
+// the Moyal factors of column col, k <= N_p / 2 (odd_factor_pre; see adj_moyal_pre for eps)
+template <int NX, int NP, int E>
+__device__ __forceinline__ void adj_moyal_pre_blk(const AArgs& a, double2* pf, int col, double eps, int t) {
+  double al, be;
+  moyal_coeffs(a, a.dx * (double)ashift(col, NX), eps, &al, &be);
+  const double mm = __ldg(a.mm + col);
+  odd_factor_pre<NP, E>(pf, t, [&](int k) {
+    const double j = (double)ashift(k, NP);
+    return adj_turn<double2>(j * fma(be, j * j, al), __ldg(a.rth + k) * mm, 1.);
+  });
 }
 
 // forward p-pass (adj_ppass), C columns per CTA; damped: out holds U and part the CTA's share of its sum.
+// Shared memory (and of adj_ppass_T_blk): the exchange regions, then C times blk_pre_slots(NP, E).
 template <int NX, int NP, int C, int E>
 __device__ __forceinline__ void adj_ppass_blk(const AArgs& a, const double2* in, double2* out, double eps,
                                               double* part) {
@@ -517,14 +551,15 @@ __device__ __forceinline__ void adj_ppass_blk(const AArgs& a, const double2* in,
   const int c = threadIdx.x % C, t = threadIdx.x / C, col = blockIdx.x * C + c;
   WIG_BOUNDS_CHECK("adjoint p-pass column", col, NX);
   const size_t base = (size_t)t * NX + col;
+  double2* pf = smd + C * RS + c * blk_pre_slots(NP, E);
+  adj_moyal_pre_blk<NX, NP, E>(a, pf, col, eps, t);
+  grid_wait();
+  grid_launch_next();
   double2 v[E], A[E];
 #pragma unroll
   for (int m = 0; m < E; ++m) v[m] = in[base + (size_t)(T * m) * NX];
   double2* X = smd + c * RS;
   const auto sync = SeqSync<NT, 1>::make(0);
-  double al, be;
-  moyal_coeffs(a, a.dx * (double)ashift(col, NX), eps, &al, &be);
-  const double mm = __ldg(a.mm + col);
   const int n_it = a.damped ? 4 : 1;
 #pragma unroll 1
   for (int it = 0; it < n_it; ++it) {
@@ -535,7 +570,7 @@ __device__ __forceinline__ void adj_ppass_blk(const AArgs& a, const double2* in,
     }
     F::template run<false>(v, X, fresh(a.btw_p), t, sync);
     if (it == 0) {
-      apply_odd_factor<NP, E>(v, X, t, sync, [&](int k) { return adj_moyal<NP>(a, al, be, mm, k); });
+      apply_odd_factor_pre<NP, E>(v, pf, t);
     } else {
       const double* ths = fresh(a.ths + t);
 #pragma unroll
@@ -578,6 +613,10 @@ __device__ __forceinline__ void adj_ppass_T_blk(const AArgs& a, double2* lam, co
   const int c = threadIdx.x % C, t = threadIdx.x / C, col = blockIdx.x * C + c;
   WIG_BOUNDS_CHECK("adjoint p-pass column", col, NX);
   const size_t base = (size_t)t * NX + col;
+  double2* pf = smd + C * RS + c * blk_pre_slots(NP, E);
+  adj_moyal_pre_blk<NX, NP, E>(a, pf, col, eps, t);
+  grid_wait();
+  grid_launch_next();
   double2 w[2][E];   // [0] lam, [1] the Horner base of C^H, then Y
 #pragma unroll
   for (int m = 0; m < E; ++m) w[0][m] = lam[base + (size_t)(T * m) * NX];
@@ -614,19 +653,12 @@ __device__ __forceinline__ void adj_ppass_T_blk(const AArgs& a, double2* lam, co
   for (int m = 0; m < E; ++m) w[1][m] = Y[base + (size_t)(T * m) * NX];
   F::template run_many<false>(w, X, fresh(a.btw_p), t, sync);
   const double xc = a.dx * (double)ashift(col, NX);
-  double al, be;
-  moyal_coeffs(a, xc, eps, &al, &be);
-  const double mm = __ldg(a.mm + col);
   const double h = 0.5 * a.hbar * a.dtheta;   // u = h j
-  sync();
-#pragma unroll 2
-  for (int k = t; k <= NP / 2; k += T) X[k] = adj_moyal<NP>(a, al, be, mm, k);
-  sync();
   double gq[3] = {0., 0., 0.};
 #pragma unroll
   for (int m = 0; m < E; ++m) {
     const int k = t + T * m;
-    const double2 d = k <= NP / 2 ? X[k] : cconj(X[NP - k]);
+    const double2 d = k <= NP / 2 ? pf[k] : cconj(pf[NP - k]);
     const double2 U = w[0][m], yd = cmul(w[1][m], d);
     const double re = U.y * yd.x - U.x * yd.y;   // Re(i conj(U) yd)
     const double j = (double)ashift(k, NP), u = h * j;

@@ -30,16 +30,12 @@ wiga_bx(wig::AArgs a, const double2* in, double2* out, double sgn, const double*
 
 extern "C" __global__ void __launch_bounds__(WIGA_BPC * (WIGA_NP / WIGA_BPE), WIGA_BPMB)
 wiga_bp(wig::AArgs a, const double2* in, double2* out, const double* eps, long long step, double* part) {
-  wig::grid_wait();
-  wig::grid_launch_next();
   wig::adj_ppass_blk<WIGA_NX, WIGA_NP, WIGA_BPC, WIGA_BPE>(a, in, out, eps[step], part);
 }
 
 extern "C" __global__ void __launch_bounds__(WIGA_BPC * (WIGA_NP / WIGA_BPE), WIGA_BPMB)
 wiga_bpt(wig::AArgs a, double2* lam, const double2* Y, const double* eps, long long step, double* part,
          const double* dot, int n_dot, const double2* s_in) {
-  wig::grid_wait();
-  wig::grid_launch_next();
   wig::adj_ppass_T_blk<WIGA_NX, WIGA_NP, WIGA_BPC, WIGA_BPE>(a, lam, Y, eps[step], part, dot, n_dot, s_in, step);
 }
 

@@ -121,9 +121,10 @@ ADJOINT_LAUNCHES = """
   const std::vector<double2> bx = wighost::block_twiddles(nx, WIGA_BXE), bp = wighost::block_twiddles(np, WIGA_BPE);
   a.btw_x = bx.data(); a.btw_p = bp.data();
   const int bxn = np / WIGA_BXR, bxt = WIGA_BXR * (nx / WIGA_BXE), bpn = nx / WIGA_BPC, bpt = WIGA_BPC * (np / WIGA_BPE);
-  const size_t sbx = (size_t)WIGA_BXR * pad(nx, WIGA_BXE) * 16;
-  const size_t sbp = (size_t)WIGA_BPC * wig::blk_stride(pad(np, WIGA_BPE), WIGA_BPC) * 16;
-  const size_t sbt = (size_t)WIGA_BPC * wig::blk_stride(2 * pad(np, WIGA_BPE), WIGA_BPC) * 16;
+  const size_t sbx = (size_t)WIGA_BXR * (pad(nx, WIGA_BXE) + wig::blk_pre_slots(nx, WIGA_BXE)) * 16;
+  const size_t pre = (size_t)WIGA_BPC * wig::blk_pre_slots(np, WIGA_BPE) * 16;
+  const size_t sbp = (size_t)WIGA_BPC * wig::blk_stride(pad(np, WIGA_BPE), WIGA_BPC) * 16 + pre;
+  const size_t sbt = (size_t)WIGA_BPC * wig::blk_stride(2 * pad(np, WIGA_BPE), WIGA_BPC) * 16 + pre;
   std::vector<double> bpart(3 * bpn), dot(2 * bxn);
   double* part_p = bpart.data();
   const double2* cur = W.data();
