@@ -123,6 +123,8 @@ class Dirac3Desc(ctypes.Structure):
 SIGNATURES = [
     ('wig_create', c_int, [POINTER(WigDesc), POINTER(c_void_p)]),
     ('wig_run', c_int, [c_void_p, c_void_p, c_int64, c_int64, c_uint32, _DP, c_void_p]),
+    ('wig_run_observables', c_int, [c_void_p, c_void_p, c_int64, c_void_p]),
+    ('wig_check_observables', c_int, [_DP, c_int64]),
     ('wig_run_host', c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_uint32, _DP, c_void_p]),
     ('wig_run_many', c_int, [POINTER(c_void_p), POINTER(c_void_p), c_int64, c_int64, c_int64, c_uint32,
                              POINTER(_DP), c_void_p]),

@@ -1095,6 +1095,20 @@ extern "C" int wig_run(wig_handle* h, void* W_dev, int64_t t_index0, int64_t n_p
   return WIG_OK;
 }
 
+extern "C" int wig_run_observables(wig_handle* h, double* out_dev, int64_t n_rows, void* stream) {
+  if (!h || !out_dev) return fail(WIG_ERR_ARG, "wig_run_observables: null argument");
+  if (n_rows < 1 || (size_t)n_rows * WIG_NOBS > h->obs_cap)
+    return fail(WIG_ERR_ARG, "wig_run_observables: the last run did not record %lld rows", (long long)n_rows);
+  cudaStream_t st = (cudaStream_t)stream;
+  WIG_CUDA(cudaMemcpyAsync(out_dev, h->obs, (size_t)n_rows * WIG_NOBS * sizeof(double), cudaMemcpyDeviceToDevice, st));
+  return h->tma ? wig_check_status(h, st) : WIG_OK;
+}
+
+extern "C" int wig_check_observables(const double* obs_host, int64_t n_rows) {
+  if (!obs_host || n_rows < 0) return fail(WIG_ERR_ARG, "wig_check_observables: bad arguments");
+  return check_finite(obs_host, (size_t)n_rows * WIG_NOBS, "wig_run observables");
+}
+
 // ------------------------------------------------------------------ Bloch (imaginary time)
 // GPU_Wigner2D_GPitaevskii_Bloch.Run / Run_ExitedState1 (:2105-2545): the device
 // work of one step; the host keeps the reference's accept / reject and

@@ -289,6 +289,14 @@ class GPU_Wigner2D_FFT(Propagator_Base):
                                   st.cuda_stream), 'wig_run')
         return obs
 
+    def _stretch(self, W, n_prop, t_index0, continue_run, samples):
+        """``propagate`` on the current stream without waiting for it: rows ``t_index0`` ..
+        ``t_index0 + n_prop`` of the device tensor ``samples`` receive the observables."""
+        lib, st = _lib.load(), _torch().cuda.current_stream(W.device).cuda_stream
+        flags = _lib.WIG_RUN_CONTINUE if continue_run else 0
+        check(lib.wig_run(self._handle, W.data_ptr(), t_index0, n_prop, flags, None, st), 'wig_run')
+        check(lib.wig_run_observables(self._handle, samples[t_index0].data_ptr(), n_prop + 1, st), 'wig_run')
+
     def _frame_writer(self, W):
         """The output file (when ``fileName`` is set) with its header, and the
         asynchronous frame writer that fills ``frames`` and the file."""
@@ -318,7 +326,8 @@ class GPU_Wigner2D_FFT(Propagator_Base):
             W = torch.from_numpy(W0.copy()).to(dev)
             n_total = int(self.timeSteps) + 1             # Run :1776 loops over 0..timeSteps
             skip = max(int(self.skipFrames), 1)
-            obs = np.empty((n_total + 1, _lib.WIG_NOBS))
+            # the stretches between frames run without a host wait: their samples collect on the device
+            samples = torch.zeros((max(n_total, 0) + 1, _lib.WIG_NOBS), dtype=torch.float64, device=dev)
             sink, writer = self._frame_writer(W)
             saved = []
             t, cont = 0, False
@@ -326,15 +335,16 @@ class GPU_Wigner2D_FFT(Propagator_Base):
                 while t < n_total:
                     if t % skip == 0 and t <= self.timeSteps:
                         if not cont:                       # W must be normalised first
-                            obs[0] = self.propagate(W, 0)[0]
+                            self._stretch(W, 0, 0, False, samples)
                             cont = True
                         writer.capture(t, W)               # the sample before step t (:1880-1882)
                         saved.append(t)
                     nxt = min(n_total, (t // skip + 1) * skip)
-                    o = self.propagate(W, nxt - t, t_index0=t, continue_run=cont)
-                    obs[t:nxt + 1] = o
+                    self._stretch(W, nxt - t, t, cont, samples)
                     t, cont = nxt, True
                 W_end = W.cpu().numpy()
+                obs = samples.cpu().numpy()
+                check(_lib.load().wig_check_observables(dptr(obs), obs.shape[0]), 'wig_run')
             finally:
                 writer.close()
         n = int(self.timeSteps) + 1
