@@ -46,7 +46,7 @@ template <class C, int N> struct RegFft {
   static_assert(E * G == N && E >= G && (N & (N - 1)) == 0, "RegFft: N must be a power of two in [64, 1024]");
 
   // lane g (0 <= g < G) of its group; x.put(s, v) / x.get(s) store and load
-  // the sequence's exchange slot s < N (an exchange functor, see SlotX / PairX).
+  // the sequence's exchange slot s < N (an exchange functor, see SlotX).
   template <class X>
   __device__ __forceinline__ static void fwdx(C (&v)[E], const X& x, const C* tf, int g) {
     dft_r<E, false>(v);
@@ -109,22 +109,12 @@ template <int CT> struct TileSlot {
   __device__ __forceinline__ int operator()(int k) const { return k * CT + (c ^ tile_sw<CT>(k)); }
 };
 
-// Exchange functors of RegFft::fwdx / invx.
-// SlotX: element s at sm[slot(s)] (the element type of the transform).
+// Exchange functor of RegFft::fwdx / invx: element s at sm[slot(s)] (the element type of the transform).
 template <class C, class Slot> struct SlotX {
   C* sm;
   Slot slot;
   __device__ __forceinline__ void put(int s, C v) const { sm[slot(s)] = v; }
   __device__ __forceinline__ C get(int s) const { return sm[slot(s)]; }
-};
-// PairX: an FP64 sequence exchanged through the 8-byte slots of two columns of
-// a float2 tile: the real part of element s in slot s of column 1, the
-// imaginary part in slot s of column 2 (each slot reinterpreted as one double).
-template <class Slot> struct PairX {
-  double* sm;
-  Slot s1, s2;
-  __device__ __forceinline__ void put(int s, double2 v) const { sm[s1(s)] = v.x; sm[s2(s)] = v.y; }
-  __device__ __forceinline__ double2 get(int s) const { return make_double2(sm[s1(s)], sm[s2(s)]); }
 };
 
 template <class C, int N>
