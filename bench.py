@@ -503,10 +503,10 @@ def run_gp(args, world, rank, local):
             'config': {'workload': 'GPU_Wigner2D_GPitaevskii 1024x1024 double well V=0.05x^4-x^2, a_GP=0.5, '
                                    'Caldeira-Leggett gamma=0.1 D_theta=0.1 f=|p|, cat state, dt=0.005',
                        'replicas_per_gpu': R, 'l2': 'per-step working set %d MB > 126 MB L2' % (R * 24)},
-            'roofline': {'bound': 'hbm', 'kernel': 'Strang step (9 launches, step average)',
+            'roofline': {'bound': 'hbm', 'kernel': 'Strang step (6 launches, step average)',
                          'algorithmic_bytes_per_point': GP_BYTES, 'achieved': achieved, 'peak': peak,
                          'unit': 'GB/s', 'frac': achieved / peak, 'peak_kind': peak_kind, 'traffic': None},
-            'gpu_launches': R * 9 * steps, 'clocks': clk.summary()}
+            'gpu_launches': R * 6 * steps, 'clocks': clk.summary()}
     if rank == 0 and args.cpu_baseline:
         prm = WignerParams(NX, NP, AMP, AMP, DT, potential=POT, dpotential=DPOT, kinetic='0.5*p*p', gamma=GAMMA,
                            d_theta=D_THETA, damping='CaldeiraLeggett', fp_damping='fabs(p)')

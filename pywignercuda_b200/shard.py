@@ -18,10 +18,10 @@ import math
 # (SM clock 1965 MHz, default register caps).  The cost per point is nearly flat in the size:
 # the passes are bound by latency and issue, not by the transform's log factor.
 MEASURED_NS = {
-    '128': 0.01832, '128d': 0.02487,
-    '256': 0.01807, '256d': 0.02531,
-    '512': 0.01957, '512d': 0.02508,
-    '1024': 0.02102, '1024d': 0.02808,
+    '128': 0.01308, '128d': 0.01897,
+    '256': 0.01342, '256d': 0.01952,
+    '512': 0.01224, '512d': 0.01744,
+    '1024': 0.01339, '1024d': 0.01935,
 }
 
 
