@@ -533,23 +533,27 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
     P->bx = !stockham && NX >= 32 ? 1 : 0;
     P->bp = !stockham && NP >= 32 ? 1 : 0;
     // Elements a thread: as many as the grid leaves threads for.  16 (two stage boundaries in
-    // shared memory up to 4096 points, 128 registers, 16 warps per SM) from 2^19 points, 8 from
-    // 2^17, below that 4, where the step is a chain of latencies and more warps shorten it.
-    // Damped Lie step, us: 1024^2 65 / 83 with 16 / 8; 512^2 32 / 26 / 32 with 16 / 8 / 4;
-    // 512 x 256 - / 21 / 21; 256^2 24 / 18 / 15; 128^2 24 / 17 / 13; 1024 x 64 - / 20 / 16.
+    // shared memory up to 4096 points, 128 registers, 16 warps per SM) from 2^20 points along x and
+    // 2^19 along p, 8 from 2^17, below that 4, where the step is a chain of latencies and more warps
+    // shorten it.  Damped step, us, x,p of 16,16 / 8,16 / 8,8: 1024^2 65 / 65 / 75; 512 x 1024
+    // 42 / 38 / 39; 1024 x 512 39 / 38 / 36; 2048 x 256 38 / 37 / 38 (time-dependent 40 / 38 / 45);
+    // 4096 x 128 41 / 39 / 50.  Both of 16 / 8 / 4: 512^2 36 / 22 / 28; 512 x 256 - / 16 / 16;
+    // 256^2 26 / 13 / 11; 128^2 - / 12 / 10; 1024 x 64 - / 15 / 13.
     const long pts = (long)NX * NP;
-    const auto elems = [&](int n) { return std::max(pts >= (1L << 19) ? 16 : (pts >= (1L << 17) ? 8 : 4), n / 512); };
-    P->bxe = elems(NX);
-    P->bpe = elems(NP);
+    const auto elems = [&](int n, long top) {
+      return std::max(pts >= top ? 16 : (pts >= (1L << 17) ? 8 : 4), n / 512);
+    };
+    P->bxe = elems(NX, 1L << 20);
+    P->bpe = elems(NP, 1L << 19);
     // x: one row per CTA (at least a warp).  p: two columns (32-byte segments of a grid row) where that
-    // leaves a CTA for every SM, else one: 256^2 undamped step 9.1 / 10.2 us with one / two, 128 x 1024
-    // damped 22 / 28, 512 x 256 21 / 21, 1024^2 98 / 76.
+    // leaves a CTA for every SM, else one: 256^2 undamped step 7.7 / 8.7 us with one / two, 128 x 1024
+    // damped 17.3 / 23.9, 512 x 256 16.4 / 15.8, 1024^2 68 / 65.
     P->bxr = std::max(1, 32 * P->bxe / NX);
     P->bpc = std::max(P->bpe >= 8 && NX / 2 >= 148 ? 2 : 1, 32 * P->bpe / NP);
     while (P->bpc > 1 && P->bpc * (NP / P->bpe) > 512) P->bpc /= 2;
     P->bxmb = P->bpmb = 0;
     // the Caldeira-Leggett base: with 16 elements a thread in tensor memory (1024^2 damped step 65 us;
-    // in shared memory, two CTAs per SM instead of four, 70), else in registers
+    // in registers, spilling, 80), else in registers
     P->bpa = P->damp && P->bpe == 16 ? 1 : 0;
     // WIG_BTILING="xe,xr,xmb,pe,pc,pmb,pa" overrides the tiles for tuning runs (0: default; pa: -1 default)
     if (const char* tv = getenv("WIG_BTILING")) {

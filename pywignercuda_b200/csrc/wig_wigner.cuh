@@ -798,13 +798,13 @@ __device__ __forceinline__ void apply_odd_factor(double2 (&v)[E], double2* s, in
   }
 }
 
-// With at most 8 elements a thread (grids below 2^19 points, where a CTA of the next pass is resident
-// beside the current one) the factors, which do not depend on W, are evaluated before the wait for the
-// preceding pass, into their own N / 2 + 1 slots a sequence (blk_pre_slots).  Steps, us, before /
-// after: 256^2 9.4 / 7.8, 128 x 64 damped 12.8 / 10.1, 512^2 16.4 / 13.2, 512^2 damped 26.0 / 21.8,
-// 4096 x 64 damped 31.9 / 26.7, Gross-Pitaevskii 512^2 (phases and the sines of the mean field) 61.4 /
-// 56.0.  With 16 elements the slots take the shared memory of resident CTAs of the same pass: 1024^2
-// damped 64.6 / 69.4, 2048 x 256 damped 39.6 / 64.4, so those evaluate them in place.
+// With at most 8 elements a thread (grids below 2^19 points, rows below 2^20, where a CTA of the next
+// pass is resident beside the current one) the factors, which do not depend on W, are evaluated before
+// the wait for the preceding pass, into their own N / 2 + 1 slots a sequence (blk_pre_slots).  Steps,
+// us, before / after: 256^2 9.4 / 7.8, 128 x 64 damped 12.8 / 10.1, 512^2 16.4 / 13.2, 512^2 damped
+// 26.0 / 21.8, 4096 x 64 damped 31.9 / 26.7, Gross-Pitaevskii 512^2 (phases and the sines of the mean
+// field) 61.4 / 56.0.  With 16 elements the slots take the shared memory of resident CTAs of the same
+// pass: 1024^2 damped 64.6 / 69.4, 2048 x 256 damped 39.6 / 64.4, so those evaluate them in place.
 __host__ __device__ constexpr bool blk_pre(int e) { return e <= 8; }
 __host__ __device__ constexpr int blk_pre_slots(int n, int e) { return blk_pre(e) ? n / 2 + 1 : 0; }
 template <int N, int E, class Factor>
