@@ -45,22 +45,6 @@ constexpr int kGradChunk = 64;   // adjoint steps whose gradient partials one la
 
 bool pow2_64_1024(int n) { return n >= 64 && n <= 1024 && (n & (n - 1)) == 0; }
 
-int check_desc(const wiga_desc* d) {
-  if (!d) return fail(WIG_ERR_ARG, "wiga: null descriptor");
-  if (d->abi_version != WIG_ABI_VERSION)
-    return fail(WIG_ERR_ARG, "wiga: abi_version %d, library %d", d->abi_version, WIG_ABI_VERSION);
-  if (!pow2_64_1024(d->n_x) || !pow2_64_1024(d->n_p))
-    return fail(WIG_ERR_ARG, "wiga: grid %d x %d, grids must be powers of two in [64, 1024]", d->n_x, d->n_p);
-  if (!(d->x_amplitude > 0) || !(d->p_amplitude > 0) || !(d->hbar != 0) || !(d->mass != 0) ||
-      !std::isfinite(d->dt))
-    return fail(WIG_ERR_ARG, "wiga: amplitudes > 0, hbar and mass nonzero, dt finite");
-  if (d->precision != WIGA_PREC_C64 && d->precision != WIGA_PREC_C128)
-    return fail(WIG_ERR_ARG, "wiga: precision must be WIGA_PREC_C64 or WIGA_PREC_C128");
-  if (!std::isfinite(d->gamma) || !(d->f_eps >= 0.))
-    return fail(WIG_ERR_ARG, "wiga: gamma must be finite and f_eps >= 0");
-  return WIG_OK;
-}
-
 // Tiles of the register-blocked complex128 passes: 8 elements a thread, 4 on grids below 2^17 points;
 // one row per CTA; two columns where that leaves a CTA for every SM (as the Lie step's passes).
 struct BlkTiles {
@@ -76,13 +60,34 @@ BlkTiles blk_tiles(int nx, int np) {
     int v[3];
     if (sscanf(tv, "%d,%d,%d", &v[0], &v[1], &v[2]) == 3) {
       if (v[0] == 4 || v[0] == 8) t.e = v[0];
-      t.xr = std::max(v[1], std::max(1, 32 * t.e / nx));
-      t.pc = std::max(v[2] > 0 ? v[2] : 1, std::max(1, 32 * t.e / np));
+      t.xr = clampi(v[1], std::max(1, 32 * t.e / nx), 1024);
+      t.pc = clampi(v[2], std::max(1, 32 * t.e / np), 1024);
     }
   }
   t.xmb = std::max(1, std::min(32, 512 / (t.xr * (nx / t.e))));
   t.pmb = std::max(1, std::min(32, 512 / (t.pc * (np / t.e))));
   return t;
+}
+
+int check_desc(const wiga_desc* d) {
+  if (!d) return fail(WIG_ERR_ARG, "wiga: null descriptor");
+  if (d->abi_version != WIG_ABI_VERSION)
+    return fail(WIG_ERR_ARG, "wiga: abi_version %d, library %d", d->abi_version, WIG_ABI_VERSION);
+  if (!pow2_64_1024(d->n_x) || !pow2_64_1024(d->n_p))
+    return fail(WIG_ERR_ARG, "wiga: grid %d x %d, grids must be powers of two in [64, 1024]", d->n_x, d->n_p);
+  if (!(d->x_amplitude > 0) || !(d->p_amplitude > 0) || !(d->hbar != 0) || !(d->mass != 0) ||
+      !std::isfinite(d->dt))
+    return fail(WIG_ERR_ARG, "wiga: amplitudes > 0, hbar and mass nonzero, dt finite");
+  if (d->precision != WIGA_PREC_C64 && d->precision != WIGA_PREC_C128)
+    return fail(WIG_ERR_ARG, "wiga: precision must be WIGA_PREC_C64 or WIGA_PREC_C128");
+  if (!std::isfinite(d->gamma) || !(d->f_eps >= 0.))
+    return fail(WIG_ERR_ARG, "wiga: gamma must be finite and f_eps >= 0");
+  if (d->precision == WIGA_PREC_C128) {
+    const BlkTiles t = blk_tiles(d->n_x, d->n_p);
+    if (int rc = check_blk_tile("WIG_ADJ_BTILING", t.xr, d->n_x / t.e, d->n_p, 1024)) return rc;
+    return check_blk_tile("WIG_ADJ_BTILING", t.pc, d->n_p / t.e, d->n_x, 32);
+  }
+  return WIG_OK;
 }
 
 std::string source(const wiga_desc* d) {

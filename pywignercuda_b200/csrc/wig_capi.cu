@@ -316,6 +316,13 @@ int occupancy(CUfunction f, int threads, int dyn_smem) {
   return n < 1 ? 1 : n;
 }
 
+int check_blk_tile(const char* env, int seqs, int threads, long total, int most) {
+  const long nt = (long)seqs * threads;
+  if (seqs < 1 || (seqs & (seqs - 1)) || seqs > most || total % seqs || nt > 1024 || nt % 32)
+    return fail(WIG_ERR_ARG, "%s: tile of %d of %ld sequences, %ld threads", env, seqs, total, nt);
+  return WIG_OK;
+}
+
 int ensure_obs(double** buf, size_t* cap, size_t need) {
   if (need <= *cap) return WIG_OK;
   if (*buf) cudaFree(*buf);

@@ -1,0 +1,44 @@
+"""The tile overrides of the register-blocked passes (WIG_*_BTILING) are checked
+on the host before any compile: a tile that leaves rows or columns of the grid
+to no CTA, or that a CTA cannot run, is WIG_ERR_ARG."""
+import ctypes
+
+import pytest
+
+from pywignercuda_b200 import _lib
+
+
+def refused(monkeypatch, fn, desc, env, value):
+    """The message of the refusal (asserted); the descriptor itself is accepted."""
+    buf = ctypes.create_string_buffer(1 << 16)
+    monkeypatch.setenv(env, value)
+    assert getattr(_lib.load(), fn)(desc, buf, len(buf)) == 1, buf.value[:300]
+    assert env in buf.value.decode()
+
+
+def accepted(monkeypatch, fn, desc, env, value):
+    buf = ctypes.create_string_buffer(1 << 16)
+    monkeypatch.setenv(env, value)
+    assert getattr(_lib.load(), fn)(desc, buf, len(buf)) == 0, buf.value[:300]
+
+
+def adjoint_desc(n_x, n_p):
+    d = _lib.WigaDesc()
+    d.abi_version = _lib.ABI_VERSION
+    d.n_x, d.n_p = n_x, n_p
+    d.precision = _lib.WIGA_PREC_C128
+    d.x_amplitude = d.p_amplitude = 10.
+    d.hbar = d.mass = 1.
+    d.dt = 0.005
+    return d
+
+
+# rows and columns that do not divide the grid, more than 1024 threads, more than 32 columns, no tile at all
+@pytest.mark.parametrize('n_x,n_p,value', [(256, 128, '8,3,1'), (128, 256, '8,1,3'), (256, 128, '8,64,1'),
+                                           (128, 64, '8,1,64'), (64, 64, '8,128,1')])
+def test_adjoint_tile_refused(monkeypatch, n_x, n_p, value):
+    refused(monkeypatch, 'wiga_jit_check', adjoint_desc(n_x, n_p), 'WIG_ADJ_BTILING', value)
+
+
+def test_adjoint_tile_accepted(monkeypatch):
+    accepted(monkeypatch, 'wiga_jit_check', adjoint_desc(256, 128), 'WIG_ADJ_BTILING', '4,2,2')
