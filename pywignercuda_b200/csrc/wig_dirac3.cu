@@ -116,15 +116,17 @@ int d3_plan(const dirac3_desc* d, Dirac3Plan* P) {
     int nt[3];
     for (int i = 0; i < 3; ++i) {
       P->be[i] = v[3 * i] ? v[3 * i] : (i == 1 ? (n[i] >= 128 ? 16 : (small ? 4 : 8)) : (small ? 4 : 8));
+      if (P->be[i] != 4 && P->be[i] != 8 && P->be[i] != 16)
+        return fail(WIG_ERR_ARG, "WIG_D3_BTILING: %d elements a thread", P->be[i]);
       const int T = n[i] / P->be[i];
       int c = least[i];
       while (c * T < 32) c *= 2;
       while (c < most[i] && 2 * c * T <= 256 && lines[i] / (2 * c) >= 2 * 148) c *= 2;
       P->bc[i] = v[3 * i + 1] ? v[3 * i + 1] : c;
+      if (int rc = check_blk_tile("WIG_D3_BTILING", P->bc[i], T, i == 0 ? NY * NZ : NX, i == 0 ? 1024 : 32)) return rc;
       nt[i] = P->bc[i] * T;
-      P->bmb[i] = v[3 * i + 2] ? v[3 * i + 2]
+      P->bmb[i] = v[3 * i + 2] > 0 ? v[3 * i + 2]
                                : std::max(1, std::min(32, (i == 1 || P->be[i] == 4 ? 512 : 256) / nt[i]));
-      if (nt[i] > 1024 || nt[i] % 32 || (i > 0 && P->bc[i] > 32)) return fail(WIG_ERR_ARG, "WIG_D3_BTILING: tile of %d threads", nt[i]);
     }
     const auto pad = [](int n, int e) { return n + n / std::min(e, 8); };
     P->xnt = nt[0];

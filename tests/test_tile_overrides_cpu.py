@@ -42,3 +42,27 @@ def test_adjoint_tile_refused(monkeypatch, n_x, n_p, value):
 
 def test_adjoint_tile_accepted(monkeypatch):
     accepted(monkeypatch, 'wiga_jit_check', adjoint_desc(256, 128), 'WIG_ADJ_BTILING', '4,2,2')
+
+
+def dirac3_desc(*shape):
+    d = _lib.Dirac3Desc()
+    d.abi_version = _lib.ABI_VERSION
+    d.n_x, d.n_y, d.n_z = shape
+    d.constants = _lib.CONST_CUDA_F
+    d.precision = _lib.PREC_C128
+    d.x_amplitude = d.y_amplitude = d.z_amplitude = 8.
+    d.mass, d.c, d.hbar, d.dt = 1., 137.036, 1., 1e-4
+    return d
+
+
+# lines of x, y and z that do not divide the grid, 2048 threads, 64 columns, no line, 5 elements a thread
+@pytest.mark.parametrize('shape,value', [((256, 32, 32), '8,3,0,0,0,0,0,0,0'), ((64, 256, 32), '0,0,0,16,6,0,0,0,0'),
+                                         ((64, 32, 256), '0,0,0,0,0,0,8,3,0'), ((256, 32, 32), '8,64,0,0,0,0,0,0,0'),
+                                         ((64, 64, 64), '0,0,0,8,64,0,0,0,0'), ((64, 64, 64), '8,-4,0,0,0,0,0,0,0'),
+                                         ((64, 64, 64), '0,0,0,0,0,0,5,0,0')])
+def test_dirac3d_tile_refused(monkeypatch, shape, value):
+    refused(monkeypatch, 'dirac3_jit_check', dirac3_desc(*shape), 'WIG_D3_BTILING', value)
+
+
+def test_dirac3d_tile_accepted(monkeypatch):
+    accepted(monkeypatch, 'dirac3_jit_check', dirac3_desc(64, 32, 32), 'WIG_D3_BTILING', '4,4,1,4,8,1,4,8,1')
