@@ -84,7 +84,7 @@ int check_desc(const wiga_desc* d) {
     return fail(WIG_ERR_ARG, "wiga: gamma must be finite and f_eps >= 0");
   if (d->precision == WIGA_PREC_C128) {
     const BlkTiles t = blk_tiles(d->n_x, d->n_p);
-    if (int rc = check_blk_tile("WIG_ADJ_BTILING", t.xr, d->n_x / t.e, d->n_p, 1024)) return rc;
+    if (int rc = check_blk_tile("WIG_ADJ_BTILING", t.xr, d->n_x / t.e, d->n_p, wig::seq_max(d->n_x / t.e))) return rc;
     return check_blk_tile("WIG_ADJ_BTILING", t.pc, d->n_p / t.e, d->n_x, 32);
   }
   return WIG_OK;

@@ -582,8 +582,10 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
     // 512 threads per SM: 128 registers each (the x-pass of 16 elements a thread: 448, 144, no spill)
     if (!P->bxmb) P->bxmb = std::max(1, std::min(32, (P->bxe == 16 ? 448 : 512) / nt));
     if (!P->bpmb) P->bpmb = std::max(1, std::min(32, 512 / ntp));
-    if (nt > 1024 || ntp > 1024 || (P->bpc & (P->bpc - 1)) || NP % P->bxr)
-      return fail(WIG_ERR_ARG, "WIG_BTILING: tiles of %d / %d threads", nt, ntp);
+    if (P->bx)
+      if (int rc = check_blk_tile("WIG_BTILING", P->bxr, NX / P->bxe, NP, wig::seq_max(NX / P->bxe))) return rc;
+    if (P->bp)
+      if (int rc = check_blk_tile("WIG_BTILING", P->bpc, NP / P->bpe, NX, 32)) return rc;
     P->gx = NP / P->bxr + 1;
     P->gx_nt = nt;
     P->gx_smem = P->bxr * (pad(NX, P->bxe) + wig::blk_pre_slots(NX, P->bxe)) * (int)sizeof(double2);
@@ -1460,6 +1462,8 @@ static int dirac_plan(const dirac_desc* d, DiracPlan* P) {
     if (v[3] == 4 || v[3] == 8) P->bce = v[3];
     P->brows = std::max(v[1], std::max(1, 32 * P->bre / NX));
     P->bc = std::max(v[4] > 0 ? v[4] : (e == 8 && NX >= 512 ? (NY <= 512 ? 4 : (NY <= 1024 ? 2 : 1)) : 1), std::max(1, 32 * P->bce / NY));
+    if (int rc = check_blk_tile("WIG_DIRAC_BTILING", P->brows, NX / P->bre, NY, wig::seq_max(NX / P->bre))) return rc;
+    if (int rc = check_blk_tile("WIG_DIRAC_BTILING", P->bc, NY / P->bce, NX, 32)) return rc;
     P->rnt = P->brows * (NX / P->bre);
     P->cnt = P->bc * (NY / P->bce);
     P->brmb = v[2] > 0 ? v[2] : std::max(1, std::min(32, (P->bre == 8 ? 256 : 512) / P->rnt));
@@ -1469,8 +1473,6 @@ static int dirac_plan(const dirac_desc* d, DiracPlan* P) {
     P->n_col = NX / P->bc;
     P->smem_row = P->brows * 4 * pad(NX, P->bre) * (int)sizeof(double2);
     P->smem_col = P->bc * wig::blk_stride(4 * pad(NY, P->bce), P->bc) * (int)sizeof(double2);
-    if (P->rnt > 1024 || P->cnt > 1024 || NY % P->brows || NX % P->bc)
-      return fail(WIG_ERR_ARG, "WIG_DIRAC_BTILING: tiles of %d / %d threads", P->rnt, P->cnt);
   }
   // GPU_Dirac2D.py:312-346
   P->dX = 2. * d->x_amplitude / (double)NX;

@@ -123,7 +123,8 @@ int d3_plan(const dirac3_desc* d, Dirac3Plan* P) {
       while (c * T < 32) c *= 2;
       while (c < most[i] && 2 * c * T <= 256 && lines[i] / (2 * c) >= 2 * 148) c *= 2;
       P->bc[i] = v[3 * i + 1] ? v[3 * i + 1] : c;
-      if (int rc = check_blk_tile("WIG_D3_BTILING", P->bc[i], T, i == 0 ? NY * NZ : NX, i == 0 ? 1024 : 32)) return rc;
+      if (int rc = check_blk_tile("WIG_D3_BTILING", P->bc[i], T, i == 0 ? NY * NZ : NX, i == 0 ? wig::seq_max(T) : 32))
+        return rc;
       nt[i] = P->bc[i] * T;
       P->bmb[i] = v[3 * i + 2] > 0 ? v[3 * i + 2]
                                : std::max(1, std::min(32, (i == 1 || P->be[i] == 4 ? 512 : 256) / nt[i]));

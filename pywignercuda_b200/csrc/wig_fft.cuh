@@ -504,8 +504,11 @@ template <int NTH> struct SyncGroup {
 #endif
   }
 };
-// The barrier of a sequence of T threads, `per_cta` sequences in the CTA (consecutive threads)
+// The barrier of a sequence of T threads, `per_cta` sequences in the CTA (consecutive threads).  A CTA has
+// 16 hardware barriers, the first of them __syncthreads': 15 sequences of more than a warp.
+__host__ __device__ constexpr int seq_max(int t) { return t <= 32 ? 1024 : 15; }
 template <int T, int PER_CTA> struct SeqSync {
+  static_assert(PER_CTA <= seq_max(T), "a hardware barrier for every sequence");
   __device__ __forceinline__ static auto make(int seq) {
     if constexpr (T <= 32) return SyncWarp{};
     else if constexpr (PER_CTA == 1) return SyncCta{};

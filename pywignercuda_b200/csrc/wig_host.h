@@ -58,8 +58,8 @@ bool safe_expr(const std::string& e);
 extern const char* kMathPrelude;
 // The tile of a register-blocked pass, which an override (the variable `env`) may have set: `seqs` sequences
 // (rows or columns) of `threads` threads a CTA, `total` sequences in the pass.  WIG_ERR_ARG unless seqs is a
-// power of two of at most `most` that divides total (a rest would be left to no CTA) and the CTA is whole
-// warps of at most 1024 threads.
+// power of two of at most `most` (rows: wig::seq_max; columns: a warp's 32) that divides total (a rest would
+// be left to no CTA) and the CTA is whole warps of at most 1024 threads.
 int check_blk_tile(const char* env, int seqs, int threads, long total, int most);
 // Grow a device observable buffer to `need` doubles.
 int ensure_obs(double** buf, size_t* cap, size_t need);

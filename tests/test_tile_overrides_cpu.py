@@ -66,3 +66,35 @@ def test_dirac3d_tile_refused(monkeypatch, shape, value):
 
 def test_dirac3d_tile_accepted(monkeypatch):
     accepted(monkeypatch, 'dirac3_jit_check', dirac3_desc(64, 32, 32), 'WIG_D3_BTILING', '4,4,1,4,8,1,4,8,1')
+
+
+def wigner_desc(n_x, n_p):
+    d = _lib.WigDesc()
+    d.abi_version = _lib.ABI_VERSION
+    d.n_x, d.n_p = n_x, n_p
+    d.x_amplitude = d.p_amplitude = 10.
+    d.hbar = d.mass = 1.
+    d.dt = 0.01
+    return d
+
+
+def dirac_desc(n_x, n_y):
+    d = _lib.DiracDesc()
+    d.abi_version = _lib.ABI_VERSION
+    d.n_x, d.n_y = n_x, n_y
+    d.x_amplitude = d.y_amplitude = 12.
+    d.mass, d.c, d.hbar, d.dt = 1., 137.036, 1., 1e-4
+    return d
+
+
+ROWS = [('wig_jit_check', wigner_desc, 'WIG_BTILING', (256, 64), '4,%d,0,0,0,0,-1'),
+        ('dirac_jit_check', dirac_desc, 'WIG_DIRAC_BTILING', (256, 64), '4,%d,0,0,0,0'),
+        ('dirac3_jit_check', dirac3_desc, 'WIG_D3_BTILING', (256, 32, 32), '4,%d,0,0,0,0,0,0,0'),
+        ('wiga_jit_check', adjoint_desc, 'WIG_ADJ_BTILING', (256, 64), '4,%d,0')]
+
+
+@pytest.mark.parametrize('fn,desc,env,shape,value', ROWS, ids=[r[2] for r in ROWS])
+def test_rows_beyond_the_hardware_barriers_refused(monkeypatch, fn, desc, env, shape, value):
+    """Rows of 64 threads each take one of a CTA's 15 named barriers: 16 rows (1024 threads) have none."""
+    refused(monkeypatch, fn, desc(*shape), env, value % 16)
+    accepted(monkeypatch, fn, desc(*shape), env, value % 8)
