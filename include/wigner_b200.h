@@ -150,10 +150,11 @@ int wig_create(const wig_desc* desc, wig_handle** out);
 int wig_run(wig_handle* h, void* W_dev, int64_t t_index0, int64_t n_prop, uint32_t flags,
             double* obs_host, void* stream);
 
-/* The (n_prop + 1) x WIG_NOBS observables of the handle's last wig_run (n_rows = its n_prop + 1, with
- * obs_host NULL there) into out_dev, device memory, in the order of `stream`: a caller that splits a run
- * into several calls reads them once, at the end.  wig_check_observables is the check that wig_run makes
- * of obs_host (WIG_ERR_NONFINITE).  (Run keeps its averages on the host, :1845-1879.) */
+/* The first n_rows of the (n_prop + 1) x WIG_NOBS observables of the handle's last wig_run (or wig_run_many)
+ * into out_dev, device memory, in the order of `stream`: a caller that splits a run into several calls
+ * (with obs_host NULL) reads them once, at the end.  More rows than that run recorded, and a current device
+ * other than the handle's, are WIG_ERR_ARG.  wig_check_observables is the check that wig_run makes of
+ * obs_host (WIG_ERR_NONFINITE).  (Run keeps its averages on the host, :1845-1879.) */
 int wig_run_observables(wig_handle* h, double* out_dev, int64_t n_rows, void* stream);
 int wig_check_observables(const double* obs_host, int64_t n_rows);
 

@@ -386,6 +386,7 @@ struct wig_handle {
   DevBuf bufs;
   double* obs = nullptr;
   size_t obs_cap = 0;
+  int64_t obs_rows = 0;                         // rows of obs that the last run recorded
   double2* scale = nullptr;
   double2* W_host_stage = nullptr;   // device copy used by wig_run_host
   std::vector<cudaEvent_t> ev;       // WIG_RUN_PROFILE: 3 events per step
@@ -891,6 +892,7 @@ static int wig_run_check(wig_handle* h, void* W_dev, int64_t n_prop) {
   int cur;
   WIG_CUDA(cudaGetDevice(&cur));
   if (cur != h->device) return fail(WIG_ERR_ARG, "wig_run: current device %d != handle device %d", cur, h->device);
+  h->obs_rows = 0;
   if (int rc = ensure_obs(&h->obs, &h->obs_cap, (size_t)(n_prop + 1) * WIG_NOBS)) return rc;
   if (h->gp)
     if (int rc = ensure_obs(&h->psq, &h->psq_cap, (size_t)std::max<int64_t>(n_prop, 1))) return rc;
@@ -1099,6 +1101,7 @@ extern "C" int wig_run(wig_handle* h, void* W_dev, int64_t t_index0, int64_t n_p
     if (int rc = wig_run_step(h, &S, n, st)) return rc;
   if (int rc = wig_run_end(h, &S, st)) return rc;
   h->psq_n = n_prop;
+  h->obs_rows = n_prop + 1;
   h->last_stream = st;
   if (obs_host) {
     if (int rc = wig_copy_obs(h, n_prop, obs_host, st)) return rc;
@@ -1112,8 +1115,13 @@ extern "C" int wig_run(wig_handle* h, void* W_dev, int64_t t_index0, int64_t n_p
 
 extern "C" int wig_run_observables(wig_handle* h, double* out_dev, int64_t n_rows, void* stream) {
   if (!h || !out_dev) return fail(WIG_ERR_ARG, "wig_run_observables: null argument");
-  if (n_rows < 1 || (size_t)n_rows * WIG_NOBS > h->obs_cap)
-    return fail(WIG_ERR_ARG, "wig_run_observables: the last run did not record %lld rows", (long long)n_rows);
+  if (n_rows < 1 || n_rows > h->obs_rows)
+    return fail(WIG_ERR_ARG, "wig_run_observables: %lld rows asked, the last run recorded %lld", (long long)n_rows,
+                (long long)h->obs_rows);
+  int cur;
+  WIG_CUDA(cudaGetDevice(&cur));
+  if (cur != h->device)
+    return fail(WIG_ERR_ARG, "wig_run_observables: current device %d != handle device %d", cur, h->device);
   cudaStream_t st = (cudaStream_t)stream;
   WIG_CUDA(cudaMemcpyAsync(out_dev, h->obs, (size_t)n_rows * WIG_NOBS * sizeof(double), cudaMemcpyDeviceToDevice, st));
   return h->tma ? wig_check_status(h, st) : WIG_OK;
@@ -1311,8 +1319,10 @@ extern "C" int wig_run_many(wig_handle* const* hs, void* const* Ws, int64_t coun
   for (int64_t n = 0; n < n_prop; ++n)
     for (int64_t i = 0; i < count; ++i)
       if (int rc = wig_run_step(hs[i], &S[i], n, st)) return rc;
-  for (int64_t i = 0; i < count; ++i)
+  for (int64_t i = 0; i < count; ++i) {
     if (int rc = wig_run_end(hs[i], &S[i], st)) return rc;
+    hs[i]->obs_rows = n_prop + 1;
+  }
   if (obs_host) {
     for (int64_t i = 0; i < count; ++i)
       if (obs_host[i])
