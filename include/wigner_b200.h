@@ -151,11 +151,11 @@ int wig_run(wig_handle* h, void* W_dev, int64_t t_index0, int64_t n_prop, uint32
             double* obs_host, void* stream);
 
 /* The first n_rows of the (n_prop + 1) x WIG_NOBS observables of the handle's last wig_run (or wig_run_many)
- * into out_dev, device memory, in the order of `stream`: a caller that splits a run into several calls
- * (with obs_host NULL) reads them once, at the end.  More rows than that run recorded, and a current device
+ * into out, device or page-locked host memory, in the order of `stream`: a caller that splits a run into
+ * several calls (with obs_host NULL) need not wait for each.  More rows than that run recorded, and a current device
  * other than the handle's, are WIG_ERR_ARG.  wig_check_observables is the check that wig_run makes of
  * obs_host (WIG_ERR_NONFINITE).  (Run keeps its averages on the host, :1845-1879.) */
-int wig_run_observables(wig_handle* h, double* out_dev, int64_t n_rows, void* stream);
+int wig_run_observables(wig_handle* h, double* out, int64_t n_rows, void* stream);
 int wig_check_observables(const double* obs_host, int64_t n_rows);
 
 /* wig_run on host buffers: W_in (host, complex128) is copied to the device,

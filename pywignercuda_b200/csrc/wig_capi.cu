@@ -1113,8 +1113,8 @@ extern "C" int wig_run(wig_handle* h, void* W_dev, int64_t t_index0, int64_t n_p
   return WIG_OK;
 }
 
-extern "C" int wig_run_observables(wig_handle* h, double* out_dev, int64_t n_rows, void* stream) {
-  if (!h || !out_dev) return fail(WIG_ERR_ARG, "wig_run_observables: null argument");
+extern "C" int wig_run_observables(wig_handle* h, double* out, int64_t n_rows, void* stream) {
+  if (!h || !out) return fail(WIG_ERR_ARG, "wig_run_observables: null argument");
   if (n_rows < 1 || n_rows > h->obs_rows)
     return fail(WIG_ERR_ARG, "wig_run_observables: %lld rows asked, the last run recorded %lld", (long long)n_rows,
                 (long long)h->obs_rows);
@@ -1123,7 +1123,7 @@ extern "C" int wig_run_observables(wig_handle* h, double* out_dev, int64_t n_row
   if (cur != h->device)
     return fail(WIG_ERR_ARG, "wig_run_observables: current device %d != handle device %d", cur, h->device);
   cudaStream_t st = (cudaStream_t)stream;
-  WIG_CUDA(cudaMemcpyAsync(out_dev, h->obs, (size_t)n_rows * WIG_NOBS * sizeof(double), cudaMemcpyDeviceToDevice, st));
+  WIG_CUDA(cudaMemcpyAsync(out, h->obs, (size_t)n_rows * WIG_NOBS * sizeof(double), cudaMemcpyDefault, st));
   return h->tma ? wig_check_status(h, st) : WIG_OK;
 }
 

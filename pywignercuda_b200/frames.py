@@ -136,8 +136,10 @@ class FrameWriter:
     ``capture(key, state, stream)`` snapshots ``state`` (a contiguous CUDA tensor) on ``stream`` and
     returns; the write happens later on the writer thread as ``sink[...]`` assignments made by
     ``emit(sink, key, host_array)``.  ``keep`` (a dict, may be None) receives a private copy of each
-    host frame as ``emit`` formed it.  ``close()`` waits for every pending frame and re-raises the
-    first error of the writer thread."""
+    host frame as ``emit`` formed it.  ``check()``, if given to ``capture``, runs on the writer thread once
+    the frame is on the host; what it raises is the writer's error, and this frame and the later ones are
+    not written.  ``close()`` waits for every pending frame and, as ``capture`` does, re-raises the first
+    error of the writer thread."""
 
     def __init__(self, like, sink, emit, keep=None, depth=3):
         import torch
@@ -156,12 +158,13 @@ class FrameWriter:
         self.thread.start()
         self.n_frames = 0
 
-    def capture(self, key, state, stream=None):
+    def capture(self, key, state, stream=None, check=None):
         torch = self._torch
-        if self.error is not None:
-            raise self.error
         st = stream if stream is not None else torch.cuda.current_stream(self.device)
         slot = self.free.get()
+        if self.error is not None:
+            self.free.put(slot)
+            raise self.error
         with torch.cuda.stream(st):
             self.snap[slot].copy_(state)                  # device to device on the compute stream
             snapped = torch.cuda.Event()
@@ -171,7 +174,7 @@ class FrameWriter:
             self.host[slot].copy_(self.snap[slot], non_blocking=True)
             done = torch.cuda.Event()
             done.record(self.copy_stream)
-        self.todo.put((key, slot, done))
+        self.todo.put((key, slot, done, check))
         self.n_frames += 1
 
     def _loop(self):
@@ -180,10 +183,12 @@ class FrameWriter:
             if item is None:
                 self.todo.task_done()
                 return
-            key, slot, done = item
+            key, slot, done, check = item
             try:
                 if self.error is None:
                     done.synchronize()
+                    if check is not None:
+                        check()
                     frame = self.emit(self.sink, key, self.host[slot].numpy())
                     if self.keep is not None:
                         self.keep[key] = copy_frame(frame)

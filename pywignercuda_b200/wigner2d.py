@@ -20,6 +20,7 @@ The propagation runs on the GPU through ``libwigner_b200.so``; device memory
 and the stream come from PyTorch.  There is no CPU path.
 """
 import ctypes
+from functools import partial
 
 import numpy as np
 
@@ -291,7 +292,7 @@ class GPU_Wigner2D_FFT(Propagator_Base):
 
     def _stretch(self, W, n_prop, t_index0, continue_run, samples):
         """``propagate`` on the current stream without waiting for it: rows ``t_index0`` ..
-        ``t_index0 + n_prop`` of the device tensor ``samples`` receive the observables."""
+        ``t_index0 + n_prop`` of the page-locked ``samples`` receive the observables."""
         lib, st = _lib.load(), _torch().cuda.current_stream(W.device).cuda_stream
         flags = _lib.WIG_RUN_CONTINUE if continue_run else 0
         check(lib.wig_run(self._handle, W.data_ptr(), t_index0, n_prop, flags, None, st), 'wig_run')
@@ -326,8 +327,15 @@ class GPU_Wigner2D_FFT(Propagator_Base):
             W = torch.from_numpy(W0.copy()).to(dev)
             n_total = int(self.timeSteps) + 1             # Run :1776 loops over 0..timeSteps
             skip = max(int(self.skipFrames), 1)
-            # the stretches between frames run without a host wait: their samples collect on the device
-            samples = torch.zeros((max(n_total, 0) + 1, _lib.WIG_NOBS), dtype=torch.float64, device=dev)
+            # the stretches between frames run without a host wait: their samples arrive in page-locked
+            # memory, where each frame's writer finds those of the steps before it
+            samples = torch.zeros((max(n_total, 0) + 1, _lib.WIG_NOBS), dtype=torch.float64, pin_memory=True)
+            obs = samples.numpy()
+
+            def finite(first, last):
+                if not np.isfinite(obs[first:last + 1]).all():
+                    check(_lib.load().wig_check_observables(dptr(obs[first:last + 1]), last + 1 - first), 'wig_run')
+
             sink, writer = self._frame_writer(W)
             saved = []
             t, cont = 0, False
@@ -337,14 +345,18 @@ class GPU_Wigner2D_FFT(Propagator_Base):
                         if not cont:                       # W must be normalised first
                             self._stretch(W, 0, 0, False, samples)
                             cont = True
-                        writer.capture(t, W)               # the sample before step t (:1880-1882)
+                        # the sample before step t (:1880-1882); a run whose samples up to here are not finite
+                        # ends with this frame unwritten (at the next capture that waits for its buffer)
+                        writer.capture(t, W, check=partial(finite, max(t - skip, 0), t))
                         saved.append(t)
                     nxt = min(n_total, (t // skip + 1) * skip)
                     self._stretch(W, nxt - t, t, cont, samples)
                     t, cont = nxt, True
-                W_end = W.cpu().numpy()
-                obs = samples.cpu().numpy()
-                check(_lib.load().wig_check_observables(dptr(obs), obs.shape[0]), 'wig_run')
+                W_end = W.cpu().numpy()                    # the samples have arrived, too
+                finite(0, obs.shape[0] - 1)
+            except BaseException:
+                torch.cuda.current_stream(dev).synchronize()   # no copy into `samples` outlives it
+                raise
             finally:
                 writer.close()
         n = int(self.timeSteps) + 1
