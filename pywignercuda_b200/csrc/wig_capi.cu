@@ -266,6 +266,17 @@ std::vector<double> shifted_range(double amp, int n) {
   return out;
 }
 
+// Whether a shifted table of n (even) values is odd about 0, t[k] = -t[n - k], to the rounding of a linspace
+// (below 1e-15 of its ends; entry n / 2 has no partner); no table counts as odd.
+bool odd_table(const double* t, int n) {
+  if (!t) return true;
+  double top = 0.;
+  for (int k = 0; k < n; ++k) top = std::max(top, fabs(t[k]));
+  for (int k = 0; k < n / 2; ++k)
+    if (!(fabs(t[k] + t[(n - k) % n]) <= 1e-14 * top)) return false;
+  return true;
+}
+
 // tw[m] = exp(-2 pi i m / n), extended precision, exact zeros on the axes
 std::vector<double2> twiddles(int n) {
   const long double pi = 3.141592653589793238462643383279502884L;
@@ -537,7 +548,11 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
 
   // ---- register-blocked passes (BlockFft)
   {
-    const bool stockham = P->rf || getenv("WIG_TILING") || getenv("WIG_RADIX");   // tile overrides of the other forms
+    // Tile overrides of the other forms; and ODM or mean-field terms on a caller's table that is not odd about
+    // 0: the register-blocked ones evaluate one point of each pair +-lambda (+-theta) and mirror it.
+    const bool stockham = P->rf || getenv("WIG_TILING") || getenv("WIG_RADIX") ||
+                          ((P->odm || P->gp) && !odd_table(d->lambda_table, NX)) ||
+                          (P->gp && !odd_table(d->theta_table, NP));
     P->bx = !stockham && NX >= 32 ? 1 : 0;
     P->bp = !stockham && NP >= 32 ? 1 : 0;
     // Elements a thread: as many as the grid leaves threads for.  16 (two stage boundaries in
