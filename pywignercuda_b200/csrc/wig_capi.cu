@@ -514,9 +514,9 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
 
   // ---- register-FFT passes (wig_wigner_rf.cuh) for Lie plans without ODM damping on
   // 64..1024-point axes, with the p-pass tile loaded by 2-D tensor copies: opt-in (WIG_RF="1",
-  // or WIG_RF="xw,pw" with the warps per x-pass / p-pass CTA).  On the 1024^2 Caldeira-Leggett
-  // case they measured slower than the Stockham passes (2.47 vs 2.18 ms per 16-replica step:
-  // 255 registers a thread leave 5 warps per SM), so the Stockham passes are the default.
+  // or WIG_RF="xw,pw" with the warps per x-pass / p-pass CTA).  A 16-replica step of the 1024^2
+  // Caldeira-Leggett case takes 2.47 ms on them (255 registers a thread leave 5 warps per SM), 2.18 on
+  // the Stockham passes and 1.01 on the register-blocked ones below, which are the default.
   const auto rf_size = [](int n) { return n >= 64 && n <= 1024; };
   P->rf = 0;
   if (const char* rv = getenv("WIG_RF")) {
@@ -558,10 +558,21 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
     // Elements a thread: as many as the grid leaves threads for.  16 (two stage boundaries in
     // shared memory up to 4096 points, 128 registers, 16 warps per SM) from 2^20 points along x and
     // 2^19 along p, 8 from 2^17, below that 4, where the step is a chain of latencies and more warps
-    // shorten it.  Damped step, us, x,p of 16,16 / 8,16 / 8,8: 1024^2 65 / 65 / 75; 512 x 1024
-    // 42 / 38 / 39; 1024 x 512 39 / 38 / 36; 2048 x 256 38 / 37 / 38 (time-dependent 40 / 38 / 45);
-    // 4096 x 128 41 / 39 / 50.  Both of 16 / 8 / 4: 512^2 36 / 22 / 28; 512 x 256 - / 16 / 16;
-    // 256^2 26 / 13 / 11; 128^2 - / 12 / 10; 1024 x 64 - / 15 / 13.
+    // shorten it.  Steps, us, x,p of 16,16 / 8,16 / 8,8 (two columns a CTA of the p-pass):
+    //                 damped           driven           undamped         mean field
+    //   2048^2        227 / 237 / 299  232 / 242 / 311  119 / 129 / 156  424 / 437 / 531
+    //   1024^2         62 /  62 /  75   64 /  65 /  78   35 /  35 /  40  128 / 106 / 126
+    //   1024 x 512     38 /  36 /  33   40 /  39 /  33   23 /  28 /  20   90 /  70 /  67
+    //   512 x 1024     40 /  37 /  38   42 /  38 /  40   24 /  27 /  20   96 /  72 /  71
+    //   2048 x 256     37 /  35 /  32   37 /  36 /  34   29 /  26 /  20   81 /  73 /  67
+    //   4096 x 128     40 /  37 /  32   40 /  38 /  34   30 /  28 /  21   82 /  76 /  77
+    //   256 x 2048     43 /  40 /  42   45 /  42 /  43   25 /  33 /  22   97 /  81 /  81
+    //   128 x 4096     46 /  41 /  50   49 /  44 /  51   28 /  34 /  23  107 /  98 /  96
+    // (Fokker-Planck as damped and undamped.)  From 2^20 points on 16 along p is the faster one in every
+    // form.  At 2^19 points it is so for damped steps on p-axes of 1024 points and more; on shorter
+    // ones and undamped 8 would be faster by 5 to 40 %: this line does not tell them apart.  Both of
+    // 16 / 8 / 4, damped: 512^2 36 / 22 / 28; 512 x 256 - / 16 / 16; 256^2 26 / 13 / 11; 128^2 - / 12 / 10;
+    // 1024 x 64 - / 15 / 13.
     const long pts = (long)NX * NP;
     const auto elems = [&](int n, long top) {
       return std::max(pts >= top ? 16 : (pts >= (1L << 17) ? 8 : 4), n / 512);
@@ -614,7 +625,9 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
     if (!P->bp) { P->gp_n = P->n_cta_p; P->gp_nt = P->pnt; P->gp_smem = P->smem_p; P->gph_smem = P->smem_ph; }
     P->odm2 = P->odm && P->bx && P->bp ? 1 : 0;
     // ODM: 8 elements a thread, 4 below 2^17 points on axes up to 2048 (both axes alike).  Steps, us, with
-    // 8 / 4: 64 x 128 27 / 19, 256^2 32 / 24, 64 x 1024 36 / 29, 1024 x 64 36 / 30, 512 x 128 31 / 30.
+    // 8 / 4: 64 x 128 26 / 19, 256^2 31 / 23, 64 x 1024 36 / 29, 1024 x 64 36 / 30, 512 x 128 31 / 29;
+    // 512 x 256 33 / 32, 512^2 41 / 52, 1024 x 256 45 / 51, 1024^2 127 / 169, 2048^2 522 / 741.  The line by
+    // points is off for long p-axes on narrow grids: 128 x 2048 61 / 53.  16: 1024^2 144, 2048^2 585.
     P->oe = pts >= (1L << 17) || std::max(NX, NP) > 2048 ? 8 : 4;
     P->oxr = std::max(1, 32 * P->oe / NX);
     P->opc = P->oe == 4 || NP / P->oe >= 512 ? std::max(1, 32 * P->oe / NP) : std::max(2, 32 * P->oe / NP);
@@ -1773,13 +1786,12 @@ struct BVariant {
 
 // Whether the x-pass stages its rows in shared memory (WIGB_XSTAGE).  Off by
 // default.  At the register caps below, the staging buffer is what limits the
-// x-pass's resident warps (a 2-warp mixed CTA: 33 KB of exchange + 16 KB of
-// staging, 4 CTAs per SM); without it the x-pass runs 12 (mixed) or 16 (FP32)
-// warps per SM.  On the 64-instance mixed-grid batch (B200, CUDA events): mixed
-// x-pass 253 us staged at 8 warps per SM, 220 us direct at 12; FP32 173 us staged
-// at 12, 164 us direct at 16.  (At the earlier 8 / 12-warp caps staging had been
-// the faster one: 272 -> 240 and 182 -> 169 us.)  Tuning override (read per
-// compile): WIG_BATCH_XSTAGE=0|1.
+// x-pass's resident warps (a 4-warp CTA: 37 KB of exchange, mixed, or 33 KB,
+// FP32, and 32 KB of staging: 3 CTAs per SM); without it the x-pass runs 16 warps
+// per SM.  On the 64-instance mixed-grid batch (B200, CUDA events, 4-warp tiles),
+// x-pass us direct / staged: mixed 120 / 130 at 16 warps per SM and 127 / 129 at
+// 12; FP32 146 / 158 and 166 / 156.  Tuning override (read per compile):
+// WIG_BATCH_XSTAGE=0|1.
 int batch_xstage(int) {
   const char* e = getenv("WIG_BATCH_XSTAGE");
   if (e && *e) return atoi(e) ? 1 : 0;

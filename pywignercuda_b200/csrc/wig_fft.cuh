@@ -377,8 +377,8 @@ __device__ __forceinline__ void cta_fft(C* s, const C* __restrict__ tw) {
 // Twiddles.  The input r of a radix-16 butterfly carries w^{k r}, w = exp(-2 pi i /
 // (16 NS)); with r = 4 a + b the factor w^{4 k a} is applied before the butterfly's
 // first four 4-point DFTs (over a) and w^{k b} after them, so 6 table entries serve
-// a butterfly instead of 15: the loads, not the FP64 pipe, bound these passes
-// (shared + L1 wavefronts 75 % of peak, FP64 34 %, 1024^2 damped p-pass).
+// a butterfly instead of 15: the passes wait for loads, boundaries and dependent
+// chains rather than for the FP64 pipe (44 % busy in the 1024^2 damped p-pass).
 // Table (host: wighost::block_twiddles), stage after stage (NS > 1), NS entries
 // each: radix 16: w^{4 k a}, a = 1..3, then w^{k b}, b = 1..3; radix R < 16: w^{k r},
 // r = 1..R - 1, w = exp(-2 pi i / (R NS)).  Entry k of one factor is next to k + 1:

@@ -10,7 +10,7 @@
 #define WIGA_PREC 0
 #endif
 #if WIGA_PREC == 1
-typedef double2 WigaC;
+typedef double2 WigaC;   // without WIGA_B only on the host (the device code's tests): the library always sets it
 #else
 typedef float2 WigaC;
 #endif

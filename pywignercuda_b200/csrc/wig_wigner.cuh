@@ -4,6 +4,12 @@
 // both axes (array index 0 holds coordinate 0) -- the reference's layout
 // (GPU_Wigner2D_FFT.py:577-581).
 //
+// Axes of at least 32 points run on the register-blocked passes at the end of this file
+// (xpass_blk_body, ppass_blk_body, odm_*_blk_body, gp_phase_blk_body: a thread keeps its
+// elements of a row or column in registers from load to store); shorter axes, the Bloch
+// steps, plans with a tile override of these forms, and ODM or mean-field plans whose lambda
+// or theta table is not odd about 0 on the shared-memory tiles before them.  Both do:
+//
 //  x-pass (one CTA = ROWS contiguous rows):
 //      prologue: deferred normalisation W <- W * s, s = 1/(dX dP sum W) taken
 //                from the previous pass's per-CTA partial sums;
@@ -15,7 +21,7 @@
 //      two absorbing masks, column IFFT (1/N_p folded in)
 //      (expPotential_source :80-126, :1891-1899);
 //      Caldeira-Leggett order 3 (CaldeiraDissipatorOrder3 :1145-1157) on the
-//      tile still in shared memory;
+//      columns still on the chip;
 //      epilogue: store W' and this CTA's partial sums of the 10 observables
 //      plus sum W (Run :1857-1878,1912).
 //
