@@ -558,7 +558,7 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
     // Elements a thread: as many as the grid leaves threads for.  16 (two stage boundaries in
     // shared memory up to 4096 points, 128 registers, 16 warps per SM) from 2^20 points along x and
     // 2^19 along p, 8 from 2^17, below that 4, where the step is a chain of latencies and more warps
-    // shorten it.  Steps, us, x,p of 16,16 / 8,16 / 8,8 (two columns a CTA of the p-pass):
+    // shorten it.  Steps, us, x,p of 16,16 / 8,16 / 8,8 (columns a CTA of the p-pass as below):
     //                 damped           driven           undamped         mean field
     //   2048^2        227 / 237 / 299  232 / 242 / 311  119 / 129 / 156  424 / 437 / 531
     //   1024^2         62 /  62 /  75   64 /  65 /  78   35 /  35 /  40  128 / 106 / 126
@@ -568,9 +568,10 @@ static int wig_plan(const wig_desc* d, WigPlan* P) {
     //   4096 x 128     40 /  37 /  32   40 /  38 /  34   30 /  28 /  21   82 /  76 /  77
     //   256 x 2048     43 /  40 /  42   45 /  42 /  43   25 /  33 /  22   97 /  81 /  81
     //   128 x 4096     46 /  41 /  50   49 /  44 /  51   28 /  34 /  23  107 /  98 /  96
-    // (Fokker-Planck as damped and undamped.)  From 2^20 points on 16 along p is the faster one in every
-    // form.  At 2^19 points it is so for damped steps on p-axes of 1024 points and more; on shorter
-    // ones and undamped 8 would be faster by 5 to 40 %: this line does not tell them apart.  Both of
+    // (Fokker-Planck as damped and undamped; mean field damped.)  From 2^20 points on 16 along p is the
+    // faster one in every form.  At 2^19 points it is so for damped steps on p-axes of 1024 points and more;
+    // on shorter ones 8 would be faster by 6 to 14 % and undamped by 24 to 34 %: this line does not tell
+    // them apart, nor the x-pass of 1024^2 mean-field steps, which 8 would serve better.  Both of
     // 16 / 8 / 4, damped: 512^2 36 / 22 / 28; 512 x 256 - / 16 / 16; 256^2 26 / 13 / 11; 128^2 - / 12 / 10;
     // 1024 x 64 - / 15 / 13.
     const long pts = (long)NX * NP;
